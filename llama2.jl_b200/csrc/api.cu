@@ -2,6 +2,7 @@
 // per-token CUDA graph, and the isolated-operator entry points.
 #include "../../include/llama2_b200.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -57,6 +58,9 @@ struct DevMatrix {
     int64_t file_bytes = 0;   // bytes in the stored (file) format
     bool panels = false;      // k-quant rows longer than one stage, stored as column panels
     int kb = MV_TILE_BLOCKS;  // stage width in super-blocks this matrix is laid out for (panel width)
+    // for the many-column product: the blocks as [panels][rows][panel row bytes], and a narrower last panel (encoded at upload)
+    CUtensorMap map_main, map_tail;
+    bool maps_ready = false;
     bool present() const { return data != nullptr; }
 };
 
@@ -108,7 +112,29 @@ static int32_t panelize(DevMatrix& m, cudaStream_t st) {
     return L2B_OK;
 }
 
-static int32_t upload_matrix(DevMatrix& m, int type, const void* host, int64_t in, int64_t out, cudaStream_t st, bool panels = true) {
+// Tensor maps of a k-quant matrix: box = one super-block of 128 rows.  A matrix without maps is refused where they are needed.
+static void encode_matrix_maps(DevMatrix& w) {
+    EncodeTiledFn enc = encode_tiled_fn();
+    w.maps_ready = false;
+    if (!enc) return;
+    const int bb = dev_block_bytes(w.type);
+    const int64_t nb = w.in / QK_K, kb = w.panels ? w.kb : nb;
+    const int64_t full_panels = nb / kb, tail_blocks = nb % kb;
+    auto make = [&](CUtensorMap& m, uint8_t* base, int64_t blocks, int64_t panels) {
+        const cuuint64_t dims[3] = {(cuuint64_t)(blocks * bb), (cuuint64_t)w.out, (cuuint64_t)panels};
+        const cuuint64_t strides[2] = {(cuuint64_t)(blocks * bb), (cuuint64_t)(blocks * bb) * (cuuint64_t)w.out};
+        const cuuint32_t box[3] = {(cuuint32_t)bb, (cuuint32_t)GM_ROWS, 1u};
+        const cuuint32_t estr[3] = {1u, 1u, 1u};
+        return enc(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    bool ok = make(w.map_main, w.data, kb, full_panels);
+    w.map_tail = w.map_main;
+    if (ok && tail_blocks > 0) ok = make(w.map_tail, w.data + (size_t)full_panels * w.out * kb * bb, tail_blocks, 1);
+    w.maps_ready = ok;
+}
+
+static int32_t upload_blocks(DevMatrix& m, int type, const void* host, int64_t in, int64_t out, cudaStream_t st, bool panels) {
     if (!type_supported(type)) return fail(L2B_ERR_UNSUPPORTED_TYPE, "tensor type " + std::to_string(type) + " not implemented");
     if (!host || in <= 0 || out <= 0) return fail(L2B_ERR_BAD_ARG, "upload: null pointer or empty shape");
     if (type != T_F32 && in % QK_K != 0) return fail(L2B_ERR_BAD_ARG, "k-quant tensors need in_dim % 256 == 0");
@@ -145,6 +171,12 @@ static int32_t upload_matrix(DevMatrix& m, int type, const void* host, int64_t i
     cudaFree(raw);
     CU(e);
     return panels ? panelize(m, st) : L2B_OK;
+}
+
+static int32_t upload_matrix(DevMatrix& m, int type, const void* host, int64_t in, int64_t out, cudaStream_t st, bool panels = true) {
+    L2B_TRY(upload_blocks(m, type, host, in, out, st, panels));
+    if (type != T_F32) encode_matrix_maps(m);
+    return L2B_OK;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -269,7 +301,9 @@ static void set_kernel_attrs() {
         set((const void*)fused_matvec_kernel<true, 1, true>);
         set((const void*)fused_matvec_kernel<true, 2, true>);
         set((const void*)fused_matvec_kernel<true, 3, true>);
-        set((const void*)kq_gemm_kernel);
+        set((const void*)kq_gemm_kernel<32>);
+        set((const void*)kq_gemm_kernel<64>);
+        set((const void*)kq_gemm_kernel<128>);
         set((const void*)token_kernel<1>);
         set((const void*)token_kernel<2>);
         set((const void*)token_kernel<3>);
@@ -364,71 +398,128 @@ static int choose_gq(int n_heads, int n_kv) {
 // ---- tensor-core GEMM (kq_gemm.cuh): host side ----------------------------------------------------------
 static bool gemm_supported(const DevMatrix& w) { return (w.type == T_Q4_K || w.type == T_Q5_K) && w.out >= 1; }
 
-// The matrix as a 3-D byte tensor [panels][rows][panel row bytes]; box = one super-block of 128 rows.
-static int32_t gemm_tensor_maps(const DevMatrix& w, CUtensorMap& main_map, CUtensorMap& tail_map, int& kb_eff) {
-    EncodeTiledFn enc = encode_tiled_fn();
-    if (!enc) return fail(L2B_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    const int bb = dev_block_bytes(w.type);
-    const int64_t nb = w.in / QK_K;
-    kb_eff = w.panels ? w.kb : (int)nb;
-    const int64_t full_panels = nb / kb_eff, tail_blocks = nb % kb_eff;
-    auto make = [&](CUtensorMap& m, uint8_t* base, int64_t blocks, int64_t panels) -> int32_t {
-        const cuuint64_t dims[3] = {(cuuint64_t)(blocks * bb), (cuuint64_t)w.out, (cuuint64_t)panels};
-        const cuuint64_t strides[2] = {(cuuint64_t)(blocks * bb), (cuuint64_t)(blocks * bb) * (cuuint64_t)w.out};
-        const cuuint32_t box[3] = {(cuuint32_t)bb, (cuuint32_t)GM_ROWS, 1u};
-        const cuuint32_t estr[3] = {1u, 1u, 1u};
-        const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) return fail(L2B_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
-        return L2B_OK;
-    };
-    if (full_panels > 0) L2B_TRY(make(main_map, w.data, kb_eff, full_panels));
-    if (tail_blocks > 0) L2B_TRY(make(tail_map, w.data + (size_t)full_panels * w.out * kb_eff * bb, tail_blocks, 1));
-    else tail_map = main_map;
-    if (full_panels == 0) main_map = tail_map;
-    return L2B_OK;
+// Operands of a product: the activations of n_tok tokens as two fp16 terms, their sub-block sums, the tokens' factors.
+struct GemmInput {
+    uint8_t *act = nullptr, *xs = nullptr;
+    float* scale = nullptr;
+    int groups = 0;
+};
+static int gemm_groups(int n_tok) { return (n_tok + 15) / 16 * 2; }
+static size_t gemm_input_bytes(int64_t n_in, int n_tok) {
+    const size_t g = gemm_groups(n_tok);
+    return (size_t)(n_in / QK_K) * g * (4 * GM_GROUP_BYTES + GM_XS_BYTES) + g * 32;
+}
+static GemmInput gemm_input(uint8_t* buf, int64_t n_in, int n_tok) {
+    GemmInput in;
+    in.groups = gemm_groups(n_tok);
+    const size_t g = in.groups, nb = n_in / QK_K;
+    in.act = buf;
+    in.xs = buf + nb * g * 4 * GM_GROUP_BYTES;
+    in.scale = (float*)(in.xs + nb * g * GM_XS_BYTES);
+    return in;
 }
 
-static size_t gemm_act_bytes(int64_t n_in, int n_tok) { return (size_t)((n_tok + GM_TOK - 1) / GM_TOK) * (size_t)(n_in / QK_K) * GM_ACT_BYTES; }
+// Tokens per tile and super-blocks per block.  `whole`: every tile by one block (no partial results).  Otherwise the super-blocks are
+// dealt out evenly, but never so thinly that a tile falls into more than eight parts or a block's start-up outweighs its work.
+static GemmSplit gemm_split(int row_tiles, int nb, int n_tok, int sms, bool whole) {
+    GemmSplit s;
+    const int t16 = (n_tok + 15) / 16 * 16;
+    s.nb = nb;
+    s.ntile = (t16 + GM_MAX_TOK - 1) / GM_MAX_TOK;
+    s.tok = ((t16 + s.ntile - 1) / s.ntile + 15) / 16 * 16;
+    const int tiles = row_tiles * s.ntile;
+    if (whole) s.U = nb * ((tiles + sms - 1) / sms);
+    else s.U = std::max({(int)(((int64_t)tiles * nb + sms - 1) / sms), std::min(nb, 2), (nb + 6) / 7});
+    return s;
+}
+// Most parts a tile of this split can fall into.
+static int gemm_max_parts(const GemmSplit& s) { return s.U % s.nb == 0 ? 1 : s.nb % s.U == 0 ? s.nb / s.U : (s.nb - 2) / s.U + 2; }
 
-// x [n_tok][ldx] f32 (optionally rmsnorm'ed with `gain`) -> int8 planes in the GEMM's operand layout
-static int32_t launch_quantise_rows(const float* x, const float* gain, uint8_t* act, int n, int ldx, int n_tok, cudaStream_t st) {
-    CU(cudaMemsetAsync(act, 0, gemm_act_bytes(n, n_tok), st));  // unused columns and tokens must read as zero
-    QuantRowsParams q;
-    q.x = x; q.gain = gain; q.act = act; q.n = n; q.ldx = ldx; q.n_tok = n_tok;
-    quantise_rows_kernel<<<n_tok, 512, 0, st>>>(q);
+static int gemm_row_tiles(const DevMatrix& w) { return (int)((w.out + GM_ROWS - 1) / GM_ROWS); }
+
+template <int MODE>
+static int32_t launch_split_rows(const SplitRowsParams& q, cudaStream_t st) {
+    split_rows_kernel<MODE><<<q.n_tok, 512, 0, st>>>(q);
+    CU(cudaGetLastError());
+    return L2B_OK;
+}
+static SplitRowsParams split_rows_params(float* x, const float* gain, int n, int n_tok, const GemmInput& in) {
+    SplitRowsParams q;
+    memset(&q, 0, sizeof(q));
+    q.x = x; q.gain = gain; q.n = n; q.n_tok = n_tok; q.groups = in.groups; q.act = in.act; q.xs = in.xs; q.scale = in.scale;
+    return q;
+}
+
+// y[part][t][ldy] = the matrices' rows (each matrix from a multiple of 128 on) times the tokens of `in`
+static int32_t launch_kq_gemm(const DevMatrix* const* ws, int nw, const GemmInput& in, int n_tok, const GemmSplit& sp, float* y, size_t part_stride, int ldy, int* status,
+                              cudaStream_t st) {
+    GemmParams g;
+    GemmMaps maps;
+    memset(&g, 0, sizeof(g));
+    int tiles = 0, max_bb = 0;
+    for (int i = 0; i < nw; ++i) {
+        const DevMatrix& w = *ws[i];
+        if (w.type == T_F32) return fail(L2B_ERR_UNSUPPORTED_TYPE, "the tensor-core GEMM takes k-quant matrices");
+        if (!w.maps_ready) return fail(L2B_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver, or refused this matrix");
+        GemmSeg& sg = g.seg[i];
+        sg.type = w.type; sg.rows = (int)w.out; sg.row_tiles = gemm_row_tiles(w); sg.kb = w.panels ? w.kb : sp.nb; sg.d6 = w.d6;
+        maps.main[i] = w.map_main;
+        maps.tail[i] = w.map_tail;
+        tiles += sg.row_tiles;
+        max_bb = std::max(max_bb, dev_block_bytes(w.type));
+    }
+    for (int i = nw; i < GM_MAX_SEG; ++i) maps.main[i] = maps.main[0], maps.tail[i] = maps.tail[0];
+    g.nseg = nw; g.sp = sp; g.total = tiles * sp.ntile * sp.nb; g.n_tok = n_tok; g.groups = in.groups;
+    g.act = in.act; g.xs = in.xs; g.scale = in.scale; g.y = y; g.part_stride = part_stride; g.ldy = ldy; g.status = status;
+    const int grid = (g.total + sp.U - 1) / sp.U;
+    auto go = [&](auto kernel, auto layout, int threads) {
+        g.np = GM_MAX_PACKED;
+        while (layout(max_bb, g.np).total + 1024 > GM_SMEM) --g.np;  // + room to align the base to 1024 bytes
+        kernel<<<grid, threads, layout(max_bb, g.np).total + 1024, st>>>(g, maps);
+    };
+    if (sp.tok <= 32) go(kq_gemm_kernel<32>, gm_smem_layout<32>, GmCfg<32>::THREADS);
+    else if (sp.tok <= 64) go(kq_gemm_kernel<64>, gm_smem_layout<64>, GmCfg<64>::THREADS);
+    else go(kq_gemm_kernel<128>, gm_smem_layout<128>, GmCfg<128>::THREADS);
     CU(cudaGetLastError());
     return L2B_OK;
 }
 
-// y[t][ldy] (+= resid) = W x_t for n_tok activation vectors already quantised by launch_quantise_rows
-static int32_t launch_kq_gemm(const DevMatrix& w, const uint8_t* act, int n_tok, float* y, int ldy, const float* resid, int* status, cudaStream_t st) {
-    if (!gemm_supported(w)) return fail(L2B_ERR_UNSUPPORTED_TYPE, "the tensor-core GEMM takes q4_K and q5_K matrices");
-    CUtensorMap mm, mt;
-    int kb_eff = 0;
-    L2B_TRY(gemm_tensor_maps(w, mm, mt, kb_eff));
-    GemmParams g;
-    memset(&g, 0, sizeof(g));
-    g.type = w.type; g.rows = (int)w.out; g.nb = (int)(w.in / QK_K); g.kb = kb_eff; g.n_tok = n_tok;
-    g.act = act; g.y = y; g.resid = resid; g.ldy = ldy; g.mode = resid ? GM_RESIDUAL : GM_STORE; g.status = status;
-    const dim3 grid((unsigned)((w.out + GM_ROWS - 1) / GM_ROWS), (unsigned)((n_tok + GM_TOK - 1) / GM_TOK));
-    const size_t smem = (size_t)gm_smem_layout(dev_block_bytes(w.type)).total + 1024;  // + room to align the base to 1024 bytes
-    kq_gemm_kernel<<<grid, GM_THREADS, smem, st>>>(g, mm, mt);
+// One product wanted as such, y[n_tok][out]: whole tiles straight to y, or shared tiles and a pass that adds their parts where whole
+// tiles would leave the last wave so empty that the extra pass (about five super-blocks' time) is cheaper.
+static GemmSplit gemm_product_split(const DevMatrix& w, int n_tok, int sms) {
+    const int nb = (int)(w.in / QK_K), rt = gemm_row_tiles(w);
+    const GemmSplit whole = gemm_split(rt, nb, n_tok, sms, true), shared = gemm_split(rt, nb, n_tok, sms, false);
+    return shared.U + 5 < whole.U ? shared : whole;
+}
+static size_t gemm_product_bytes(const DevMatrix& w, int n_tok, int sms) {
+    const int parts = gemm_max_parts(gemm_product_split(w, n_tok, sms));
+    return parts == 1 ? 0 : (size_t)parts * n_tok * w.out * 4;
+}
+static int32_t launch_product(const DevMatrix& w, const GemmInput& in, int n_tok, float* y, float* parts, int sms, int* status, cudaStream_t st) {
+    const GemmSplit sp = gemm_product_split(w, n_tok, sms);
+    const DevMatrix* ws[1] = {&w};
+    if (gemm_max_parts(sp) == 1) return launch_kq_gemm(ws, 1, in, n_tok, sp, y, 0, (int)w.out, status, st);
+    const size_t stride = (size_t)n_tok * w.out;
+    L2B_TRY(launch_kq_gemm(ws, 1, in, n_tok, sp, parts, stride, (int)w.out, status, st));
+    sum_parts_kernel<<<dim3((unsigned)std::min<int64_t>(16, (w.out + 255) / 256), n_tok), 256, 0, st>>>(parts, stride, sp, (int)w.out, (int)w.out, y);
     CU(cudaGetLastError());
     return L2B_OK;
 }
 
 // Buffers of a many-token pass: activations of up to PF_MAX_TOK tokens, attention scratch, quantised activations.
 struct GemmBufs {
-    float *x = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *att = nullptr, *g = nullptr, *u = nullptr;
+    float *x = nullptr, *q = nullptr, *att = nullptr, *h = nullptr;  // residual stream, rotated queries, attention output, SwiGLU output
+    float* y = nullptr;  // partial results of the product at hand
+    size_t y_bytes = 0;
     float *pm = nullptr, *pl = nullptr, *pacc = nullptr;
     int* tickets = nullptr;
     uint8_t* act = nullptr;
     int nsplit = 1;
+    int sms = 0;
 };
 
 static void free_gemm_bufs(GemmBufs& B) {
-    void* pf[] = {B.x, B.q, B.k, B.v, B.att, B.g, B.u, B.pm, B.pl, B.pacc, B.tickets, B.act};
+    void* pf[] = {B.x, B.q, B.att, B.h, B.y, B.pm, B.pl, B.pacc, B.tickets, B.act};
     for (void* b : pf)
         if (b) cudaFree(b);
     B = GemmBufs();
@@ -1764,31 +1855,53 @@ static int32_t run_one(l2b_session* s, int token, int pos, float temperature, do
 // ---- many-token prompt pass ---------------------------------------------------------------------------------
 // The reference runs transformer! once per prompt token (src/inference.jl:349-356).  For prompt positions that are all followed
 // by a prompt token (no logits needed) the layers are run for up to PF_MAX_TOK tokens at once: every matrix product is one
-// launch of the tensor-core GEMM (20 tokens per pass over a weight tile), the element-wise steps are small kernels over
+// launch of the tensor-core GEMM (up to 128 tokens per pass over a weight tile), the element-wise steps are small kernels over
 // [tokens][dim] arrays, attention serves every token's query against the cache (causal: token t sees positions <= pos0 + t).
 // Needs q4_K / q5_K layer matrices, three activation planes, one GPU; otherwise the caller uses the decode passes.
-constexpr int PF_MAX_TOK = 240;
+constexpr int PF_MAX_TOK = 512;
 constexpr int PF_MIN_TOK = 12;
+constexpr int BATCH_MAX_SEQ = 240;
 constexpr int STACK_MIN_ROWS = 2;  // layer-stack models
 
 // Every layer for n tokens whose residual-stream rows are in B.x.  One sequence: token t sits at position pos0 + t and the
 // layer's caches are kc / vc + l * layer_stride.  Batched decode (pos_list non-null): token t is the next position pos_list[t]
 // of sequence t, whose caches lie seq_stride * t further.
+//
+// A layer is ten launches: q, k and v share one product, gate and up another; every product leaves partial results which the
+// kernel behind it adds (RoPE and cache write; residual + norm + operand; SwiGLU + operand).  On return the last feed-forward's
+// residual is added to B.x, and B.act holds the operands of B.x behind `final_gain` where that is given.
 static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n, float* kc, float* vc, size_t layer_stride, int pos0, const int* pos_list,
-                                   size_t seq_stride, const float* rope_cs, int gq, int* status, cudaStream_t st) {
+                                   size_t seq_stride, const float* rope_cs, int gq, const float* final_gain, int* status, cudaStream_t st) {
     const l2b_config& c = m->cfg;
     const int hs = c.dim / c.n_heads, kv_dim = hs * c.n_kv_heads;
+    const GemmInput in_dim = gemm_input(B.act, c.dim, n), in_hid = gemm_input(B.act, c.hidden_dim, n);
+    auto product = [&](std::initializer_list<const DevMatrix*> ws, const GemmInput& in, GemmSplit& sp, size_t& stride, int& ldy) -> int32_t {
+        int rt = 0;
+        for (const DevMatrix* w : ws) rt += gemm_row_tiles(*w);
+        sp = gemm_split(rt, (int)((*ws.begin())->in / QK_K), n, B.sms, false);
+        ldy = rt * GM_ROWS;
+        stride = (size_t)n * ldy;
+        if (gemm_max_parts(sp) * stride * 4 > B.y_bytes) return fail(L2B_ERR_STATE, "many-token pass: buffer of the partial results too small");
+        return launch_kq_gemm(ws.begin(), (int)ws.size(), in, n, sp, B.y, stride, ldy, status, st);
+    };
+    auto behind = [&](SplitRowsParams q, const GemmSplit& sp, size_t stride, int ldy, int up_row) {
+        q.y = B.y; q.sp = sp; q.part_stride = stride; q.ldy = ldy; q.up_row = up_row;
+        return q;
+    };
+    GemmSplit sp;
+    size_t stride = 0;
+    int ldy = 0;
+    L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.x, m->layers[0].rms_att, c.dim, n, in_dim), st));
     for (int l = 0; l < c.n_layers; ++l) {
         const LayerW& w = m->layers[l];
         float* kcl = kc + (size_t)l * layer_stride;
         float* vcl = vc + (size_t)l * layer_stride;
-        L2B_TRY(launch_quantise_rows(B.x, w.rms_att, B.act, c.dim, c.dim, n, st));
-        L2B_TRY(launch_kq_gemm(w.wq, B.act, n, B.q, c.dim, nullptr, status, st));
-        L2B_TRY(launch_kq_gemm(w.wk, B.act, n, B.k, kv_dim, nullptr, status, st));
-        L2B_TRY(launch_kq_gemm(w.wv, B.act, n, B.v, kv_dim, nullptr, status, st));
+        L2B_TRY(product({&w.wq, &w.wk, &w.wv}, in_dim, sp, stride, ldy));
         RopeKvParams r;
         memset(&r, 0, sizeof(r));
-        r.q = B.q; r.k = B.k; r.v = B.v; r.kc = kcl; r.vc = vcl; r.rope_cs = rope_cs;
+        r.y = B.y; r.part_stride = stride; r.ldy = ldy; r.sp = sp;
+        r.k_row = gemm_row_tiles(w.wq) * GM_ROWS; r.v_row = r.k_row + gemm_row_tiles(w.wk) * GM_ROWS;
+        r.q = B.q; r.kc = kcl; r.vc = vcl; r.rope_cs = rope_cs;
         r.n_tok = n; r.q_dim = c.dim; r.kv_dim = kv_dim; r.hs = hs; r.seq_len = c.seq_len; r.pos0 = pos0; r.neox = c.rope_is_neox;
         r.pos_list = pos_list; r.cache_stride = seq_stride;
         rope_kv_kernel<<<dim3(8, n), 256, 0, st>>>(r);
@@ -1804,15 +1917,14 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
         a.min_chunk = 256;  // many queries already fill the GPU: split a query's positions only when there are many
         if (n < 2) return fail(L2B_ERR_BAD_ARG, "a many-token pass needs at least two tokens");
         CU(launch_attention(a, gq, st, false));
-        L2B_TRY(launch_quantise_rows(B.att, nullptr, B.act, c.dim, c.dim, n, st));
-        L2B_TRY(launch_kq_gemm(w.wo, B.act, n, B.x, c.dim, B.x, status, st));
-        L2B_TRY(launch_quantise_rows(B.x, w.rms_ffn, B.act, c.dim, c.dim, n, st));
-        L2B_TRY(launch_kq_gemm(w.w1, B.act, n, B.g, c.hidden_dim, nullptr, status, st));
-        L2B_TRY(launch_kq_gemm(w.w3, B.act, n, B.u, c.hidden_dim, nullptr, status, st));
-        swiglu_rows_kernel<<<1184, 256, 0, st>>>(B.g, B.u, (size_t)n * c.hidden_dim);
-        CU(cudaGetLastError());
-        L2B_TRY(launch_quantise_rows(B.g, nullptr, B.act, c.hidden_dim, c.hidden_dim, n, st));
-        L2B_TRY(launch_kq_gemm(w.w2, B.act, n, B.x, c.dim, B.x, status, st));
+        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.att, nullptr, c.dim, n, in_dim), st));
+        L2B_TRY(product({&w.wo}, in_dim, sp, stride, ldy));
+        L2B_TRY(launch_split_rows<SR_RESIDUAL>(behind(split_rows_params(B.x, w.rms_ffn, c.dim, n, in_dim), sp, stride, ldy, 0), st));
+        L2B_TRY(product({&w.w1, &w.w3}, in_dim, sp, stride, ldy));
+        L2B_TRY(launch_split_rows<SR_SWIGLU>(behind(split_rows_params(B.h, nullptr, c.hidden_dim, n, in_hid), sp, stride, ldy, gemm_row_tiles(w.w1) * GM_ROWS), st));
+        L2B_TRY(product({&w.w2}, in_hid, sp, stride, ldy));
+        const float* gain = l + 1 < c.n_layers ? m->layers[l + 1].rms_att : final_gain;
+        L2B_TRY(launch_split_rows<SR_RESIDUAL>(behind(split_rows_params(B.x, gain, c.dim, n, gain ? in_dim : GemmInput()), sp, stride, ldy, 0), st));
     }
     return L2B_OK;
 }
@@ -1827,16 +1939,28 @@ static bool gemm_layers_supported(const l2b_model* m) {
     return true;
 }
 
-static bool alloc_gemm_bufs(const l2b_model* m, GemmBufs& B, size_t T) {
+static bool alloc_gemm_bufs(const l2b_model* m, GemmBufs& B, size_t T, bool classifier) {
     const l2b_config& c = m->cfg;
-    const int hs = c.dim / c.n_heads, kv_dim = hs * c.n_kv_heads;
+    const int hs = c.dim / c.n_heads;
+    DeviceInfo di;
+    if (query_device(di) != L2B_OK) return false;
+    B.sms = di.sms;
     B.nsplit = c.seq_len >= 2048 ? 4 : 1;
+    const LayerW& w = m->layers[0];  // every layer has these shapes
+    auto need = [&](std::initializer_list<const DevMatrix*> ws, size_t n) {
+        int rt = 0;
+        for (const DevMatrix* x : ws) rt += gemm_row_tiles(*x);
+        return (size_t)gemm_max_parts(gemm_split(rt, (int)((*ws.begin())->in / QK_K), (int)n, B.sms, false)) * n * rt * GM_ROWS * 4;
+    };
+    for (size_t n = 2; n <= T; ++n) {
+        B.y_bytes = std::max({B.y_bytes, need({&w.wq, &w.wk, &w.wv}, n), need({&w.wo}, n), need({&w.w1, &w.w3}, n), need({&w.w2}, n)});
+        if (classifier && m->output.type != T_F32) B.y_bytes = std::max(B.y_bytes, gemm_product_bytes(m->output, (int)n, B.sms));
+    }
     auto alloc = [&](auto*& ptr, size_t bytes) { return cudaMalloc((void**)&ptr, bytes) == cudaSuccess; };
-    bool ok = alloc(B.x, T * c.dim * 4) && alloc(B.q, T * c.dim * 4) && alloc(B.k, T * kv_dim * 4) && alloc(B.v, T * kv_dim * 4) &&
-              alloc(B.att, T * c.dim * 4) && alloc(B.g, T * c.hidden_dim * 4) && alloc(B.u, T * c.hidden_dim * 4) &&
+    bool ok = alloc(B.x, T * c.dim * 4) && alloc(B.q, T * c.dim * 4) && alloc(B.att, T * c.dim * 4) && alloc(B.h, T * c.hidden_dim * 4) && alloc(B.y, B.y_bytes) &&
               alloc(B.pm, T * c.n_heads * B.nsplit * 4) && alloc(B.pl, T * c.n_heads * B.nsplit * 4) &&
               alloc(B.pacc, T * c.n_heads * B.nsplit * hs * 4) && alloc(B.tickets, T * c.n_heads * 4) &&
-              alloc(B.act, gemm_act_bytes(std::max(c.dim, c.hidden_dim), (int)T));
+              alloc(B.act, gemm_input_bytes(std::max(c.dim, c.hidden_dim), (int)T));
     if (ok) ok = cudaMemset(B.tickets, 0, T * c.n_heads * 4) == cudaSuccess;
     if (!ok) {
         (void)cudaGetLastError();
@@ -1850,7 +1974,7 @@ static bool prefill_gemm_eligible(l2b_session* s) {
     if (s->pf_checked) return s->pf_ok;
     s->pf_checked = true;
     // (a pass that cannot get its buffers leaves prompts to the decode passes)
-    s->pf_ok = env_long("L2B_PREFILL_GEMM", 1) != 0 && gemm_layers_supported(s->model) && alloc_gemm_bufs(s->model, s->pf, PF_MAX_TOK);
+    s->pf_ok = env_long("L2B_PREFILL_GEMM", 1) != 0 && gemm_layers_supported(s->model) && alloc_gemm_bufs(s->model, s->pf, std::min(PF_MAX_TOK, std::max(2, s->model->cfg.seq_len)), false);
     return s->pf_ok;
 }
 
@@ -1872,10 +1996,10 @@ static int32_t enqueue_prefill_gemm(l2b_session* s, int pos0, int n) {
     embed_rows_kernel<<<dim3(std::max(1, std::min(16, c.dim / 256)), n), 256, 0, st>>>(m->tok_emb.type, m->tok_emb.data, m->tok_emb.d6, s->prompt + pos0, c.dim,
                                                                                       c.vocab_size, s->pf.x);
     CU(cudaGetLastError());
-    L2B_TRY(enqueue_layers_gemm(m, s->pf, n, s->kc, s->vc, kv_layer_elems(m), pos0, nullptr, 0, s->rope_cs, s->gq, s->status, st));
+    L2B_TRY(enqueue_layers_gemm(m, s->pf, n, s->kc, s->vc, kv_layer_elems(m), pos0, nullptr, 0, s->rope_cs, s->gq, nullptr, s->status, st));
     fill_forced_kernel<<<1, 256, 0, st>>>(s->prompt, s->out_tokens, pos0, n);
     CU(cudaGetLastError());
-    s->last_launches += 2 + 14LL * c.n_layers;  // per layer: 4 quantise, 7 GEMM, RoPE + cache write, attention, SwiGLU
+    s->last_launches += 3 + 10LL * c.n_layers;  // per layer: 4 products, 4 operand kernels, RoPE + cache write, attention
     return L2B_OK;
 }
 
@@ -2234,7 +2358,7 @@ extern "C" int32_t l2b_batch_create(l2b_model* m, int32_t n_seq, l2b_batch** out
     if (!m || !out) return fail(L2B_ERR_BAD_ARG, "null argument");
     *out = nullptr;
     if (!m->finalized) return fail(L2B_ERR_STATE, "l2b_model_finalize has not been called");
-    if (n_seq < 2 || n_seq > PF_MAX_TOK) return fail(L2B_ERR_BAD_ARG, "a batch holds 2 .. " + std::to_string(PF_MAX_TOK) + " sequences");
+    if (n_seq < 2 || n_seq > BATCH_MAX_SEQ) return fail(L2B_ERR_BAD_ARG, "a batch holds 2 .. " + std::to_string(BATCH_MAX_SEQ) + " sequences");
     CU(cudaSetDevice(m->device));
     L2B_TRY(check_kernel_attrs());
     if (!m->stack && !gemm_layers_supported(m))
@@ -2265,7 +2389,7 @@ extern "C" int32_t l2b_batch_create(l2b_model* m, int32_t n_seq, l2b_batch** out
             return L2B_OK;
         }
         b->gq = choose_gq(c.n_heads, c.n_kv_heads);
-        if (!alloc_gemm_bufs(m, b->B, (size_t)n_seq)) return fail(L2B_ERR_OOM, "out of device memory for the batch buffers");
+        if (!alloc_gemm_bufs(m, b->B, (size_t)n_seq, true)) return fail(L2B_ERR_OOM, "out of device memory for the batch buffers");
         const size_t cache = kv_layer_elems(m) * c.n_layers * (size_t)n_seq * 4;
         CU(cudaMalloc(&b->kc, cache));
         CU(cudaMalloc(&b->vc, cache));
@@ -2319,12 +2443,11 @@ static int32_t enqueue_batch_llama(l2b_batch* b, cudaStream_t st) {
                                                                                       c.vocab_size, b->B.x);
     CU(cudaGetLastError());
     const size_t kvl = kv_layer_elems(m);
-    L2B_TRY(enqueue_layers_gemm(m, b->B, n, b->kc, b->vc, kvl * (size_t)n, 0, b->pos, kvl, b->rope_cs, b->gq, b->status, st));
     // final rmsnorm + classifier (src/inference.jl:309-312) for every sequence, then argmax (:360)
-    if (gemm_supported(m->output)) {
-        L2B_TRY(launch_quantise_rows(b->B.x, m->rms_final, b->B.act, c.dim, c.dim, n, st));
-        L2B_TRY(launch_kq_gemm(m->output, b->B.act, n, b->logits, c.vocab_size, nullptr, b->status, st));
-    } else {  // a q6_K classifier: one pass of the matrix-vector kernel per sequence
+    L2B_TRY(enqueue_layers_gemm(m, b->B, n, b->kc, b->vc, kvl * (size_t)n, 0, b->pos, kvl, b->rope_cs, b->gq, m->rms_final, b->status, st));
+    if (m->output.type != T_F32) {
+        L2B_TRY(launch_product(m->output, gemm_input(b->B.act, c.dim, n), n, b->logits, b->B.y, b->di.sms, b->status, st));
+    } else {  // an f32 classifier: one pass of the matrix-vector kernel per sequence
         for (int i = 0; i < n; ++i) {
             MvLaunch L;
             memset(&L.p, 0, sizeof(L.p));
@@ -2645,7 +2768,7 @@ struct l2b_matrix {
     int device = 0;
     DeviceInfo di;
     int* status = nullptr;
-    uint8_t* act = nullptr;  // quantised activation columns of l2b_matrix_matmul_device (grown on demand)
+    uint8_t* act = nullptr;  // operands and partial results of l2b_matrix_matmul_device (grown on demand)
     size_t act_bytes = 0;
 };
 
@@ -2682,14 +2805,14 @@ extern "C" int32_t l2b_matrix_destroy(l2b_matrix* m) {
 }
 
 // y[c] = A' x[c] for ncols columns on device pointers (x: [ncols][in], y: [ncols][out]) through the tensor-core GEMM:
-// the columns are quantised once, then every weight tile is unpacked once per 20 columns.
+// the columns are split into operand terms once, then every weight tile is unpacked once per 128 columns.
 extern "C" int32_t l2b_matrix_matmul_device(l2b_matrix* m, int32_t copy, const float* dev_x, int32_t ncols, float* dev_y, void* stream) {
     if (!m || !dev_x || !dev_y || ncols < 1) return fail(L2B_ERR_BAD_ARG, "bad argument");
     if (copy < 0 || copy >= (int)m->copies.size()) return fail(L2B_ERR_BAD_ARG, "copy index out of range");
     const DevMatrix& w = m->copies[copy];
     if (!gemm_supported(w)) return fail(L2B_ERR_UNSUPPORTED_TYPE, "the tensor-core GEMM takes q4_K and q5_K matrices");
     CU(cudaSetDevice(m->device));
-    const size_t need = gemm_act_bytes(w.in, ncols);
+    const size_t in_bytes = (gemm_input_bytes(w.in, ncols) + 255) & ~(size_t)255, need = in_bytes + gemm_product_bytes(w, ncols, m->di.sms);
     if (need > m->act_bytes) {
         if (m->act) cudaFree(m->act);
         m->act = nullptr;
@@ -2697,8 +2820,9 @@ extern "C" int32_t l2b_matrix_matmul_device(l2b_matrix* m, int32_t copy, const f
         CU(cudaMalloc(&m->act, need));
         m->act_bytes = need;
     }
-    L2B_TRY(launch_quantise_rows(dev_x, nullptr, m->act, (int)w.in, (int)w.in, ncols, (cudaStream_t)stream));
-    return launch_kq_gemm(w, m->act, ncols, dev_y, (int)w.out, nullptr, m->status, (cudaStream_t)stream);
+    const GemmInput in = gemm_input(m->act, w.in, ncols);
+    L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(const_cast<float*>(dev_x), nullptr, (int)w.in, ncols, in), (cudaStream_t)stream));
+    return launch_product(w, in, ncols, dev_y, (float*)(m->act + in_bytes), m->di.sms, m->status, (cudaStream_t)stream);
 }
 
 extern "C" int32_t l2b_matrix_matvec_device(l2b_matrix* m, int32_t copy, const float* dev_x, float* dev_y, int32_t planes, void* stream) {
@@ -2730,14 +2854,16 @@ extern "C" int32_t l2b_matrix_matvec(l2b_matrix* m, const float* host_x, int32_t
     DevBuf x, y;
     L2B_TRY(dev_upload(x, host_x, (size_t)ncols * w.in * 4));
     L2B_TRY(dev_alloc(y, (size_t)ncols * w.out * 4));
-    // Several columns: one pass of the tensor-core GEMM per 20 columns (every weight is unpacked once for all of them)
+    // Several columns: one pass of the tensor-core GEMM per 128 columns (every weight is unpacked once for all of them)
     // instead of one matrix-vector pass per column.  L2B_GEMM_MIN_COLS sets the threshold (default 4; 0 switches it off).
     const long gemm_min = env_long("L2B_GEMM_MIN_COLS", 4);
     if (gemm_min > 0 && ncols >= gemm_min && (planes == 0 || planes == 3) && gemm_supported(w)) {
-        DevBuf act;
-        L2B_TRY(dev_alloc(act, gemm_act_bytes(w.in, ncols)));
-        L2B_TRY(launch_quantise_rows(x.as<float>(), nullptr, act.as<uint8_t>(), (int)w.in, (int)w.in, ncols, nullptr));
-        L2B_TRY(launch_kq_gemm(w, act.as<uint8_t>(), ncols, y.as<float>(), (int)w.out, nullptr, m->status, nullptr));
+        DevBuf act, parts;
+        L2B_TRY(dev_alloc(act, gemm_input_bytes(w.in, ncols)));
+        L2B_TRY(dev_alloc(parts, gemm_product_bytes(w, ncols, m->di.sms)));
+        const GemmInput in = gemm_input(act.as<uint8_t>(), w.in, ncols);
+        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(x.as<float>(), nullptr, (int)w.in, ncols, in), nullptr));
+        L2B_TRY(launch_product(w, in, ncols, y.as<float>(), parts.as<float>(), m->di.sms, m->status, nullptr));
     } else {
         for (int c = 0; c < ncols; ++c)
             L2B_TRY(l2b_matrix_matvec_device(m, 0, x.as<float>() + (size_t)c * w.in, y.as<float>() + (size_t)c * w.out, planes, nullptr));

@@ -1,189 +1,339 @@
 // k-quant weights x many activation vectors on the 5th-generation tensor cores (tcgen05): the dense GEMM that prompt
-// prefill and batched matmul! need.  The reference feeds a prompt one token at a time through matmul! (src/matmul.jl:13-23,
-// src/inference.jl:349-356); here 20 tokens share one pass over the weights, with the SAME exact integer arithmetic as the
-// decode path (kquants.cuh): activations as three int8 planes, weights as their stored 4/5-bit integers, s32 accumulation.
+// prefill, batched decode and matmul! over several columns need.  The reference feeds a prompt one token at a time through
+// matmul! (src/matmul.jl:13-23, src/inference.jl:349-356); here up to 128 tokens share one pass over the weights.
 //
-//   Y[t][o] = sum_b ( d_ob * sum_j sc_obj * sum_p dpl_tbp * <q_obj, a_tbpj>  -  dmin_ob * sum_j m_obj * xs_tbj )
+//   Y[t][o] = sum_b ( d_ob * sum_k A_obk * X_tbk  +  sum_j C_obj * xs_tbj )
 //
-// with b the 256-value super-blocks of a row, j its eight 32-value sub-blocks, p the activation planes.
+// b: 256-value super-blocks of a row, j: sub-blocks of 32, xs_tbj: sum of the sub-block's activations.
+//   A = sub-block scale times (quant - centre), centre 8 (q4_K), 16 (q5_K), 32 (q6_K): an integer of at most 11 bits, exact in
+//       fp16 (q6_K: 12 bits, so its scale is cut into an even part and the last bit, two passes).
+//   X = the activations, scaled per token by a power of two, as two fp16 terms (high, low): 24 significant bits, as many as
+//       f32 has.  Products are exact in f32; sums run over 64 values inside the tensor core, which rounds toward zero, and from
+//       there in f32 registers: with sums over 256 values the rounding of the tensor core is what the error consists of.
+//   C = centre * d * scale - dmin * min, the part of the weight that a sub-block's values share, as two fp16 terms.
 //
-// One block = 128 weight rows x 20 tokens, walking the row's super-blocks:
-//   producer warp   one TMA tiled copy (cp.async.bulk.tensor) brings the 128 packed super-blocks of this step (a
-//                   128 x 144/176-byte box of the row-major matrix) and one bulk copy brings the step's activation planes
-//                   (already in the tensor core's operand layout, written by quantise_rows_kernel) plus their scales;
-//   unpack warps    thread r unpacks row r's nibbles (and fifth bits) to bytes into the canonical K-major operand layout
-//                   (8-row x 16-byte core matrices), and decodes the row's 6-bit scales / mins and fp16 d / dmin;
-//   MMA warp        one thread issues eight tcgen05.mma.kind::i8 (M 128, N 64, K 32), one per sub-block, each into its own
-//                   64 columns of tensor memory: 8 x 64 = all 512 columns;
-//   epilogue warps  thread = weight row: tcgen05.ld of the row's s32 dot products, times the sub-block scale (integer),
-//                   then plane scales, d, and the dmin term in f32, accumulated over the super-blocks in registers.
-// The tensor-memory accumulators are handed back to the MMA warp as soon as the integer part of the epilogue has read
-// them, so the next step's MMAs overlap the float part.
+// Work is counted in super-blocks of (128 weight rows x up to 128 tokens): block c takes units c*U .. c*U + U - 1 of the list
+// (tile, super-block), whatever tile they belong to, so that every SM has the same share.  A tile that several blocks share
+// leaves one partial result per block in a buffer of its own (no atomics: the sum's order is fixed); the kernel that reads
+// the product anyway (norm, SwiGLU, RoPE) adds them.
+//
+//   packed-copy warp  one TMA tiled copy (cp.async.bulk.tensor) per super-block: a 128-row box of the stored blocks
+//   operand warp      one bulk copy per 64 values: the tokens' two terms, already in operand layout (split_rows_kernel)
+//   unpack warps      groups of four on steps of 64 values in turn; thread = row: nibbles -> fp16 times scale, into core matrices (8 rows x 16 bytes)
+//   MMA warp          tcgen05.mma.kind::f16 (M 128, K 16), four or eight per 64 values
+//   8 epilogue warps  thread = weight row, half of the tokens: tensor memory -> times d -> f32 accumulators
 //
 // Every mbarrier wait is bounded; a wait that runs out sets the status word, after which the block drains and still frees
 // its tensor memory.
 #pragma once
+#include <cuda_fp16.h>
+
 #include "fused_matvec.cuh"
 #include "tcgen05.cuh"
 
 namespace l2b {
 
-constexpr int GM_ROWS = 128;    // weight rows per block = MMA M
-constexpr int GM_N = 64;        // MMA N: two halves of 32 columns, each 10 tokens x 3 planes + 2 unused columns
-constexpr int GM_TOK = 20;      // tokens per block
-constexpr int GM_HALF_TOK = 10;
-constexpr int GM_STAGES = 3;
-constexpr int GM_B_BYTES = 8 * GM_N * 32;              // activation operand of one super-block: 8 sub-blocks x (64 x 32) int8 = 16 KiB
-constexpr int GM_SCALE_BYTES = 1024;                   // dpl[20][3] + xs[20][8] f32 = 880 bytes, padded
-constexpr int GM_ACT_BYTES = GM_B_BYTES + GM_SCALE_BYTES;  // one (token chunk, super-block) record in global memory
-constexpr int GM_A_TILE = GM_ROWS * 32;                // unpacked weights of one sub-block: 4 KiB
-constexpr int GM_A_BYTES = 8 * GM_A_TILE;              // of one super-block: 32 KiB
-constexpr int GM_EPI_WARPS = 8, GM_UNPACK_WARPS = 4;
-constexpr int GM_THREADS = (GM_EPI_WARPS + 2 + GM_UNPACK_WARPS) * 32;  // warps 0-7 epilogue, 8 producer, 9 MMA, 10-13 unpack
-enum : int { GM_STORE = 0, GM_RESIDUAL = 1 };
+constexpr int GM_ROWS = 128;          // weight rows per tile = MMA M
+constexpr int GM_MAX_TOK = 128;       // tokens per tile
+constexpr int GM_GROUP_BYTES = 2048;  // operand of 8 tokens x 64 values: [term][k / 16][half][8 rows][16 bytes]
+constexpr int GM_XS_BYTES = 256;      // sub-block sums of 8 tokens x one super-block: [term][8 rows][8 sub-blocks] fp16
+constexpr int GM_A_BYTES = GM_ROWS * 64 * 2;
+constexpr int GM_MAX_SEG = 3;         // matrices of one launch
+constexpr int GM_HDRS = 4;
+constexpr int GM_EPI_WARPS = 8;
 
-struct GmRowHdr {  // what the epilogue needs to know about one row's super-block
-    float d, dmin;
-    uint8_t sc[8], m[8];
+// How a product's tiles are shared out; the kernels that read the partial results derive their number from it.
+struct GemmSplit {
+    int U;        // units (super-blocks of a tile) per block
+    int nb;       // units per tile
+    int ntile;    // token tiles
+    int tok;      // tokens per tile (a multiple of 16)
 };
+__host__ __device__ inline int gm_tile(const GemmSplit& s, int row, int tok) { return (row / GM_ROWS) * s.ntile + tok / s.tok; }
+__host__ __device__ inline int gm_parts(const GemmSplit& s, int tile) {
+    const unsigned lo = (unsigned)tile * s.nb;
+    return (int)((lo + s.nb - 1) / s.U - lo / s.U) + 1;
+}
 
+struct GemmSeg {
+    int type, rows, row_tiles;
+    int kb;               // super-blocks per stored column panel (nb when the matrix is not stored as panels)
+    const __half* d6;     // q6_K: block scales [row][nb]
+};
 struct GemmParams {
-    int type;         // T_Q4_K or T_Q5_K
-    int rows;         // weight rows (outputs)
-    int nb;           // super-blocks per row
-    int kb;           // super-blocks per stored column panel (nb when the matrix is not stored as panels)
-    int n_tok;        // activation vectors
-    const uint8_t* act;  // [chunks][nb] records of GM_ACT_BYTES (quantise_rows_kernel)
-    float* y;         // [n_tok][ldy]
-    const float* resid;  // GM_RESIDUAL: y = resid + W x (same indexing as y; may alias it)
+    GemmSeg seg[GM_MAX_SEG];
+    int nseg;
+    GemmSplit sp;
+    int total;            // units
+    int n_tok, groups;    // tokens; groups of 8 in the operand buffers
+    int np;               // slots for packed super-blocks
+    const uint8_t* act;   // [nb][4][groups] x GM_GROUP_BYTES
+    const uint8_t* xs;    // [nb][groups] x GM_XS_BYTES
+    const float* scale;   // [groups * 8] factor of a token's results
+    float* y;             // [part][n_tok][ldy]; the segments' rows follow one another, each starting at a multiple of 128
+    size_t part_stride;
     int ldy;
-    int mode;
     int* status;
+};
+struct GemmMaps {
+    CUtensorMap main[GM_MAX_SEG], tail[GM_MAX_SEG];  // [panels][rows][kb * block bytes]; tail: the last, narrower panel
 };
 
 // ---- shared memory -----------------------------------------------------------------------------
-struct GmSmem {
-    int off_bar, off_tmem, off_hdr, off_au, off_stage, stage_bytes, packed_bytes, total;
+// NT tokens at most per tile.  NS slots for operands and accumulators; as many slots for packed super-blocks as fit (2 .. 5): more tokens
+// need more room per slot (128: 32 KiB of X), fewer tokens need more packed bytes in flight.
+// UG groups of four unpack warps take the steps in turn.  With 128 tokens a step's MMAs take 512 cycles and two groups keep up; with fewer the
+// unpacking is what a step takes, so there are four, and the epilogue's smaller share of the accumulators leaves the registers for them.
+// PAIR: high and low terms are columns of one MMA (half as many instructions, each of which reads the 4 KiB of A again: 32 cycles
+// whatever its columns); with 128 tokens the accumulators would not fit tensor memory.
+template <int NT>
+struct GmCfg {
+    static constexpr int NS = NT == 128 ? 3 : 4;
+    static constexpr int UG = NT == 128 ? 2 : 4;
+    static constexpr bool PAIR = NT != 128;
+    static constexpr int DCOLS = PAIR ? 2 * NT : NT;  // accumulator columns per slot
+    static constexpr int THREADS = (GM_EPI_WARPS + 3 + 4 * UG) * 32;  // warps 0-7 epilogue, 8 packed copies, 9 MMA, 10 operand copies, 11 .. unpack
 };
-__host__ __device__ inline GmSmem gm_smem_layout(int block_bytes) {
+constexpr int GM_MAX_PACKED = 5;
+constexpr int GM_SMEM = 227 * 1024;
+struct GmSmem {
+    int off_bar, off_tmem, off_hdr, off_a, off_b, off_packed, slot_b, slot_packed, total;
+};
+template <int NT>
+__host__ __device__ inline GmSmem gm_smem_layout(int max_block_bytes, int np) {
     GmSmem s;
-    int o = 0;
-    s.off_bar = o;  // full[3] stage_free[3] unpacked[2] mma_done[2] tmem_free[1]
-    o += 16 * 8;
-    s.off_tmem = o;
-    o += 16;
-    o = (o + 127) & ~127;
-    s.off_hdr = o;  // [GM_STAGES][128] GmRowHdr: one set per ring stage, because a stage is refilled only after the epilogue
-                    // of the step that used it has finished (a set per unpack buffer would be rewritten while still being read)
-    o += GM_STAGES * GM_ROWS * (int)sizeof(GmRowHdr);
-    o = (o + 1023) & ~1023;
-    s.off_au = o;   // [2] unpacked weights
-    o += 2 * GM_A_BYTES;
-    s.packed_bytes = (GM_ROWS * block_bytes + 1023) & ~1023;
-    s.stage_bytes = s.packed_bytes + GM_ACT_BYTES;
-    s.off_stage = o;
-    o += GM_STAGES * s.stage_bytes;
-    s.total = o;
+    s.off_bar = 0;  // done[4] ready[4] p_full[5] p_free[5]
+    s.off_tmem = 18 * 8;
+    s.off_hdr = 256;  // [GM_HDRS][128] {d, factor of the shared part}
+    s.off_a = (s.off_hdr + GM_HDRS * GM_ROWS * 8 + 1023) & ~1023;
+    s.off_b = s.off_a + GmCfg<NT>::NS * GM_A_BYTES;
+    s.slot_b = NT * 256;
+    s.off_packed = s.off_b + GmCfg<NT>::NS * s.slot_b;
+    s.slot_packed = (GM_ROWS * max_block_bytes + 1023) & ~1023;
+    s.total = s.off_packed + np * s.slot_packed;
     return s;
 }
 
-// ---- activations: f32 rows -> int8 planes in operand layout --------------------------------------------
-// One block per token.  Optional rmsnorm (src/inference.jl:102-110) as in the decode prologue: planes from gain .* x, 1/rms on
-// the scales.  Record (chunk c = token / 20, super-block b) at act + (c * nb + b) * GM_ACT_BYTES:
-//   bytes  [0, 16384)  B operand: sub-block j at j*2048; value k (0..31) of column n at (k/16)*1024 + (n/8)*128 + (n%8)*16 + k%16;
-//                      column n = 32*(t/10) + 3*(t%10) + plane, t = token % 20
-//   floats [0, 60)     dpl[t][plane];   floats [60, 220) xs[t][j] = sum of the represented activations of sub-block j
-// Columns and tokens that do not exist must read as zero: the caller clears the buffer first.
-struct QuantRowsParams {
-    const float* x;     // [n_tok][ldx]
-    const float* gain;  // rmsnorm gain, or null for none
-    uint8_t* act;
-    int n, ldx, n_tok;
+// ---- activations: f32 rows -> two fp16 terms in operand layout --------------------------------------------
+// One block per token.  Where the values come from:
+//   SR_PLAIN    x[t][i]
+//   SR_RESIDUAL x[t][i] + the product's partial results, stored back to x: the residual update of src/inference.jl:285, :305
+//   SR_SWIGLU   silu(gate) * up of the product's partial results (src/inference.jl:295-299), stored to x
+// then, where `gain` is given, rmsnorm (src/inference.jl:102-110): terms of gain .* x, 1/rms in the token's factor.
+// Value k of a super-block: chunk k / 64, MMA step 2 * (k / 16 % 2) + (k / 32 % 2), half k / 8 % 2, and inside four values the order 0 2 1 3:
+// the order in which the unpack warps meet the nibbles.  Bound by latency (n_tok blocks, two passes over a row held in L2).
+enum : int { SR_PLAIN = 0, SR_RESIDUAL = 1, SR_SWIGLU = 2 };
+struct SplitRowsParams {
+    float* x;            // [n_tok][n]
+    const float* gain;
+    const float* y;      // partial results [part][n_tok][ldy] of the product before
+    size_t part_stride;
+    int ldy, up_row;     // SR_SWIGLU: rows of the up projection begin here
+    GemmSplit sp;
+    int n, n_tok, groups;
+    uint8_t *act, *xs;   // null: only the values are wanted (x)
+    float* scale;
 };
 
-__global__ void __launch_bounds__(512) quantise_rows_kernel(const __grid_constant__ QuantRowsParams p) {
-    __shared__ float s_red[16];
-    __shared__ float s_dpl[8 * 64];    // scratch of quantise_block for the block a warp works on: [warp][8]  (only [0..2] used)
-    __shared__ float s_xs[16 * 16];    // [warp][16]
-    __shared__ __align__(16) uint8_t s_act[16][3][256];
-    const int tok = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int nb = p.n / QK_K;
-    const float* x = p.x + (size_t)tok * p.ldx;
-    float scale = 1.f;
-    if (p.gain) {
-        float ss = 0.f;
-        for (int i = threadIdx.x; i < p.n / 4; i += blockDim.x) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(x) + i);
-            ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
-        }
-        ss = warp_sum(ss);
-        if (lane == 0) s_red[warp] = ss;
-        __syncthreads();
-        float tot = 0.f;
-        for (int i = 0; i < nwarps; ++i) tot += s_red[i];
-        scale = 1.0f / sqrtf(tot / (float)p.n + 1e-5f);
+__device__ __forceinline__ void gm_sum_parts8(const float* y, size_t part_stride, const GemmSplit& sp, int tok, int ldy, int row, float (&v)[8]) {
+    const int parts = gm_parts(sp, gm_tile(sp, row, tok));
+    const float* src = y + (size_t)tok * ldy + row;
+    float4 a = __ldcg(reinterpret_cast<const float4*>(src)), b = __ldcg(reinterpret_cast<const float4*>(src) + 1);
+    for (int p = 1; p < parts; ++p) {
+        const float4* s = reinterpret_cast<const float4*>(src + p * part_stride);
+        const float4 c = __ldcg(s), d = __ldcg(s + 1);
+        a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
+        b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
     }
-    const int c = tok / GM_TOK, t = tok % GM_TOK;
-    const int col0 = 32 * (t / GM_HALF_TOK) + 3 * (t % GM_HALF_TOK);
-    for (int b = warp; b < nb; b += nwarps) {
-        float4 a = __ldcg(reinterpret_cast<const float4*>(x + 256 * b + 8 * lane));
-        float4 bq = __ldcg(reinterpret_cast<const float4*>(x + 256 * b + 8 * lane + 4));
-        if (p.gain) {
-            const float4 ga = __ldg(reinterpret_cast<const float4*>(p.gain + 256 * b + 8 * lane));
-            const float4 gb = __ldg(reinterpret_cast<const float4*>(p.gain + 256 * b + 8 * lane + 4));
-            a.x *= ga.x; a.y *= ga.y; a.z *= ga.z; a.w *= ga.w;
-            bq.x *= gb.x; bq.y *= gb.y; bq.z *= gb.z; bq.w *= gb.w;
-        }
-        // quantise into this warp's scratch (block index 0 of a one-block vector), then scatter into the operand layout
-        quantise_block<3, 8>(a, bq, lane, &s_act[warp][0][0], 256, s_dpl + warp * 8, s_xs + warp * 16, 0);
-        __syncwarp();
-        uint8_t* rec = p.act + ((size_t)c * nb + b) * GM_ACT_BYTES;
-        const int j = lane >> 2, kk = 8 * (lane & 3);  // this lane's 8 values: sub-block j, k = kk .. kk+7
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(512) split_rows_kernel(const __grid_constant__ SplitRowsParams p) {
+    __shared__ float s_sum[16], s_max[16];
+    const int tok = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* x = p.x + (size_t)tok * p.n;
+    float ss = 0.f, mx = 0.f;
+    auto load = [&](int i, float (&v)[8]) {
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldcg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    };
+    for (int i = threadIdx.x; i < p.n / 8; i += blockDim.x) {
+        float v[8];
+        if (MODE == SR_SWIGLU) {
+            float u[8];
+            gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, 8 * i, v);
+            gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, p.up_row + 8 * i, u);
 #pragma unroll
-        for (int pl = 0; pl < 3; ++pl) {
-            const int n = col0 + pl;
-            const uint2 v = *reinterpret_cast<const uint2*>(&s_act[warp][pl][8 * lane]);
-            *reinterpret_cast<uint2*>(rec + j * 2048 + (kk >> 4) * 1024 + (n >> 3) * 128 + (n & 7) * 16 + (kk & 15)) = v;
+            for (int k = 0; k < 8; ++k) v[k] = (v[k] * (1.0f / (1.0f + expf(-v[k])))) * u[k];
+        } else {
+            load(i, v);
+            if (MODE == SR_RESIDUAL) {
+                float u[8];
+                gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, 8 * i, u);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] += u[k];
+            }
         }
-        float* sc = reinterpret_cast<float*>(rec + GM_B_BYTES);
-        if (lane < 3) sc[t * 3 + lane] = s_dpl[warp * 8 + lane] * scale;
-        if (lane < 8) sc[60 + t * 8 + lane] = (s_xs[warp * 16 + 2 * lane] + s_xs[warp * 16 + 2 * lane + 1]) * scale;
-        __syncwarp();
+        if (MODE != SR_PLAIN) {
+            __stcg(reinterpret_cast<float4*>(x) + 2 * i, make_float4(v[0], v[1], v[2], v[3]));
+            __stcg(reinterpret_cast<float4*>(x) + 2 * i + 1, make_float4(v[4], v[5], v[6], v[7]));
+        }
+        if (p.gain) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i + 1);
+            const float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                ss = fmaf(v[k], v[k], ss);
+                mx = fmaxf(mx, fabsf(v[k] * g[k]));
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) mx = fmaxf(mx, fabsf(v[k]));
+        }
+    }
+    if (!p.act) return;
+    ss = warp_sum(ss);
+    mx = warp_max(mx);
+    if (lane == 0) {
+        s_sum[warp] = ss;
+        s_max[warp] = mx;
+    }
+    __syncthreads();
+    ss = 0.f;
+    mx = 0.f;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
+        ss += s_sum[i];
+        mx = fmaxf(mx, s_max[i]);
+    }
+    // power of two that brings the largest value into [2^13, 2^14): a value 2^-16 of the largest still has 24 significant bits in its
+    // two terms, and sums of 32 values, over 32, stay below 2^14 too
+    const int ex = (int)(__float_as_uint(mx) >> 23);
+    const int up = ex == 0 || ex == 255 ? 127 : min(267 - ex, 252);  // 127 + 13 - (ex - 127)
+    const float s = __uint_as_float((uint32_t)up << 23), inv = __uint_as_float((uint32_t)(254 - up) << 23);
+    const float rms = p.gain ? 1.0f / sqrtf(ss / (float)p.n + 1e-5f) : 1.f;
+    if (threadIdx.x == 0) p.scale[tok] = inv * rms;
+    const int group = tok >> 3, row = tok & 7;
+    for (int i = threadIdx.x; i < p.n / 8; i += blockDim.x) {  // p.n / 8 is a multiple of 32: whole warps stay together
+        float v[8];
+        load(i, v);
+        if (p.gain) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i + 1);
+            const float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] *= g[k];
+        }
+        float sum = 0.f;
+        __half h[8], l[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            v[k] *= s;
+            h[k] = __float2half_rn(v[k]);
+            l[k] = __float2half_rn(v[k] - __half2float(h[k]));
+            sum += v[k];
+        }
+        auto pack = [](__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); };
+        const int b = i >> 5, q = i & 31;  // super-block, which eight values of it
+        const int c = q >> 3, step = 2 * ((q >> 1) & 1) + ((q >> 2) & 1), half = q & 1;
+        uint8_t* dst = p.act + ((size_t)(b * 4 + c) * p.groups + group) * GM_GROUP_BYTES + step * 256 + half * 128 + row * 16;
+        *reinterpret_cast<uint4*>(dst) = make_uint4(pack(h[0], h[2]), pack(h[1], h[3]), pack(h[4], h[6]), pack(h[5], h[7]));
+        *reinterpret_cast<uint4*>(dst + 1024) = make_uint4(pack(l[0], l[2]), pack(l[1], l[3]), pack(l[4], l[6]), pack(l[5], l[7]));
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if ((q & 3) == 0) {
+            sum *= 0.03125f;
+            const __half sh = __float2half_rn(sum), sl = __float2half_rn(sum - __half2float(sh));
+            uint8_t* xd = p.xs + ((size_t)b * p.groups + group) * GM_XS_BYTES + row * 16 + (q >> 2) * 2;
+            *reinterpret_cast<__half*>(xd) = sh;
+            *reinterpret_cast<__half*>(xd + 128) = sl;
+        }
     }
 }
 
+// A product that is wanted as such: dst[t][i] = the sum of its partial results.  Grid (blocks per row, n_tok).
+__global__ void sum_parts_kernel(const float* __restrict__ y, size_t part_stride, const __grid_constant__ GemmSplit sp, int ldy, int rows, float* __restrict__ dst) {
+    const int tok = blockIdx.y;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
+        const int parts = gm_parts(sp, gm_tile(sp, i, tok));
+        float v = __ldcg(y + (size_t)tok * ldy + i);
+        for (int p = 1; p < parts; ++p) v += __ldcg(y + p * part_stride + (size_t)tok * ldy + i);
+        dst[(size_t)tok * rows + i] = v;
+    }
+}
+
+// ---- unpacking -------------------------------------------------------------------------------------------
+__device__ __forceinline__ __half2 h2_bits(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t h2_raw(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ __half2 h2_small_int(uint32_t u8) { return __hsub2(h2_bits(u8 * 0x00010001u | 0x64006400u), h2_bits(0x64006400u)); }
+__device__ __forceinline__ float f_small_int(uint32_t u8) { return __uint_as_float(0x4B000000u | u8) - 8388608.f; }
+
+// Quant bits become fp16 numbers where they stand: a field at bits i .. of a 16-bit lane (i + its width <= 10) is the subnormal
+// field * 2^(i - 24), and one fused multiply-add with a power of two times the scale puts it where it belongs: no shifts, no
+// conversions.  Everything is (quant - centre) * scale * 2^-GM_A_EXP, at most 11 significant bits and a multiple of 2^-20: exact.
+// (Shifting the fields into the mantissa of a number in [64, 128) takes 19 instructions per 8 q5_K values, 13 of them on the
+// half-rate integer pipe; this takes 17, 9 of them integer.)
+constexpr int GM_A_EXP = 20;
+struct GmScale {
+    __half2 low, high, off;  // scale * 2^4 (bits 0-3), scale (bits 4-7), -centre * scale * 2^-20
+};
+__device__ __forceinline__ GmScale gm_scale(__half2 S, float centre) {
+    GmScale g;
+    g.low = __hmul2(S, __float2half2_rn(16.f));
+    g.high = S;
+    g.off = __hmul2(S, __float2half2_rn(-centre * 9.5367431640625e-07f));
+    return g;
+}
+// 16 values of one MMA step from the nibbles of q (HIGH: the upper ones); f: words whose bits `top_mask` of every byte stand above the
+// nibble, with the factor `top`.  Pairs are bytes (0, 2) and (1, 3) of a word.
+template <bool HIGH, bool TOP>
+__device__ __forceinline__ void gm_store16(uint8_t* dst, const uint4& q, const uint4& f, uint32_t top_mask, __half2 top, const GmScale& g) {
+    const uint32_t qw[4] = {q.x, q.y, q.z, q.w}, fw[4] = {f.x, f.y, f.z, f.w};
+    const uint32_t m = HIGH ? 0x00F000F0u : 0x000F000Fu;
+    uint32_t o[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const uint32_t w = e ? qw[i] >> 8 : qw[i];
+            __half2 v = __hfma2(h2_bits(w & m), HIGH ? g.high : g.low, g.off);
+            if (TOP) v = __hfma2(h2_bits((e ? fw[i] >> 8 : fw[i]) & top_mask), top, v);
+            o[2 * i + e] = h2_raw(v);
+        }
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(dst + 2048) = make_uint4(o[4], o[5], o[6], o[7]);
+}
+
 // ---- the GEMM ----------------------------------------------------------------------------------------
-// Grid (row tiles, token chunks).  tmap_main: the matrix as [panels][rows][kb * block bytes] (one panel when it is stored row
-// by row); tmap_tail: the last, narrower panel when nb is not a multiple of kb.
-__global__ void __launch_bounds__(GM_THREADS, 1) kq_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ CUtensorMap tmap_main,
-                                                                const __grid_constant__ CUtensorMap tmap_tail) {
+__device__ __forceinline__ int gm_steps(int type) { return type == T_Q6_K ? 8 : 5; }  // operand steps per super-block
+
+template <int NT>
+__global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ GemmMaps maps) {
+    constexpr int NS = GmCfg<NT>::NS, UG = GmCfg<NT>::UG, DCOLS = GmCfg<NT>::DCOLS;
+    constexpr bool PAIR = GmCfg<NT>::PAIR;
+    const int NP = p.np;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the copies and operands want their alignment
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bb = dev_block_bytes(p.type);
-    const GmSmem L = gm_smem_layout(bb);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.off_bar);
-    uint64_t* stage_free = full + GM_STAGES;
-    uint64_t* unpacked = stage_free + GM_STAGES;
-    uint64_t* mma_done = unpacked + 2;
-    uint64_t* tmem_free = mma_done + 2;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (the same for a warp's threads, and known to be)
+    int max_bb = 0;
+    for (int i = 0; i < p.nseg; ++i) max_bb = max(max_bb, dev_block_bytes(p.seg[i].type));
+    const GmSmem L = gm_smem_layout<NT>(max_bb, p.np);
+    uint64_t* done = reinterpret_cast<uint64_t*>(smem + L.off_bar);
+    // ready: weights unpacked, activations landed and the accumulators of the slot's last use read.  One barrier for all three, because the
+    // MMA thread's own instructions bound this kernel: with a barrier each it took 1450 cycles per step of 64 values, whatever the tile.
+    uint64_t *ready = done + 4, *p_full = done + 8, *p_free = done + 13;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.off_tmem);
-    GmRowHdr* hdr = reinterpret_cast<GmRowHdr*>(smem + L.off_hdr);
-    uint8_t* au = smem + L.off_au;
-    uint8_t* stages = smem + L.off_stage;
-    const int row0 = blockIdx.x * GM_ROWS, chunk = blockIdx.y;
-    const int nb = p.nb;
+    float2* hdr = reinterpret_cast<float2*>(smem + L.off_hdr);
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < GM_STAGES; ++i) {
-            mbar_init(full + i, 1);
-            mbar_init(stage_free + i, GM_EPI_WARPS);
+        for (int i = 0; i < NS; ++i) {
+            mbar_init(done + i, 1);
+            mbar_init(ready + i, 4 + 1 + GM_EPI_WARPS);
         }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(unpacked + i, GM_UNPACK_WARPS);
-            mbar_init(mma_done + i, 1);
+        for (int i = 0; i < NP; ++i) {
+            mbar_init(p_full + i, 1);
+            mbar_init(p_free + i, 4 * UG);
         }
-        mbar_init(tmem_free, GM_EPI_WARPS);
         fence_barrier_init();
         fence_proxy_async();
     }
@@ -193,160 +343,342 @@ __global__ void __launch_bounds__(GM_THREADS, 1) kq_gemm_kernel(const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    // the walk over this block's units, the same for every role
+    const int nb = p.sp.nb;
+    const int u0 = blockIdx.x * p.sp.U, u1 = min(u0 + p.sp.U, p.total);
+    struct Where {
+        int seg, row_tile, ntile, b;  // matrix, its row tile, token tile, super-block
+    };
+    auto first_unit = [&]() {
+        Where w;
+        const int tile = u0 / nb;
+        w.b = u0 - tile * nb;
+        w.row_tile = tile / p.sp.ntile;
+        w.ntile = tile - w.row_tile * p.sp.ntile;
+        w.seg = 0;
+        while (w.seg + 1 < p.nseg && w.row_tile >= p.seg[w.seg].row_tiles) w.row_tile -= p.seg[w.seg++].row_tiles;
+        return w;
+    };
+    auto advance = [&](Where& w) {  // (divisions here, once per super-block and role, had cost 2000 cycles of every 5700)
+        if (++w.b < nb) return;
+        w.b = 0;
+        if (++w.ntile < p.sp.ntile) return;
+        w.ntile = 0;
+        if (++w.row_tile < p.seg[w.seg].row_tiles || w.seg + 1 == p.nseg) return;
+        w.row_tile = 0;
+        ++w.seg;
+    };
+    bool ok = true;
+
     if (warp == 8) {
-        // ================= producer: one tiled copy of packed weights + one bulk copy of activations per step =================
+        // ================= packed weights: one tiled copy per super-block =================
         if (lane == 0) {
-            const uint64_t policy = policy_evict_first();
-            const int full_panels = nb / p.kb;
-            bool ok = true;
-            for (int b = 0; b < nb && ok; ++b) {
-                const int s = b % GM_STAGES, use = b / GM_STAGES;
-                if (use > 0 && !mbar_wait_bounded(stage_free + s, (uint32_t)((use - 1) & 1))) {
+            Where w = first_unit();
+            int s = 0;
+            uint32_t parity = 1;  // of the use before
+            for (int u = u0; u < u1; ++u, advance(w)) {
+                if (u - u0 >= NP && !mbar_wait_bounded(p_free + s, parity)) {
                     ok = false;
                     break;
                 }
-                uint8_t* st = stages + (size_t)s * L.stage_bytes;
-                mbar_arrive_expect_tx(full + s, (uint32_t)(GM_ROWS * bb + GM_ACT_BYTES));
-                const int panel = b / p.kb;
-                if (panel < full_panels) tma_load_3d(st, &tmap_main, (b - panel * p.kb) * bb, row0, panel, full + s);
-                else tma_load_3d(st, &tmap_tail, (b - panel * p.kb) * bb, row0, 0, full + s);
-                bulk_g2s(st + L.packed_bytes, p.act + ((size_t)chunk * nb + b) * GM_ACT_BYTES, GM_ACT_BYTES, full + s, policy);
+                const GemmSeg& sg = p.seg[w.seg];
+                const int bb = dev_block_bytes(sg.type), panel = w.b / sg.kb;
+                mbar_arrive_expect_tx(p_full + s, (uint32_t)(GM_ROWS * bb));
+                const bool tail = (panel + 1) * sg.kb > nb;
+                tma_load_3d(smem + L.off_packed + s * L.slot_packed, tail ? &maps.tail[w.seg] : &maps.main[w.seg], (w.b - panel * sg.kb) * bb,
+                            w.row_tile * GM_ROWS, tail ? 0 : panel, p_full + s);
+                if (++s == NP) {
+                    s = 0;
+                    parity ^= 1u;
+                }
             }
             if (!ok) {
                 atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
                 for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // copies in flight land within microseconds
             }
         }
-    } else if (warp == 9) {
-        // ================= MMA issue: eight K = 32 products per step, one per sub-block, into 8 x 64 columns =================
+    } else if (warp == 10) {
+        // ================= activation operands: one bulk copy per 64 values =================
         if (lane == 0) {
-            const uint32_t idesc = umma_idesc_i8(GM_ROWS, GM_N);
-            bool ok = true;
-            for (int b = 0; b < nb && ok; ++b) {
-                const int s = b % GM_STAGES, buf = b & 1;
-                if (!mbar_wait_bounded(unpacked + buf, (uint32_t)((b >> 1) & 1))) ok = false;       // weights unpacked (and the stage has landed)
-                if (ok && b > 0 && !mbar_wait_bounded(tmem_free, (uint32_t)((b - 1) & 1))) ok = false;  // the epilogue has read step b-1
-                if (!ok) break;
-                tc_fence_after();
-                const uint8_t* a_base = au + (size_t)buf * GM_A_BYTES;
-                const uint8_t* b_base = stages + (size_t)s * L.stage_bytes + L.packed_bytes;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    umma_i8(tmem_base + (uint32_t)(j * GM_N), umma_desc(a_base + j * GM_A_TILE, 16 * 128, 128), umma_desc(b_base + j * 2048, 8 * 128, 128),
-                            idesc, 0u);
-                umma_commit(mma_done + buf);
-            }
-            if (!ok) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
-        }
-    } else if (warp >= 10) {
-        // ================= unpack: thread r turns row r's packed quants into bytes in operand layout =================
-        const int r = threadIdx.x - 10 * 32;  // 0..127
-        bool ok = true;
-        for (int b = 0; b < nb; ++b) {
-            const int s = b % GM_STAGES, buf = b & 1;
-            if (ok && b >= 2 && !mbar_wait_bounded(mma_done + buf, (uint32_t)(((b - 2) >> 1) & 1))) ok = false;  // the MMAs of step b-2 have read this buffer
-            if (ok && !mbar_wait_bounded(full + s, (uint32_t)((b / GM_STAGES) & 1))) ok = false;
-            if (ok) {
-                const uint8_t* blk = stages + (size_t)s * L.stage_bytes + (size_t)r * bb;
-                const uint4 h = *reinterpret_cast<const uint4*>(blk);
-                uint64_t sc8, m8;
-                decode_scales_k4(h, sc8, m8);
-                GmRowHdr hd;
-                hd.d = half_bits_to_float(h.x & 0xFFFFu);
-                hd.dmin = half_bits_to_float(h.x >> 16);
-                *reinterpret_cast<uint64_t*>(hd.sc) = sc8;
-                *reinterpret_cast<uint64_t*>(hd.m) = m8;
-                hdr[s * GM_ROWS + r] = hd;
-                uint8_t* dst = au + (size_t)buf * GM_A_BYTES + (r >> 3) * 128 + (r & 7) * 16;
-                const uint8_t* qs = blk + (p.type == T_Q5_K ? 48 : 16);
-                uint4 qh0 = make_uint4(0u, 0u, 0u, 0u), qh1 = qh0;
-                if (p.type == T_Q5_K) {  // fifth bits of values l = 0..15 and 16..31 of every sub-block: bit j of byte qh[l]
-                    qh0 = *reinterpret_cast<const uint4*>(blk + 16);
-                    qh1 = *reinterpret_cast<const uint4*>(blk + 32);
-                }
-#pragma unroll
-                for (int pr = 0; pr < 4; ++pr) {
-#pragma unroll
-                    for (int hh = 0; hh < 2; ++hh) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(qs + 32 * pr + 16 * hh);
-                        const uint4 q5 = hh ? qh1 : qh0;
-                        uint4 lo, hi;
-                        lo.x = (v.x & 0x0f0f0f0fu) | (((q5.x >> (2 * pr)) & 0x01010101u) << 4);
-                        lo.y = (v.y & 0x0f0f0f0fu) | (((q5.y >> (2 * pr)) & 0x01010101u) << 4);
-                        lo.z = (v.z & 0x0f0f0f0fu) | (((q5.z >> (2 * pr)) & 0x01010101u) << 4);
-                        lo.w = (v.w & 0x0f0f0f0fu) | (((q5.w >> (2 * pr)) & 0x01010101u) << 4);
-                        hi.x = ((v.x >> 4) & 0x0f0f0f0fu) | (((q5.x >> (2 * pr + 1)) & 0x01010101u) << 4);
-                        hi.y = ((v.y >> 4) & 0x0f0f0f0fu) | (((q5.y >> (2 * pr + 1)) & 0x01010101u) << 4);
-                        hi.z = ((v.z >> 4) & 0x0f0f0f0fu) | (((q5.z >> (2 * pr + 1)) & 0x01010101u) << 4);
-                        hi.w = ((v.w >> 4) & 0x0f0f0f0fu) | (((q5.w >> (2 * pr + 1)) & 0x01010101u) << 4);
-                        *reinterpret_cast<uint4*>(dst + (2 * pr) * GM_A_TILE + hh * (16 * 128)) = lo;      // sub-block 2*pr, values 16*hh ..
-                        *reinterpret_cast<uint4*>(dst + (2 * pr + 1) * GM_A_TILE + hh * (16 * 128)) = hi;  // sub-block 2*pr + 1
+            Where w = first_unit();
+            int s = 0;
+            bool first = true;
+            uint32_t parity = 1;
+            for (int u = u0; u < u1 && ok; ++u, advance(w)) {
+                const int steps = gm_steps(p.seg[w.seg].type), g0 = (w.ntile * p.sp.tok) >> 3, ng = min(p.sp.tok >> 3, p.groups - g0);
+                for (int k = 0; k < steps; ++k) {
+                    if (!first && !mbar_wait_bounded(done + s, parity)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* dst = smem + L.off_b + s * L.slot_b;
+                    const bool shared_part = steps == 5 && k == 4;
+                    const uint32_t bytes = (uint32_t)(ng * (shared_part ? GM_XS_BYTES : GM_GROUP_BYTES));
+                    mbar_arrive_expect_tx(ready + s, bytes);
+                    if (shared_part) bulk_g2s_plain(dst, p.xs + ((size_t)w.b * p.groups + g0) * GM_XS_BYTES, bytes, ready + s);
+                    else bulk_g2s_plain(dst, p.act + ((size_t)(w.b * 4 + (k & 3)) * p.groups + g0) * GM_GROUP_BYTES, bytes, ready + s);
+                    if (++s == NS) {
+                        s = 0;
+                        first = false;
+                        parity ^= 1u;
                     }
                 }
+            }
+            if (!ok) {
+                atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
+                for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+            }
+        }
+    } else if (warp == 9) {
+        // ================= MMA issue: the whole warp walks along, one thread issues =================
+        const uint32_t idesc = umma_idesc_f16(GM_ROWS, PAIR ? 2 * p.sp.tok : p.sp.tok), idesc_xs = umma_idesc_f16(GM_ROWS, p.sp.tok);
+        // operand descriptors of slot 0; the others lie a multiple of 16 bytes further
+        const uint64_t desc_a = umma_desc(smem + L.off_a, 2048, 128), desc_b = umma_desc(smem + L.off_b, 128, PAIR ? GM_GROUP_BYTES / 2 : GM_GROUP_BYTES);
+        const uint64_t desc_xs = umma_desc(smem + L.off_b, 128, GM_XS_BYTES);
+        Where w = first_unit();
+        int s = 0;
+        uint32_t parity = 0;
+        for (int u = u0; u < u1 && ok; ++u, advance(w)) {
+            const int steps = gm_steps(p.seg[w.seg].type);
+            for (int k = 0; k < steps; ++k) {
+                if (!mbar_wait_bounded(ready + s, parity)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d = tmem_base + (uint32_t)(s * DCOLS);
+                const uint64_t da = desc_a + (uint64_t)(s * (GM_A_BYTES >> 4));
+                const bool shared_part = steps == 5 && k == 4;
+                if (elect_one()) {
+                    if (shared_part) {
+                        const uint64_t dx = desc_xs + (uint64_t)(s * (L.slot_b >> 4));
+                        umma_f16(d, da + (4096 >> 4), dx, idesc_xs, 0u);  // low terms of C first
+                        umma_f16(d, da, dx, idesc_xs, 1u);
+                    } else {
+                        const uint64_t db = desc_b + (uint64_t)(s * (L.slot_b >> 4));
+#pragma unroll
+                        for (int t = PAIR ? 0 : 1; t >= 0; --t)  // low terms of X first
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk)
+                                umma_f16(d, da + (uint64_t)(kk * (4096 >> 4)), db + (uint64_t)((t * 1024 + kk * 256) >> 4), idesc, t == (PAIR ? 0 : 1) && kk == 0 ? 0u : 1u);
+                    }
+                    umma_commit(done + s);
+                }
+                __syncwarp();
+                if (++s == NS) {
+                    s = 0;
+                    parity ^= 1u;
+                }
+            }
+        }
+        if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
+    } else if (warp > 10) {
+        // ================= unpack: groups of four warps take the steps in turn; thread = row =================
+        const int id = threadIdx.x - 11 * 32, r = id & 127, group = (warp - 11) >> 2;
+        const int row_off = (r >> 3) * 128 + (r & 7) * 16;
+        auto q6_scale = [&](const Where& w) -> float {
+            const GemmSeg& sg = p.seg[w.seg];
+            const int row = w.row_tile * GM_ROWS + r;
+            return sg.type == T_Q6_K && row < sg.rows ? __half2float(__ldg(sg.d6 + (size_t)row * nb + w.b)) : 0.f;
+        };
+        Where w = first_unit();
+        float d6_next = u0 < u1 ? q6_scale(w) : 0.f;
+        int s = 0, turn = 0, ps = 0, hs = 0;  // slot, whose turn it is, packed slot, set of factors
+        bool first = true;
+        uint32_t parity = 1, p_parity = 0;
+        for (int u = u0; u < u1 && ok; ++u) {
+            const GemmSeg& sg = p.seg[w.seg];
+            const int bb = dev_block_bytes(sg.type);
+            const float d6 = d6_next;
+            advance(w);
+            if (u + 1 < u1) d6_next = q6_scale(w);  // a super-block ahead: the latency of a global read
+            if (!mbar_wait_bounded(p_full + ps, p_parity)) {
+                ok = false;
+                break;
+            }
+            const uint8_t* blk = smem + L.off_packed + ps * L.slot_packed + r * bb;
+            const int steps = gm_steps(sg.type);
+            uint64_t sc8 = 0, m8 = 0;
+            uint4 top0 = make_uint4(0u, 0u, 0u, 0u), top1 = top0;  // q5_K: fifth bits; q6_K: scales
+            float d = d6, dmin = 0.f, s_up = 1.f, s_dn = 1.f;
+            if (sg.type != T_Q6_K) {
+                const uint4 h = *reinterpret_cast<const uint4*>(blk);
+                decode_scales_k4(h, sc8, m8);
+                d = half_bits_to_float(h.x & 0xFFFFu);
+                dmin = half_bits_to_float(h.x >> 16);
+                if (sg.type == T_Q5_K) {
+                    top0 = *reinterpret_cast<const uint4*>(blk + 16);
+                    top1 = *reinterpret_cast<const uint4*>(blk + 32);
+                }
+                // power of two that keeps the shared part C and its second term inside the range of fp16
+                const int ex = (int)(__float_as_uint(fmaxf(fabsf(d) * 1024.f, fabsf(dmin) * 64.f)) >> 23);
+                if (ex != 0 && ex < 254) {
+                    s_up = __uint_as_float((uint32_t)(254 - ex) << 23);
+                    s_dn = __uint_as_float((uint32_t)ex << 23);
+                }
+            } else {
+                top0 = *reinterpret_cast<const uint4*>(blk + 192);
+            }
+            const float cen = sg.type == T_Q5_K ? 16.f : 8.f;
+            for (int k = 0; k < steps; ++k) {
+                const int slot = s;
+                const bool mine = turn == group, reused = !first;
+                const uint32_t use_parity = parity;
+                if (++turn == UG) turn = 0;
+                if (++s == NS) {
+                    s = 0;
+                    first = false;
+                    parity ^= 1u;
+                }
+                if (!mine) continue;
+                if (reused && !mbar_wait_bounded(done + slot, use_parity)) {
+                    ok = false;
+                    break;
+                }
+                // (the epilogue may still be at the super-block before the last one: four sets of factors are enough)
+                if (k == 0) hdr[hs * GM_ROWS + r] = make_float2(d * (float)(1 << GM_A_EXP), 32.f * s_dn);
+                uint8_t* dst = smem + L.off_a + slot * GM_A_BYTES + row_off;
+                if (sg.type == T_Q6_K) {
+                    const int c = k & 3, hh = c >> 1, odd = c & 1;
+                    const uint32_t scw = c == 0 ? top0.x : c == 1 ? top0.y : c == 2 ? top0.z : top0.w;
+#pragma unroll
+                    for (int part = 0; part < 2; ++part) {
+                        const uint4 f = *reinterpret_cast<const uint4*>(blk + 128 + 32 * hh + 16 * part);
+#pragma unroll
+                        for (int hi = 0; hi < 2; ++hi) {
+                            const int sc = (int)(int8_t)(scw >> (8 * (2 * hi + part)));
+                            const __half2 S = __half2half2(__int2half_rn(k < 4 ? sc - (sc & 1) : (sc & 1)));
+                            const GmScale g = gm_scale(S, 32.f);
+                            const uint4 q = *reinterpret_cast<const uint4*>(blk + 64 * hh + 32 * hi + 16 * part);
+                            const int idx = 2 * odd + hi;  // which two bits of the byte: value 16 at bit 2 * idx
+                            const __half2 up = __hmul2(S, h2_bits(((uint32_t)(23 - 2 * idx) << 10) * 0x00010001u));  // 2^(8 - 2 idx)
+                            if (odd) gm_store16<true, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
+                            else gm_store16<false, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
+                        }
+                    }
+                } else if (k < 4) {
+                    const uint32_t two = (uint32_t)(sc8 >> (16 * k));
+                    const GmScale g0 = gm_scale(h2_small_int(two & 0xFFu), cen), g1 = gm_scale(h2_small_int((two >> 8) & 0xFFu), cen);
+                    if (sg.type == T_Q5_K) {  // the fifth bit of sub-block j is bit j: value 16 from 2^(j - 24) takes 2^(8 - j)
+                        const uint32_t p0 = (uint32_t)(23 - 2 * k) << 10;
+                        const __half2 up0 = __hmul2(g0.high, h2_bits(p0 * 0x00010001u)), up1 = __hmul2(g1.high, h2_bits((p0 - 1024u) * 0x00010001u));
+                        const uint32_t bit = 0x00010001u << (2 * k);
+#pragma unroll
+                        for (int part = 0; part < 2; ++part) {
+                            const uint4 q = *reinterpret_cast<const uint4*>(blk + 48 + 32 * k + 16 * part);
+                            gm_store16<false, true>(dst + 2 * part * 4096, q, part ? top1 : top0, bit, up0, g0);
+                            gm_store16<true, true>(dst + (2 * part + 1) * 4096, q, part ? top1 : top0, bit << 1, up1, g1);
+                        }
+                    } else {
+#pragma unroll
+                        for (int part = 0; part < 2; ++part) {
+                            const uint4 q = *reinterpret_cast<const uint4*>(blk + 16 + 32 * k + 16 * part);
+                            gm_store16<false, false>(dst + 2 * part * 4096, q, q, 0u, g0.high, g0);
+                            gm_store16<true, false>(dst + (2 * part + 1) * 4096, q, q, 0u, g1.high, g1);
+                        }
+                    }
+                } else {
+                    uint32_t o[4], o2[4];
+#pragma unroll
+                    for (int j2 = 0; j2 < 4; ++j2) {
+                        float f2[2];
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const int j = 2 * j2 + e;
+                            const float sc = f_small_int((uint32_t)byte64(sc8, j)), m = f_small_int((uint32_t)byte64(m8, j));
+                            f2[e] = fmaf(-dmin, m, d * cen * sc) * s_up;
+                        }
+                        const __half2 hi = __floats2half2_rn(f2[0], f2[1]);
+                        const float2 back = __half22float2(hi);
+                        o[j2] = h2_raw(hi);
+                        o2[j2] = h2_raw(__floats2half2_rn(f2[0] - back.x, f2[1] - back.y));
+                    }
+                    const uint4 v = make_uint4(o[0], o[1], o[2], o[3]), v2 = make_uint4(o2[0], o2[1], o2[2], o2[3]);
+                    *reinterpret_cast<uint4*>(dst) = v;  // each term times the high and the low terms of the sums
+                    *reinterpret_cast<uint4*>(dst + 2048) = v;
+                    *reinterpret_cast<uint4*>(dst + 4096) = v2;
+                    *reinterpret_cast<uint4*>(dst + 4096 + 2048) = v2;
+                }
                 fence_proxy_async();  // the tensor core reads shared memory through the asynchronous proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ready + slot);
             }
             __syncwarp();
-            if (lane == 0 && ok) mbar_arrive(unpacked + buf);
+            if (lane == 0 && ok) mbar_arrive(p_free + ps);
+            hs = (hs + 1) % GM_HDRS;
+            if (++ps == NP) {
+                ps = 0;
+                p_parity ^= 1u;
+            }
         }
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
     } else {
         // ================= epilogue: thread = weight row; warps e and e + 4 split the tokens =================
+        constexpr int NH = NT / 2;
         const int q = warp & 3, half = warp >> 2;
         const int r = 32 * q + lane;
-        const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * half);
-        float acc[GM_HALF_TOK];
+        const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16);
+        float acc[NH];
 #pragma unroll
-        for (int t = 0; t < GM_HALF_TOK; ++t) acc[t] = 0.f;
-        bool ok = true;
-        for (int b = 0; b < nb; ++b) {
-            const int s = b % GM_STAGES, buf = b & 1;
-            if (ok && !mbar_wait_bounded(mma_done + buf, (uint32_t)((b >> 1) & 1))) ok = false;
-            if (ok) {
+        for (int t = 0; t < NH; ++t) acc[t] = 0.f;
+        if (lane < NS) mbar_arrive(ready + lane);  // no accumulators to wait for at first
+        Where w = first_unit();
+        int s = 0, hs = 0;
+        uint32_t parity = 0;
+        for (int u = u0; u < u1 && ok; ++u, advance(w)) {
+            const int steps = gm_steps(p.seg[w.seg].type);
+            float2 f = make_float2(0.f, 0.f);
+            for (int k = 0; k < steps; ++k) {
+                if (!mbar_wait_bounded(done + s, parity)) {
+                    ok = false;
+                    break;
+                }
                 tc_fence_after();
-                const GmRowHdr hd = hdr[s * GM_ROWS + r];
-                int S[3 * GM_HALF_TOK];
+                if (k == 0) f = hdr[hs * GM_ROWS + r];
+                const bool shared_part = steps == 5 && k == 4;
+                const float m = shared_part ? f.y : f.x;
+                if (PAIR && !shared_part) {  // columns in eights: high terms of eight tokens, then their low terms
 #pragma unroll
-                for (int n = 0; n < 3 * GM_HALF_TOK; ++n) S[n] = 0;
+                    for (int c0 = 0; c0 < NH; c0 += 8) {
+                        float v[16];
+                        tmem_ld16f(taddr + (uint32_t)(s * DCOLS + 2 * (NH * half + c0)), v);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    int c[32];
-                    tmem_ld32(taddr + (uint32_t)(j * GM_N), c);
-                    const int sc = hd.sc[j];
+                        for (int t = 0; t < 8; ++t) acc[c0 + t] = fmaf(m, v[t] + v[8 + t], acc[c0 + t]);
+                    }
+                } else {
 #pragma unroll
-                    for (int n = 0; n < 3 * GM_HALF_TOK; ++n) S[n] += sc * c[n];
+                    for (int c0 = 0; c0 < NH; c0 += 16) {
+                        float v[16];
+                        tmem_ld16f(taddr + (uint32_t)(s * DCOLS + NH * half + c0), v);
+#pragma unroll
+                        for (int t = 0; t < 16; ++t) acc[c0 + t] = fmaf(m, v[t], acc[c0 + t]);
+                    }
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(tmem_free);  // the accumulators may be overwritten by the next step
-                const float* scl = reinterpret_cast<const float*>(stages + (size_t)s * L.stage_bytes + L.packed_bytes + GM_B_BYTES);
-                float mf[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) mf[j] = (float)hd.m[j];
-#pragma unroll
-                for (int t = 0; t < GM_HALF_TOK; ++t) {
-                    const int tt = GM_HALF_TOK * half + t;
-                    const float f = fmaf(scl[tt * 3], (float)S[3 * t], fmaf(scl[tt * 3 + 1], (float)S[3 * t + 1], scl[tt * 3 + 2] * (float)S[3 * t + 2]));
-                    float mt = 0.f;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) mt = fmaf(mf[j], scl[60 + tt * 8 + j], mt);
-                    acc[t] += hd.d * f - hd.dmin * mt;
+                if (lane == 0) mbar_arrive(ready + s);
+                if (++s == NS) {
+                    s = 0;
+                    parity ^= 1u;
                 }
             }
-            __syncwarp();
-            if (lane == 0 && ok) mbar_arrive(stage_free + s);
+            hs = (hs + 1) % GM_HDRS;
+            if (ok && (w.b == nb - 1 || u == u1 - 1)) {  // this block's part of the tile is complete
+                const int tile = u / nb;
+                const int first = tile * nb / p.sp.U;
+                int row = w.row_tile * GM_ROWS + r;
+                const bool valid = row < p.seg[w.seg].rows;
+                for (int e = 0; e < w.seg; ++e) row += p.seg[e].row_tiles * GM_ROWS;
+                float* dst = p.y + (size_t)(blockIdx.x - first) * p.part_stride + row;
+#pragma unroll
+                for (int t = 0; t < NH; ++t) {
+                    const int tt = NH * half + t, tok = w.ntile * p.sp.tok + tt;
+                    if (valid && tt < p.sp.tok && tok < p.n_tok) dst[(size_t)tok * p.ldy] = acc[t] * __ldg(p.scale + tok);
+                    acc[t] = 0.f;
+                }
+            }
         }
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
-        const int row = row0 + r;
-        if (ok && row < p.rows) {
-#pragma unroll
-            for (int t = 0; t < GM_HALF_TOK; ++t) {
-                const int tok = chunk * GM_TOK + GM_HALF_TOK * half + t;
-                if (tok < p.n_tok) {
-                    const size_t o = (size_t)tok * p.ldy + row;
-                    p.y[o] = p.mode == GM_RESIDUAL ? p.resid[o] + acc[t] : acc[t];
-                }
-            }
-        }
     }
     // every path ends here; the tensor memory is freed by the warp that allocated it
     tc_fence_before();

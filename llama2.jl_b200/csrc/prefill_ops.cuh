@@ -1,8 +1,8 @@
 // Element-wise kernels of the many-token prompt pass (the tensor-core GEMM of kq_gemm.cuh does the matrix products):
-// embedding rows, RoPE + KV-cache write, SwiGLU, bookkeeping of the loop state.  Each restates, for T tokens at once, what
+// embedding rows, RoPE + KV-cache write, bookkeeping of the loop state.  Each restates, for T tokens at once, what
 // the fused epilogues of the decode path do for one (src/inference.jl:236, 251-260, 295-299, 354-356).
 #pragma once
-#include "fused_matvec.cuh"
+#include "kq_gemm.cuh"
 
 namespace l2b {
 
@@ -27,12 +27,14 @@ __global__ void embed_rows_kernel(int type, const uint8_t* __restrict__ table, c
 }
 
 // rope!(q), rope!(k) at positions pos0 + t and the cache writes key_cache[:, :, pos] = k, value_cache[pos, :, :] = v
-// (src/inference.jl:251-260) for T tokens.  q [T][q_dim] is rotated in place; k, v [T][kv_dim] go to the caches
-// [kv_head][seq_len][hs].  The rotation multiplies exactly as the decode epilogue does (separately rounded products).
+// (src/inference.jl:251-260) for T tokens.  The projections are the partial results of one product (rows of q, then k, then v);
+// the rotated queries go to q [T][q_dim], keys and values to the caches [kv_head][seq_len][hs].  The rotation multiplies exactly as the decode epilogue does (separately rounded products).
 struct RopeKvParams {
+    const float* y;        // [part][T][ldy]
+    size_t part_stride;
+    int ldy, k_row, v_row; // rows of k and v begin here
+    GemmSplit sp;
     float* q;
-    const float* k;
-    const float* v;
     float* kc;
     float* vc;
     const float* rope_cs;  // [seq_len][hs/2] (cos, sin)
@@ -44,6 +46,13 @@ __global__ void rope_kv_kernel(const __grid_constant__ RopeKvParams p) {
     const int t = blockIdx.y, pos = p.pos_list ? __ldg(p.pos_list + t) : p.pos0 + t;
     float* const kc = p.kc + (p.pos_list ? (size_t)t * p.cache_stride : 0);
     float* const vc = p.vc + (p.pos_list ? (size_t)t * p.cache_stride : 0);
+    auto sum = [&](int row) {
+        const int parts = gm_parts(p.sp, gm_tile(p.sp, row, t));
+        const float* src = p.y + (size_t)t * p.ldy + row;
+        float v = __ldcg(src);
+        for (int i = 1; i < parts; ++i) v += __ldcg(src + i * p.part_stride);
+        return v;
+    };
     const int h2 = p.hs >> 1;
     const int qp = p.q_dim >> 1, kp = p.kv_dim >> 1;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < qp + kp + p.kv_dim; i += gridDim.x * blockDim.x) {
@@ -53,8 +62,7 @@ __global__ void rope_kv_kernel(const __grid_constant__ RopeKvParams p) {
             const int head = pr / h2, f = pr - head * h2;
             const int ia = head * p.hs + (p.neox ? f : 2 * f), ib = p.neox ? ia + h2 : ia + 1;
             const float2 cs = __ldg(reinterpret_cast<const float2*>(p.rope_cs) + (size_t)pos * h2 + f);
-            const float* src = is_q ? p.q + (size_t)t * p.q_dim : p.k + (size_t)t * p.kv_dim;
-            const float vA = src[ia], vB = src[ib];
+            const float vA = sum(ia + (is_q ? 0 : p.k_row)), vB = sum(ib + (is_q ? 0 : p.k_row));
             const float oa = __fsub_rn(__fmul_rn(vA, cs.x), __fmul_rn(vB, cs.y));
             const float ob = __fadd_rn(__fmul_rn(vA, cs.y), __fmul_rn(vB, cs.x));
             if (is_q) {
@@ -68,16 +76,8 @@ __global__ void rope_kv_kernel(const __grid_constant__ RopeKvParams p) {
         } else {
             const int e = i - qp - kp;
             const int head = e / p.hs;
-            vc[((size_t)head * p.seq_len + pos) * p.hs + (e - head * p.hs)] = p.v[(size_t)t * p.kv_dim + e];
+            vc[((size_t)head * p.seq_len + pos) * p.hs + (e - head * p.hs)] = sum(p.v_row + e);
         }
-    }
-}
-
-// hb = silu(hb) .* hb2 (src/inference.jl:295-299) over T x hidden values, in place in g.
-__global__ void swiglu_rows_kernel(float* __restrict__ g, const float* __restrict__ u, size_t n) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float v = g[i];
-        g[i] = (v * (1.0f / (1.0f + expf(-v)))) * u[i];
     }
 }
 

@@ -23,15 +23,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// D[tmem] = A[smem] * B[smem] (accumulate = 0: overwrite), u8 x s8 -> s32
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -58,9 +49,13 @@ __device__ __forceinline__ uint64_t umma_desc(const void* smem_ptr, uint32_t lbo
     d |= (uint64_t)1 << 46;  // descriptor version of this architecture
     return d;                // base offset 0, layout type 0 (no swizzle)
 }
-// Instruction descriptor: s32 accumulators, A unsigned 8-bit, B signed 8-bit, both K-major, N and M as given.
-__host__ __device__ constexpr uint32_t umma_idesc_i8(int M, int N) {
-    return (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// Instruction descriptor: f32 accumulators, A and B fp16, both K-major.
+__host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N) { return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24); }
+// One thread of a warp whose threads are all here.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t yes;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+    return yes != 0;
 }
 
 // ---- bf16 operands ---------------------------------------------------------------------------------
@@ -70,14 +65,17 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
                  "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], bf16 x bf16 -> f32
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[smem] * B[smem], both fp16 or both bf16 (as the instruction descriptor says) -> f32
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
+}
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    umma_f16(tmem_d, desc_a, desc_b, idesc, accumulate);
 }
 // Shared-memory matrix descriptor of a K-major operand tile of 64 bf16 (128 bytes) per row, 128-byte swizzle as TMA writes it:
 // groups of 8 rows are 1024 bytes apart.  The tile starts on a 1024-byte boundary; 16 values further along K are 32 bytes.
@@ -117,6 +115,19 @@ __device__ __forceinline__ float tmem_ld1f(uint32_t taddr) {
 __device__ __forceinline__ void tmem_st1f(uint32_t taddr, float v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "f"(v) : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// 16 consecutive columns of this thread's tensor-memory lane
+__device__ __forceinline__ void tmem_ld16f(uint32_t taddr, float (&v)[16]) {
+    int r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __int_as_float(r[i]);
 }
 // 32 consecutive columns of this thread's tensor-memory lane: load and store
 __device__ __forceinline__ void tmem_ld32f(uint32_t taddr, float (&v)[32]) {
