@@ -9,7 +9,7 @@ from concurrent.futures import ThreadPoolExecutor
 _HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = ["csrc/api.cu", "csrc/stack.cu", "csrc/stack_config.cpp", "csrc/safetensors.cpp", "csrc/gguf_reader.cpp", "csrc/tokenizer.cpp"]
 HEADERS = ["csrc/common.cuh", "csrc/kquants.cuh", "csrc/fused_matvec.cuh", "csrc/attention.cuh", "csrc/sampling.cuh",
-           "csrc/small_ops.cuh", "csrc/token_kernel.cuh", "csrc/kq_gemm.cuh", "csrc/prefill_ops.cuh", "csrc/gguf_reader.h", "csrc/host_common.h",
+           "csrc/small_ops.cuh", "csrc/token_kernel.cuh", "csrc/kq_gemm.cuh", "csrc/prefill_ops.cuh", "csrc/prompt_attention.cuh", "csrc/gguf_reader.h", "csrc/host_common.h",
            "csrc/tcgen05.cuh", "csrc/json.h", "csrc/safetensors.h", "csrc/stack_config.h", "csrc/stack.h", "csrc/dense_ops.cuh",
            "csrc/dense_matvec.cuh", "csrc/dense_gemm.cuh", "csrc/stack_rows.cuh", "csrc/cache_scan.cuh", "csrc/latent_attention.cuh",
            "csrc/head_attention.cuh", "csrc/head_prefill.cuh", "csrc/mlstm.cuh", "csrc/mlstm_prefill.cuh", "csrc/latent_prefill.cuh",

@@ -21,6 +21,7 @@
 #include "small_ops.cuh"
 #include "kq_gemm.cuh"
 #include "prefill_ops.cuh"
+#include "prompt_attention.cuh"
 #include "token_kernel.cuh"
 
 using namespace l2b;
@@ -304,6 +305,10 @@ static void set_kernel_attrs() {
         set((const void*)kq_gemm_kernel<32>);
         set((const void*)kq_gemm_kernel<64>);
         set((const void*)kq_gemm_kernel<128>);
+        set((const void*)prompt_attention_kernel<1>);
+        set((const void*)prompt_attention_kernel<2>);
+        set((const void*)prompt_attention_kernel<4>);
+        set((const void*)prompt_attention_kernel<8>);
         set((const void*)token_kernel<1>);
         set((const void*)token_kernel<2>);
         set((const void*)token_kernel<3>);
@@ -1863,6 +1868,22 @@ constexpr int PF_MIN_TOK = 12;
 constexpr int BATCH_MAX_SEQ = 240;
 constexpr int STACK_MIN_ROWS = 2;  // layer-stack models
 
+// Attention of one sequence's tokens at pos0 ..: heads of a multiple of 16 values, at most 128, take the tensor-core kernel.
+static bool prompt_attention_supported(int hs) { return hs % 16 == 0 && hs <= PA_MAX_HS; }
+static int32_t launch_prompt_attention(const PromptAttnParams& a, int gq, cudaStream_t st) {
+    const size_t smem = (size_t)pa_smem_layout(a.hs).total + 1024;
+    const int tq = PA_ROWS / gq;
+    const dim3 grid((a.n + tq - 1) / tq, a.n_heads / gq);
+    switch (gq) {
+        case 8: prompt_attention_kernel<8><<<grid, PA_THREADS, smem, st>>>(a); break;
+        case 4: prompt_attention_kernel<4><<<grid, PA_THREADS, smem, st>>>(a); break;
+        case 2: prompt_attention_kernel<2><<<grid, PA_THREADS, smem, st>>>(a); break;
+        default: prompt_attention_kernel<1><<<grid, PA_THREADS, smem, st>>>(a); break;
+    }
+    CU(cudaGetLastError());
+    return L2B_OK;
+}
+
 // Every layer for n tokens whose residual-stream rows are in B.x.  One sequence: token t sits at position pos0 + t and the
 // layer's caches are kc / vc + l * layer_stride.  Batched decode (pos_list non-null): token t is the next position pos_list[t]
 // of sequence t, whose caches lie seq_stride * t further.
@@ -1906,17 +1927,24 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
         r.pos_list = pos_list; r.cache_stride = seq_stride;
         rope_kv_kernel<<<dim3(8, n), 256, 0, st>>>(r);
         CU(cudaGetLastError());
-        AttnParams a;
-        memset(&a, 0, sizeof(a));
-        a.q = B.q; a.kc = kcl; a.vc = vcl; a.out = B.att; a.tickets = B.tickets;
-        a.part_m = B.pm; a.part_l = B.pl; a.part_acc = B.pacc;
-        a.pos = nullptr; a.pos_base = pos0; a.pos_list = pos_list; a.cache_stride_q = seq_stride;
-        a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.hs = hs; a.seq_len = c.seq_len; a.nsplit = B.nsplit;
-        a.nq = std::max(n, 2);  // (a one-token pass takes the many-query form of the kernel too: the second query copy leaves at once)
-        a.q_stride = c.dim;
-        a.min_chunk = 256;  // many queries already fill the GPU: split a query's positions only when there are many
-        if (n < 2) return fail(L2B_ERR_BAD_ARG, "a many-token pass needs at least two tokens");
-        CU(launch_attention(a, gq, st, false));
+        if (!pos_list && prompt_attention_supported(hs)) {
+            PromptAttnParams a;
+            a.q = B.q; a.kc = kcl; a.vc = vcl; a.out = B.att; a.n = n; a.pos0 = pos0; a.q_stride = c.dim;
+            a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.hs = hs; a.seq_len = c.seq_len; a.status = status;
+            L2B_TRY(launch_prompt_attention(a, gq, st));
+        } else {
+            AttnParams a;
+            memset(&a, 0, sizeof(a));
+            a.q = B.q; a.kc = kcl; a.vc = vcl; a.out = B.att; a.tickets = B.tickets;
+            a.part_m = B.pm; a.part_l = B.pl; a.part_acc = B.pacc;
+            a.pos = nullptr; a.pos_base = pos0; a.pos_list = pos_list; a.cache_stride_q = seq_stride;
+            a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.hs = hs; a.seq_len = c.seq_len; a.nsplit = B.nsplit;
+            a.nq = std::max(n, 2);  // (a one-token pass takes the many-query form of the kernel too: the second query copy leaves at once)
+            a.q_stride = c.dim;
+            a.min_chunk = 256;  // many queries already fill the GPU: split a query's positions only when there are many
+            if (n < 2) return fail(L2B_ERR_BAD_ARG, "a many-token pass needs at least two tokens");
+            CU(launch_attention(a, gq, st, false));
+        }
         L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.att, nullptr, c.dim, n, in_dim), st));
         L2B_TRY(product({&w.wo}, in_dim, sp, stride, ldy));
         L2B_TRY(launch_split_rows<SR_RESIDUAL>(behind(split_rows_params(B.x, w.rms_ffn, c.dim, n, in_dim), sp, stride, ldy, 0), st));

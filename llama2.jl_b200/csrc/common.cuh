@@ -71,6 +71,23 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// The same for kernels in which most warps wait most of the time: the hardware parks the warp (for at most the hinted time, then it asks
+// again), so that waiting takes no issue slots from the warps that work.
+__device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity) {
+    for (uint32_t i = 0; i < MBAR_MAX_POLLS / 16; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(2000u)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
 // The same wait bounded by TIME (nanoseconds of %globaltimer) instead of by polls: for warps whose partner may itself be
 // inside a long, legitimate wait (the tensor-parallel wait for another GPU's partial results).
 __device__ __forceinline__ bool mbar_wait_bounded_ns(uint64_t* bar, uint32_t parity, unsigned long long limit_ns) {
