@@ -462,6 +462,7 @@ static int32_t launch_kq_gemm(const DevMatrix* const* ws, int nw, const GemmInpu
     GemmMaps maps;
     memset(&g, 0, sizeof(g));
     int tiles = 0, max_bb = 0;
+    bool shared = false;
     for (int i = 0; i < nw; ++i) {
         const DevMatrix& w = *ws[i];
         if (w.type == T_F32) return fail(L2B_ERR_UNSUPPORTED_TYPE, "the tensor-core GEMM takes k-quant matrices");
@@ -472,6 +473,7 @@ static int32_t launch_kq_gemm(const DevMatrix* const* ws, int nw, const GemmInpu
         maps.tail[i] = w.map_tail;
         tiles += sg.row_tiles;
         max_bb = std::max(max_bb, dev_block_bytes(w.type));
+        shared = shared || w.type != T_Q6_K;
     }
     for (int i = nw; i < GM_MAX_SEG; ++i) maps.main[i] = maps.main[0], maps.tail[i] = maps.tail[0];
     g.nseg = nw; g.sp = sp; g.total = tiles * sp.ntile * sp.nb; g.n_tok = n_tok; g.groups = in.groups;
@@ -479,8 +481,8 @@ static int32_t launch_kq_gemm(const DevMatrix* const* ws, int nw, const GemmInpu
     const int grid = (g.total + sp.U - 1) / sp.U;
     auto go = [&](auto kernel, auto layout, int threads) {
         g.np = GM_MAX_PACKED;
-        while (layout(max_bb, g.np).total + 1024 > GM_SMEM) --g.np;  // + room to align the base to 1024 bytes
-        kernel<<<grid, threads, layout(max_bb, g.np).total + 1024, st>>>(g, maps);
+        while (layout(max_bb, g.np, shared).total + 1024 > GM_SMEM) --g.np;  // + room to align the base to 1024 bytes
+        kernel<<<grid, threads, layout(max_bb, g.np, shared).total + 1024, st>>>(g, maps);
     };
     if (sp.tok <= 32) go(kq_gemm_kernel<32>, gm_smem_layout<32>, GmCfg<32>::THREADS);
     else if (sp.tok <= 64) go(kq_gemm_kernel<64>, gm_smem_layout<64>, GmCfg<64>::THREADS);

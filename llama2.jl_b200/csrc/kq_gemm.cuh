@@ -18,8 +18,9 @@
 // the product anyway (norm, SwiGLU, RoPE) adds them.
 //
 //   packed-copy warp  one TMA tiled copy (cp.async.bulk.tensor) per super-block: a 128-row box of the stored blocks
-//   operand warp      one bulk copy per 64 values: the tokens' two terms, already in operand layout (split_rows_kernel)
-//   unpack warps      groups of four on steps of 64 values in turn; thread = row: nibbles -> fp16 times scale, into core matrices (8 rows x 16 bytes)
+//   2 operand warps   one bulk copy per 64 values: the tokens' two terms, already in operand layout (split_rows_kernel); a thread takes 750
+//                     cycles to see a slot free and issue a copy, so two take turns
+//   unpack warps      groups of four; thread = row: nibbles -> fp16 times scale, into core matrices (8 rows x 16 bytes)
 //   MMA warp          tcgen05.mma.kind::f16 (M 128, K 16), four or eight per 64 values
 //   8 epilogue warps  thread = weight row, half of the tokens: tensor memory -> times d -> f32 accumulators
 //
@@ -80,34 +81,46 @@ struct GemmMaps {
 };
 
 // ---- shared memory -----------------------------------------------------------------------------
-// NT tokens at most per tile.  NS slots for operands and accumulators; as many slots for packed super-blocks as fit (2 .. 5): more tokens
-// need more room per slot (128: 32 KiB of X), fewer tokens need more packed bytes in flight.
-// UG groups of four unpack warps take the steps in turn.  With 128 tokens a step's MMAs take 512 cycles and two groups keep up; with fewer the
-// unpacking is what a step takes, so there are four, and the epilogue's smaller share of the accumulators leaves the registers for them.
+// NT tokens at most per tile.
+// CH chunks of 64 values per step.  What a step costs beyond its MMAs is hand-overs: the MMA warp, the operand warps and the epilogue each spend
+// about 600 cycles per step whatever it holds.  With 128 tokens a chunk's MMAs take 512 cycles and tensor memory holds the sums of no
+// more, so a step is one chunk (and the shared part C a step of its own); with fewer a step is two chunks, each with a sum of its own, and
+// the second step of a super-block takes the shared part along.
+// NS slots for operands, ND for accumulators; as many slots for packed super-blocks as fit (2 .. 5).
+// UG groups of four unpack warps, GS of them on a step (with 64 tokens, two: a chunk each), UG / GS steps in turn.  A group waits for the slot's
+// last use by parity, so it must have seen the use before that: its own last step lies at most NS steps back, UG / GS <= NS.  (More groups
+// are no help: all read the scales of every super-block they take part in, 200 instructions a row, which with four groups on the steps
+// of one super-block made the kernel issue-bound.)
 // PAIR: high and low terms are columns of one MMA (half as many instructions, each of which reads the 4 KiB of A again: 32 cycles
-// whatever its columns); with 128 tokens the accumulators would not fit tensor memory.
+// whatever its columns); with 64 tokens the MMAs themselves take as long, with 128 the sums would not fit tensor memory.
 template <int NT>
 struct GmCfg {
-    static constexpr int NS = NT == 128 ? 3 : 4;
-    static constexpr int UG = NT == 128 ? 2 : 4;
-    static constexpr bool PAIR = NT != 128;
-    static constexpr int DCOLS = PAIR ? 2 * NT : NT;  // accumulator columns per slot
-    static constexpr int THREADS = (GM_EPI_WARPS + 3 + 4 * UG) * 32;  // warps 0-7 epilogue, 8 packed copies, 9 MMA, 10 operand copies, 11 .. unpack
+    static constexpr int CH = NT == 128 ? 1 : 2;
+    static constexpr int NS = NT == 64 ? 2 : 3, ND = NS;
+    static constexpr int GS = NT == 64 ? 2 : 1, UG = NT == 128 ? 2 : NT == 64 ? 4 : 3;
+    static_assert(UG / GS <= NS, "a group would miss a phase");
+    static constexpr bool PAIR = NT == 32;
+    static constexpr int CCOLS = PAIR ? 2 * NT : NT;            // accumulator columns per chunk
+    static constexpr int DCOLS = CH == 1 ? NT : 2 * CCOLS + NT;  // per slot: 128, 192, 160
+    static constexpr int THREADS = (GM_EPI_WARPS + 4 + 4 * UG) * 32;  // warps 0-7 epilogue, 8 packed copies, 9 MMA, 10 and 11 operand copies, 12 .. unpack
 };
 constexpr int GM_MAX_PACKED = 5;
 constexpr int GM_SMEM = 227 * 1024;
 struct GmSmem {
-    int off_bar, off_tmem, off_hdr, off_a, off_b, off_packed, slot_b, slot_packed, total;
+    int off_bar, off_tmem, off_hdr, off_a, off_b, off_packed, slot_a, slot_b, slot_packed, total;
 };
+// shared: some matrix of the launch has the part C (all but q6_K)
 template <int NT>
-__host__ __device__ inline GmSmem gm_smem_layout(int max_block_bytes, int np) {
+__host__ __device__ inline GmSmem gm_smem_layout(int max_block_bytes, int np, bool shared) {
+    constexpr int CH = GmCfg<NT>::CH;
     GmSmem s;
-    s.off_bar = 0;  // done[4] ready[4] p_full[5] p_free[5]
-    s.off_tmem = 18 * 8;
+    s.off_bar = 0;  // done[3] ready[3] p_full[5] p_free[5]
+    s.off_tmem = 16 * 8;
     s.off_hdr = 256;  // [GM_HDRS][128] {d, factor of the shared part}
     s.off_a = (s.off_hdr + GM_HDRS * GM_ROWS * 8 + 1023) & ~1023;
-    s.off_b = s.off_a + GmCfg<NT>::NS * GM_A_BYTES;
-    s.slot_b = NT * 256;
+    s.slot_a = CH * GM_A_BYTES + (CH == 2 && shared ? GM_A_BYTES / 2 : 0);
+    s.slot_b = CH * NT * 256 + (CH == 2 && shared ? NT * 32 : 0);
+    s.off_b = s.off_a + GmCfg<NT>::NS * s.slot_a;
     s.off_packed = s.off_b + GmCfg<NT>::NS * s.slot_b;
     s.slot_packed = (GM_ROWS * max_block_bytes + 1023) & ~1023;
     s.total = s.off_packed + np * s.slot_packed;
@@ -261,6 +274,18 @@ __global__ void sum_parts_kernel(const float* __restrict__ y, size_t part_stride
     }
 }
 
+// Two f32 operations in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)), "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return *reinterpret_cast<float2*>(&r);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return *reinterpret_cast<float2*>(&r);
+}
+
 // ---- unpacking -------------------------------------------------------------------------------------------
 __device__ __forceinline__ __half2 h2_bits(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 __device__ __forceinline__ uint32_t h2_raw(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
@@ -305,30 +330,36 @@ __device__ __forceinline__ void gm_store16(uint8_t* dst, const uint4& q, const u
 }
 
 // ---- the GEMM ----------------------------------------------------------------------------------------
-__device__ __forceinline__ int gm_steps(int type) { return type == T_Q6_K ? 8 : 5; }  // operand steps per super-block
+// Steps per super-block: q6_K has eight chunks (its two passes) and no shared part.
+template <int CH>
+__device__ __forceinline__ int gm_steps(int type) { return CH == 2 ? (type == T_Q6_K ? 4 : 2) : (type == T_Q6_K ? 8 : 5); }
 
 template <int NT>
 __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ GemmMaps maps) {
-    constexpr int NS = GmCfg<NT>::NS, UG = GmCfg<NT>::UG, DCOLS = GmCfg<NT>::DCOLS;
+    constexpr int NS = GmCfg<NT>::NS, ND = GmCfg<NT>::ND, UG = GmCfg<NT>::UG, GS = GmCfg<NT>::GS, DCOLS = GmCfg<NT>::DCOLS, CH = GmCfg<NT>::CH, CCOLS = GmCfg<NT>::CCOLS;
     constexpr bool PAIR = GmCfg<NT>::PAIR;
     const int NP = p.np;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the copies and operands want their alignment
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (the same for a warp's threads, and known to be)
     int max_bb = 0;
-    for (int i = 0; i < p.nseg; ++i) max_bb = max(max_bb, dev_block_bytes(p.seg[i].type));
-    const GmSmem L = gm_smem_layout<NT>(max_bb, p.np);
+    bool shared = false;
+    for (int i = 0; i < p.nseg; ++i) {
+        max_bb = max(max_bb, dev_block_bytes(p.seg[i].type));
+        shared = shared || p.seg[i].type != T_Q6_K;
+    }
+    const GmSmem L = gm_smem_layout<NT>(max_bb, p.np, shared);
     uint64_t* done = reinterpret_cast<uint64_t*>(smem + L.off_bar);
     // ready: weights unpacked, activations landed and the accumulators of the slot's last use read.  One barrier for all three, because the
     // MMA thread's own instructions bound this kernel: with a barrier each it took 1450 cycles per step of 64 values, whatever the tile.
-    uint64_t *ready = done + 4, *p_full = done + 8, *p_free = done + 13;
+    uint64_t *ready = done + 3, *p_full = done + 6, *p_free = done + 11;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.off_tmem);
     float2* hdr = reinterpret_cast<float2*>(smem + L.off_hdr);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; ++i) {
             mbar_init(done + i, 1);
-            mbar_init(ready + i, 4 + 1 + GM_EPI_WARPS);
+            mbar_init(ready + i, 4 * GS + 1 + GM_EPI_WARPS);
         }
         for (int i = 0; i < NP; ++i) {
             mbar_init(p_full + i, 1);
@@ -348,6 +379,13 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
     const int u0 = blockIdx.x * p.sp.U, u1 = min(u0 + p.sp.U, p.total);
     struct Where {
         int seg, row_tile, ntile, b;  // matrix, its row tile, token tile, super-block
+        int type, bb, steps, row_tiles;  // of the matrix (an indexed read of a parameter is slow)
+    };
+    auto enter = [&](Where& w) {
+        w.type = p.seg[w.seg].type;
+        w.bb = dev_block_bytes(w.type);
+        w.steps = gm_steps<CH>(w.type);
+        w.row_tiles = p.seg[w.seg].row_tiles;
     };
     auto first_unit = [&]() {
         Where w;
@@ -357,6 +395,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         w.ntile = tile - w.row_tile * p.sp.ntile;
         w.seg = 0;
         while (w.seg + 1 < p.nseg && w.row_tile >= p.seg[w.seg].row_tiles) w.row_tile -= p.seg[w.seg++].row_tiles;
+        enter(w);
         return w;
     };
     auto advance = [&](Where& w) {  // (divisions here, once per super-block and role, had cost 2000 cycles of every 5700)
@@ -364,10 +403,12 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         w.b = 0;
         if (++w.ntile < p.sp.ntile) return;
         w.ntile = 0;
-        if (++w.row_tile < p.seg[w.seg].row_tiles || w.seg + 1 == p.nseg) return;
+        if (++w.row_tile < w.row_tiles || w.seg + 1 == p.nseg) return;
         w.row_tile = 0;
         ++w.seg;
+        enter(w);
     };
+    const int chunk_b = p.sp.tok * 256;  // bytes of a chunk of X in its slot
     bool ok = true;
 
     if (warp == 8) {
@@ -377,12 +418,12 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
             int s = 0;
             uint32_t parity = 1;  // of the use before
             for (int u = u0; u < u1; ++u, advance(w)) {
-                if (u - u0 >= NP && !mbar_wait_bounded(p_free + s, parity)) {
+                if (u - u0 >= NP && !mbar_wait_parked(p_free + s, parity)) {
                     ok = false;
                     break;
                 }
                 const GemmSeg& sg = p.seg[w.seg];
-                const int bb = dev_block_bytes(sg.type), panel = w.b / sg.kb;
+                const int bb = w.bb, panel = w.b / sg.kb;
                 mbar_arrive_expect_tx(p_full + s, (uint32_t)(GM_ROWS * bb));
                 const bool tail = (panel + 1) * sg.kb > nb;
                 tma_load_3d(smem + L.off_packed + s * L.slot_packed, tail ? &maps.tail[w.seg] : &maps.main[w.seg], (w.b - panel * sg.kb) * bb,
@@ -397,26 +438,43 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // copies in flight land within microseconds
             }
         }
-    } else if (warp == 10) {
+    } else if (warp == 10 || warp == 11) {
         // ================= activation operands: one bulk copy per 64 values =================
         if (lane == 0) {
             Where w = first_unit();
-            int s = 0;
+            int s = 0, turn = warp - 10;
             bool first = true;
             uint32_t parity = 1;
             for (int u = u0; u < u1 && ok; ++u, advance(w)) {
-                const int steps = gm_steps(p.seg[w.seg].type), g0 = (w.ntile * p.sp.tok) >> 3, ng = min(p.sp.tok >> 3, p.groups - g0);
-                for (int k = 0; k < steps; ++k) {
-                    if (!first && !mbar_wait_bounded(done + s, parity)) {
-                        ok = false;
-                        break;
+                const int steps = w.steps, g0 = (w.ntile * p.sp.tok) >> 3, ng = min(p.sp.tok >> 3, p.groups - g0);
+                const uint8_t* act = p.act + ((size_t)w.b * 4 * p.groups + g0) * GM_GROUP_BYTES;
+                for (int k = 0; k < steps; ++k, turn ^= 1) {
+                    if (turn == 0) {
+                        if (!first && !mbar_wait_parked(done + s, parity)) {
+                            ok = false;
+                            break;
+                        }
+                        uint8_t* dst = smem + L.off_b + s * L.slot_b;
+                        const uint32_t xs_bytes = (uint32_t)(ng * GM_XS_BYTES), bytes = (uint32_t)(ng * GM_GROUP_BYTES);
+                        const uint8_t* xs = p.xs + ((size_t)w.b * p.groups + g0) * GM_XS_BYTES;
+                        if (CH == 1) {
+                            const bool shared_part = steps == 5 && k == 4;
+                            mbar_arrive_expect_tx(ready + s, shared_part ? xs_bytes : bytes);
+                            if (shared_part) bulk_g2s_plain(dst, xs, xs_bytes, ready + s);
+                            else bulk_g2s_plain(dst, act + (size_t)(k & 3) * p.groups * GM_GROUP_BYTES, bytes, ready + s);
+                        } else {
+                            const bool shared_part = steps == 2 && k == 1;
+                            const uint8_t* src = act + (size_t)(2 * (k & 1)) * p.groups * GM_GROUP_BYTES;
+                            mbar_arrive_expect_tx(ready + s, 2 * bytes + (shared_part ? xs_bytes : 0u));
+                            if (ng == p.groups) {  // the two chunks lie behind one another, here and there
+                                bulk_g2s_plain(dst, src, 2 * bytes, ready + s);
+                            } else {
+                                bulk_g2s_plain(dst, src, bytes, ready + s);
+                                bulk_g2s_plain(dst + chunk_b, src + (size_t)p.groups * GM_GROUP_BYTES, bytes, ready + s);
+                            }
+                            if (shared_part) bulk_g2s_plain(dst + 2 * chunk_b, xs, xs_bytes, ready + s);
+                        }
                     }
-                    uint8_t* dst = smem + L.off_b + s * L.slot_b;
-                    const bool shared_part = steps == 5 && k == 4;
-                    const uint32_t bytes = (uint32_t)(ng * (shared_part ? GM_XS_BYTES : GM_GROUP_BYTES));
-                    mbar_arrive_expect_tx(ready + s, bytes);
-                    if (shared_part) bulk_g2s_plain(dst, p.xs + ((size_t)w.b * p.groups + g0) * GM_XS_BYTES, bytes, ready + s);
-                    else bulk_g2s_plain(dst, p.act + ((size_t)(w.b * 4 + (k & 3)) * p.groups + g0) * GM_GROUP_BYTES, bytes, ready + s);
                     if (++s == NS) {
                         s = 0;
                         first = false;
@@ -436,35 +494,40 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         const uint64_t desc_a = umma_desc(smem + L.off_a, 2048, 128), desc_b = umma_desc(smem + L.off_b, 128, PAIR ? GM_GROUP_BYTES / 2 : GM_GROUP_BYTES);
         const uint64_t desc_xs = umma_desc(smem + L.off_b, 128, GM_XS_BYTES);
         Where w = first_unit();
-        int s = 0;
+        int s = 0, ds = 0;
         uint32_t parity = 0;
         for (int u = u0; u < u1 && ok; ++u, advance(w)) {
-            const int steps = gm_steps(p.seg[w.seg].type);
+            const int steps = w.steps;
             for (int k = 0; k < steps; ++k) {
-                if (!mbar_wait_bounded(ready + s, parity)) {
+                if (!mbar_wait_parked(ready + s, parity)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d = tmem_base + (uint32_t)(s * DCOLS);
-                const uint64_t da = desc_a + (uint64_t)(s * (GM_A_BYTES >> 4));
-                const bool shared_part = steps == 5 && k == 4;
+                const uint32_t d = tmem_base + (uint32_t)(ds * DCOLS);
+                const uint64_t da = desc_a + (uint64_t)(s * (L.slot_a >> 4)), db = desc_b + (uint64_t)(s * (L.slot_b >> 4));
+                const bool shared_part = k == (CH == 2 ? 1 : 4) && (CH == 2 ? steps == 2 : steps == 5);
                 if (elect_one()) {
-                    if (shared_part) {
-                        const uint64_t dx = desc_xs + (uint64_t)(s * (L.slot_b >> 4));
-                        umma_f16(d, da + (4096 >> 4), dx, idesc_xs, 0u);  // low terms of C first
-                        umma_f16(d, da, dx, idesc_xs, 1u);
-                    } else {
-                        const uint64_t db = desc_b + (uint64_t)(s * (L.slot_b >> 4));
+                    if (CH == 2 || !shared_part) {
 #pragma unroll
-                        for (int t = PAIR ? 0 : 1; t >= 0; --t)  // low terms of X first
+                        for (int c = 0; c < CH; ++c)
 #pragma unroll
-                            for (int kk = 0; kk < 4; ++kk)
-                                umma_f16(d, da + (uint64_t)(kk * (4096 >> 4)), db + (uint64_t)((t * 1024 + kk * 256) >> 4), idesc, t == (PAIR ? 0 : 1) && kk == 0 ? 0u : 1u);
+                            for (int t = PAIR ? 0 : 1; t >= 0; --t)  // low terms of X first
+#pragma unroll
+                                for (int kk = 0; kk < 4; ++kk)
+                                    umma_f16(d + (uint32_t)(c * CCOLS), da + (uint64_t)((c * GM_A_BYTES + kk * 4096) >> 4),
+                                             db + (uint64_t)((c * chunk_b + t * 1024 + kk * 256) >> 4), idesc, t == (PAIR ? 0 : 1) && kk == 0 ? 0u : 1u);
+                    }
+                    if (shared_part) {  // low terms of C first
+                        const uint64_t ax = da + (uint64_t)(CH == 2 ? (2 * GM_A_BYTES) >> 4 : 0), dx = desc_xs + (uint64_t)((s * L.slot_b + (CH == 2 ? 2 * chunk_b : 0)) >> 4);
+                        const uint32_t dd = d + (uint32_t)(CH == 2 ? 2 * CCOLS : 0);
+                        umma_f16(dd, ax + (4096 >> 4), dx, idesc_xs, 0u);
+                        umma_f16(dd, ax, dx, idesc_xs, 1u);
                     }
                     umma_commit(done + s);
                 }
                 __syncwarp();
+                if (++ds == ND) ds = 0;
                 if (++s == NS) {
                     s = 0;
                     parity ^= 1u;
@@ -472,41 +535,47 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
             }
         }
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
-    } else if (warp > 10) {
-        // ================= unpack: groups of four warps take the steps in turn; thread = row =================
-        const int id = threadIdx.x - 11 * 32, r = id & 127, group = (warp - 11) >> 2;
+    } else if (warp > 11) {
+        // ================= unpack: thread = row =================
+        const int id = threadIdx.x - 12 * 32, r = id & 127, group = (warp - 12) >> 2;
         const int row_off = (r >> 3) * 128 + (r & 7) * 16;
         auto q6_scale = [&](const Where& w) -> float {
+            if (w.type != T_Q6_K) return 0.f;
             const GemmSeg& sg = p.seg[w.seg];
             const int row = w.row_tile * GM_ROWS + r;
-            return sg.type == T_Q6_K && row < sg.rows ? __half2float(__ldg(sg.d6 + (size_t)row * nb + w.b)) : 0.f;
+            return row < sg.rows ? __half2float(__ldg(sg.d6 + (size_t)row * nb + w.b)) : 0.f;
         };
+        constexpr int TURNS = UG / GS;
+        const int my_turn = group / GS, sub = group % GS;
         Where w = first_unit();
         float d6_next = u0 < u1 ? q6_scale(w) : 0.f;
-        int s = 0, turn = 0, ps = 0, hs = 0;  // slot, whose turn it is, packed slot, set of factors
+        int s = 0, turn = 0, ps = 0, hs = GM_HDRS - 1;  // slot, whose turn it is, packed slot, set of factors
         bool first = true;
         uint32_t parity = 1, p_parity = 0;
         for (int u = u0; u < u1 && ok; ++u) {
-            const GemmSeg& sg = p.seg[w.seg];
-            const int bb = dev_block_bytes(sg.type);
+            const int type = w.type, bb = w.bb, steps = w.steps;
+            hs = (hs + 1) % GM_HDRS;
             const float d6 = d6_next;
             advance(w);
             if (u + 1 < u1) d6_next = q6_scale(w);  // a super-block ahead: the latency of a global read
-            if (!mbar_wait_bounded(p_full + ps, p_parity)) {
+            if (!mbar_wait_parked(p_full + ps, p_parity)) {  // (every group follows every packed slot, with or without a step in it)
                 ok = false;
                 break;
             }
             const uint8_t* blk = smem + L.off_packed + ps * L.slot_packed + r * bb;
-            const int steps = gm_steps(sg.type);
+            int ahead = my_turn - turn;  // steps until this group's next one
+            if (ahead < 0) ahead += TURNS;
+            const bool mine_here = ahead < steps;
             uint64_t sc8 = 0, m8 = 0;
             uint4 top0 = make_uint4(0u, 0u, 0u, 0u), top1 = top0;  // q5_K: fifth bits; q6_K: scales
             float d = d6, dmin = 0.f, s_up = 1.f, s_dn = 1.f;
-            if (sg.type != T_Q6_K) {
+            if (!mine_here) {
+            } else if (type != T_Q6_K) {
                 const uint4 h = *reinterpret_cast<const uint4*>(blk);
                 decode_scales_k4(h, sc8, m8);
                 d = half_bits_to_float(h.x & 0xFFFFu);
                 dmin = half_bits_to_float(h.x >> 16);
-                if (sg.type == T_Q5_K) {
+                if (type == T_Q5_K) {
                     top0 = *reinterpret_cast<const uint4*>(blk + 16);
                     top1 = *reinterpret_cast<const uint4*>(blk + 32);
                 }
@@ -519,65 +588,74 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
             } else {
                 top0 = *reinterpret_cast<const uint4*>(blk + 192);
             }
-            const float cen = sg.type == T_Q5_K ? 16.f : 8.f;
+            const float cen = type == T_Q5_K ? 16.f : 8.f;
             for (int k = 0; k < steps; ++k) {
                 const int slot = s;
-                const bool mine = turn == group, reused = !first;
+                const bool mine = turn == my_turn, reused = !first;
                 const uint32_t use_parity = parity;
-                if (++turn == UG) turn = 0;
+                if (++turn == TURNS) turn = 0;
                 if (++s == NS) {
                     s = 0;
                     first = false;
                     parity ^= 1u;
                 }
                 if (!mine) continue;
-                if (reused && !mbar_wait_bounded(done + slot, use_parity)) {
+                if (reused && !mbar_wait_parked(done + slot, use_parity)) {
                     ok = false;
                     break;
                 }
                 // (the epilogue may still be at the super-block before the last one: four sets of factors are enough)
-                if (k == 0) hdr[hs * GM_ROWS + r] = make_float2(d * (float)(1 << GM_A_EXP), 32.f * s_dn);
-                uint8_t* dst = smem + L.off_a + slot * GM_A_BYTES + row_off;
-                if (sg.type == T_Q6_K) {
-                    const int c = k & 3, hh = c >> 1, odd = c & 1;
-                    const uint32_t scw = c == 0 ? top0.x : c == 1 ? top0.y : c == 2 ? top0.z : top0.w;
+                if (k == 0 && sub == 0) hdr[hs * GM_ROWS + r] = make_float2(d * (float)(1 << GM_A_EXP), 32.f * s_dn);
+                uint8_t* const a_slot = smem + L.off_a + slot * L.slot_a + row_off;
+                if (CH == 2 || type == T_Q6_K || k < 4) {
+#pragma unroll 1
+                    for (int e = sub; e < CH; e += GS) {
+                        const int kc = CH * k + e;
+                        uint8_t* const dst = a_slot + e * GM_A_BYTES;
+                        if (type == T_Q6_K) {
+                            const int c = kc & 3, hh = c >> 1, odd = c & 1;
+                            const uint32_t scw = c == 0 ? top0.x : c == 1 ? top0.y : c == 2 ? top0.z : top0.w;
 #pragma unroll
-                    for (int part = 0; part < 2; ++part) {
-                        const uint4 f = *reinterpret_cast<const uint4*>(blk + 128 + 32 * hh + 16 * part);
+                            for (int part = 0; part < 2; ++part) {
+                                const uint4 f = *reinterpret_cast<const uint4*>(blk + 128 + 32 * hh + 16 * part);
 #pragma unroll
-                        for (int hi = 0; hi < 2; ++hi) {
-                            const int sc = (int)(int8_t)(scw >> (8 * (2 * hi + part)));
-                            const __half2 S = __half2half2(__int2half_rn(k < 4 ? sc - (sc & 1) : (sc & 1)));
-                            const GmScale g = gm_scale(S, 32.f);
-                            const uint4 q = *reinterpret_cast<const uint4*>(blk + 64 * hh + 32 * hi + 16 * part);
-                            const int idx = 2 * odd + hi;  // which two bits of the byte: value 16 at bit 2 * idx
-                            const __half2 up = __hmul2(S, h2_bits(((uint32_t)(23 - 2 * idx) << 10) * 0x00010001u));  // 2^(8 - 2 idx)
-                            if (odd) gm_store16<true, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
-                            else gm_store16<false, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
+                                for (int hi = 0; hi < 2; ++hi) {
+                                    const int sc = (int)(int8_t)(scw >> (8 * (2 * hi + part)));
+                                    const __half2 S = __half2half2(__int2half_rn(kc < 4 ? sc - (sc & 1) : (sc & 1)));
+                                    const GmScale g = gm_scale(S, 32.f);
+                                    const uint4 q = *reinterpret_cast<const uint4*>(blk + 64 * hh + 32 * hi + 16 * part);
+                                    const int idx = 2 * odd + hi;  // which two bits of the byte: value 16 at bit 2 * idx
+                                    const __half2 up = __hmul2(S, h2_bits(((uint32_t)(23 - 2 * idx) << 10) * 0x00010001u));  // 2^(8 - 2 idx)
+                                    if (odd) gm_store16<true, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
+                                    else gm_store16<false, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
+                                }
+                            }
+                        } else {
+                            const uint32_t two = (uint32_t)(sc8 >> (16 * kc));
+                            const GmScale g0 = gm_scale(h2_small_int(two & 0xFFu), cen), g1 = gm_scale(h2_small_int((two >> 8) & 0xFFu), cen);
+                            if (type == T_Q5_K) {  // the fifth bit of sub-block j is bit j: value 16 from 2^(j - 24) takes 2^(8 - j)
+                                const uint32_t p0 = (uint32_t)(23 - 2 * kc) << 10;
+                                const __half2 up0 = __hmul2(g0.high, h2_bits(p0 * 0x00010001u)), up1 = __hmul2(g1.high, h2_bits((p0 - 1024u) * 0x00010001u));
+                                const uint32_t bit = 0x00010001u << (2 * kc);
+#pragma unroll
+                                for (int part = 0; part < 2; ++part) {
+                                    const uint4 q = *reinterpret_cast<const uint4*>(blk + 48 + 32 * kc + 16 * part);
+                                    gm_store16<false, true>(dst + 2 * part * 4096, q, part ? top1 : top0, bit, up0, g0);
+                                    gm_store16<true, true>(dst + (2 * part + 1) * 4096, q, part ? top1 : top0, bit << 1, up1, g1);
+                                }
+                            } else {
+#pragma unroll
+                                for (int part = 0; part < 2; ++part) {
+                                    const uint4 q = *reinterpret_cast<const uint4*>(blk + 16 + 32 * kc + 16 * part);
+                                    gm_store16<false, false>(dst + 2 * part * 4096, q, q, 0u, g0.high, g0);
+                                    gm_store16<true, false>(dst + (2 * part + 1) * 4096, q, q, 0u, g1.high, g1);
+                                }
+                            }
                         }
                     }
-                } else if (k < 4) {
-                    const uint32_t two = (uint32_t)(sc8 >> (16 * k));
-                    const GmScale g0 = gm_scale(h2_small_int(two & 0xFFu), cen), g1 = gm_scale(h2_small_int((two >> 8) & 0xFFu), cen);
-                    if (sg.type == T_Q5_K) {  // the fifth bit of sub-block j is bit j: value 16 from 2^(j - 24) takes 2^(8 - j)
-                        const uint32_t p0 = (uint32_t)(23 - 2 * k) << 10;
-                        const __half2 up0 = __hmul2(g0.high, h2_bits(p0 * 0x00010001u)), up1 = __hmul2(g1.high, h2_bits((p0 - 1024u) * 0x00010001u));
-                        const uint32_t bit = 0x00010001u << (2 * k);
-#pragma unroll
-                        for (int part = 0; part < 2; ++part) {
-                            const uint4 q = *reinterpret_cast<const uint4*>(blk + 48 + 32 * k + 16 * part);
-                            gm_store16<false, true>(dst + 2 * part * 4096, q, part ? top1 : top0, bit, up0, g0);
-                            gm_store16<true, true>(dst + (2 * part + 1) * 4096, q, part ? top1 : top0, bit << 1, up1, g1);
-                        }
-                    } else {
-#pragma unroll
-                        for (int part = 0; part < 2; ++part) {
-                            const uint4 q = *reinterpret_cast<const uint4*>(blk + 16 + 32 * k + 16 * part);
-                            gm_store16<false, false>(dst + 2 * part * 4096, q, q, 0u, g0.high, g0);
-                            gm_store16<true, false>(dst + (2 * part + 1) * 4096, q, q, 0u, g1.high, g1);
-                        }
-                    }
-                } else {
+                }
+                if (type != T_Q6_K && k == (CH == 2 ? 1 : 4) && sub == GS - 1) {
+                    uint8_t* const dst = a_slot + (CH == 2 ? 2 * GM_A_BYTES : 0);
                     uint32_t o[4], o2[4];
 #pragma unroll
                     for (int j2 = 0; j2 < 4; ++j2) {
@@ -605,7 +683,6 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
             }
             __syncwarp();
             if (lane == 0 && ok) mbar_arrive(p_free + ps);
-            hs = (hs + 1) % GM_HDRS;
             if (++ps == NP) {
                 ps = 0;
                 p_parity ^= 1u;
@@ -618,45 +695,69 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         const int q = warp & 3, half = warp >> 2;
         const int r = 32 * q + lane;
         const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16);
-        float acc[NH];
+        const int mine = max(0, min(NH, p.sp.tok - NH * half));  // of the tile's tokens
+        float2 acc[NH / 2];
 #pragma unroll
-        for (int t = 0; t < NH; ++t) acc[t] = 0.f;
-        if (lane < NS) mbar_arrive(ready + lane);  // no accumulators to wait for at first
+        for (int t = 0; t < NH / 2; ++t) acc[t] = make_float2(0.f, 0.f);
+        if (lane < ND) mbar_arrive(ready + lane);  // no accumulators to wait for at first
         Where w = first_unit();
-        int s = 0, hs = 0;
+        int s = 0, hs = 0, ds = 0, next = ND % NS;  // next: the step that will use these accumulators again
         uint32_t parity = 0;
         for (int u = u0; u < u1 && ok; ++u, advance(w)) {
-            const int steps = gm_steps(p.seg[w.seg].type);
+            const int steps = w.steps;
             float2 f = make_float2(0.f, 0.f);
             for (int k = 0; k < steps; ++k) {
-                if (!mbar_wait_bounded(done + s, parity)) {
+                if (!mbar_wait_parked(done + s, parity)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
                 if (k == 0) f = hdr[hs * GM_ROWS + r];
-                const bool shared_part = steps == 5 && k == 4;
-                const float m = shared_part ? f.y : f.x;
-                if (PAIR && !shared_part) {  // columns in eights: high terms of eight tokens, then their low terms
+                const bool shared_part = k == (CH == 2 ? 1 : 4) && (CH == 2 ? steps == 2 : steps == 5);
+                const float2 md = make_float2(f.x, f.x), mc = make_float2(f.y, f.y);
+                const uint32_t td = taddr + (uint32_t)(ds * DCOLS);
+                if (PAIR) {  // two chunks; columns in eights: high terms of eight tokens, then their low terms
 #pragma unroll
                     for (int c0 = 0; c0 < NH; c0 += 8) {
-                        float v[16];
-                        tmem_ld16f(taddr + (uint32_t)(s * DCOLS + 2 * (NH * half + c0)), v);
+                        if (c0 >= mine) break;
+                        float v[16], w2[16];
+                        tmem_ld16f(td + (uint32_t)(2 * (NH * half + c0)), v);
+                        tmem_ld16f(td + (uint32_t)(CCOLS + 2 * (NH * half + c0)), w2);
 #pragma unroll
-                        for (int t = 0; t < 8; ++t) acc[c0 + t] = fmaf(m, v[t] + v[8 + t], acc[c0 + t]);
+                        for (int t = 0; t < 8; t += 2) {
+                            const float2 hi = add2(make_float2(v[t], v[t + 1]), make_float2(w2[t], w2[t + 1]));
+                            const float2 lo = add2(make_float2(v[8 + t], v[9 + t]), make_float2(w2[8 + t], w2[9 + t]));
+                            acc[(c0 + t) / 2] = fma2(md, add2(hi, lo), acc[(c0 + t) / 2]);
+                        }
                     }
-                } else {
+                } else if (CH == 2) {
 #pragma unroll
                     for (int c0 = 0; c0 < NH; c0 += 16) {
-                        float v[16];
-                        tmem_ld16f(taddr + (uint32_t)(s * DCOLS + NH * half + c0), v);
+                        if (c0 >= mine) break;
+                        float v[16], w2[16];
+                        tmem_ld16f(td + (uint32_t)(NH * half + c0), v);
+                        tmem_ld16f(td + (uint32_t)(CCOLS + NH * half + c0), w2);
 #pragma unroll
-                        for (int t = 0; t < 16; ++t) acc[c0 + t] = fmaf(m, v[t], acc[c0 + t]);
+                        for (int t = 0; t < 16; t += 2)
+                            acc[(c0 + t) / 2] = fma2(md, add2(make_float2(v[t], v[t + 1]), make_float2(w2[t], w2[t + 1])), acc[(c0 + t) / 2]);
+                    }
+                }
+                if (CH == 1 || shared_part) {
+                    const float2 mm = shared_part ? mc : md;
+#pragma unroll
+                    for (int c0 = 0; c0 < NH; c0 += 16) {
+                        if (c0 >= mine) break;
+                        float v[16];
+                        tmem_ld16f(td + (uint32_t)((CH == 2 ? 2 * CCOLS : 0) + NH * half + c0), v);
+#pragma unroll
+                        for (int t = 0; t < 16; t += 2) acc[(c0 + t) / 2] = fma2(mm, make_float2(v[t], v[t + 1]), acc[(c0 + t) / 2]);
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(ready + s);
+                if (lane == 0) mbar_arrive(ready + next);
+                if (++next == NS) next = 0;
+                if (++ds == ND) ds = 0;
                 if (++s == NS) {
                     s = 0;
                     parity ^= 1u;
@@ -672,10 +773,11 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 float* dst = p.y + (size_t)(blockIdx.x - first) * p.part_stride + row;
 #pragma unroll
                 for (int t = 0; t < NH; ++t) {
-                    const int tt = NH * half + t, tok = w.ntile * p.sp.tok + tt;
-                    if (valid && tt < p.sp.tok && tok < p.n_tok) dst[(size_t)tok * p.ldy] = acc[t] * __ldg(p.scale + tok);
-                    acc[t] = 0.f;
+                    const int tok = w.ntile * p.sp.tok + NH * half + t;
+                    if (valid && t < mine && tok < p.n_tok) dst[(size_t)tok * p.ldy] = (t & 1 ? acc[t / 2].y : acc[t / 2].x) * __ldg(p.scale + tok);
                 }
+#pragma unroll
+                for (int t = 0; t < NH / 2; ++t) acc[t] = make_float2(0.f, 0.f);
             }
         }
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
