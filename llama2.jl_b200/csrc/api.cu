@@ -1867,6 +1867,9 @@ static int32_t run_one(l2b_session* s, int token, int pos, float temperature, do
 // Needs q4_K / q5_K layer matrices, three activation planes, one GPU; otherwise the caller uses the decode passes.
 constexpr int PF_MAX_TOK = 512;
 constexpr int PF_MIN_TOK = 12;
+// Shortest prompt whose last position goes through the pass too, so that the matrices are read once for all of it.  At the 8B shape a pass of a
+// few tokens takes 6.4 ms and the decode kernels 1.6 ms per position or pair of forced positions: even at about eight.
+constexpr int PF_MIN_ALL = 10;
 constexpr int BATCH_MAX_SEQ = 240;
 constexpr int STACK_MIN_ROWS = 2;  // layer-stack models
 
@@ -2011,14 +2014,15 @@ static bool prefill_gemm_eligible(l2b_session* s) {
 // Shortest run of forced positions that goes through a many-token pass.
 static int min_pass_tokens(const l2b_session* s) { return s->stack ? STACK_MIN_ROWS : PF_MIN_TOK; }
 
+// `forced` of them are followed by a prompt token.
 // Positions pos0 .. pos0 + n - 1 of the prompt already in s->prompt (device), 2 <= n <= PF_MAX_TOK; all enqueued on the session stream.
-static int32_t enqueue_prefill_gemm(l2b_session* s, int pos0, int n) {
+static int32_t enqueue_prefill_gemm(l2b_session* s, int pos0, int n, int forced) {
     const l2b_model* m = s->model;
     const l2b_config& c = m->cfg;
     cudaStream_t st = s->stream;
     if (s->stack) {
         L2B_TRY(stack_enqueue_rows(s->stack, s->prompt + pos0, n, pos0, nullptr, s->status, st, &s->last_launches));
-        fill_forced_kernel<<<1, 256, 0, st>>>(s->prompt, s->out_tokens, pos0, n);
+        fill_forced_kernel<<<1, 256, 0, st>>>(s->prompt, s->out_tokens, pos0, forced);
         CU(cudaGetLastError());
         ++s->last_launches;
         return L2B_OK;
@@ -2027,7 +2031,7 @@ static int32_t enqueue_prefill_gemm(l2b_session* s, int pos0, int n) {
                                                                                       c.vocab_size, s->pf.x);
     CU(cudaGetLastError());
     L2B_TRY(enqueue_layers_gemm(m, s->pf, n, s->kc, s->vc, kv_layer_elems(m), pos0, nullptr, 0, s->rope_cs, s->gq, nullptr, s->status, st));
-    fill_forced_kernel<<<1, 256, 0, st>>>(s->prompt, s->out_tokens, pos0, n);
+    fill_forced_kernel<<<1, 256, 0, st>>>(s->prompt, s->out_tokens, pos0, forced);
     CU(cudaGetLastError());
     s->last_launches += 3 + 10LL * c.n_layers;  // per layer: 4 products, 4 operand kernels, RoPE + cache write, attention
     return L2B_OK;
@@ -2040,7 +2044,7 @@ static int32_t enqueue_forced_positions(l2b_session* s, int from, int to, const 
     if (to - from >= min_pass_tokens(s) && prefill_gemm_eligible(s)) {
         while (i < to) {
             const int n = std::min(s->stack ? stack_session_max_rows(s->stack) : PF_MAX_TOK, to - i);
-            L2B_TRY(enqueue_prefill_gemm(s, i, n));
+            L2B_TRY(enqueue_prefill_gemm(s, i, n, n));
             i += n;
         }
         // the decode graphs read the loop state from the device: move it to position i
@@ -2055,6 +2059,49 @@ static int32_t enqueue_forced_positions(l2b_session* s, int from, int to, const 
         s->last_launches += pair ? s->kernels_per_pair : s->kernels_per_token;
         i += pair ? 2 : 1;
     }
+    return L2B_OK;
+}
+
+// All positions [from, end) of a prompt in many-token passes, the last one included: its logits and the choice of the token behind it as the
+// one-position graph leaves them (and its row in the buffers that l2b_session_read shows).  False: not taken, nothing enqueued.
+static int32_t enqueue_whole_prompt(l2b_session* s, int from, int end, int32_t last_token, bool& taken) {
+    taken = !s->stack && end - from >= PF_MIN_ALL && prefill_gemm_eligible(s);
+    if (!taken) return L2B_OK;
+    const l2b_model* m = s->model;
+    const l2b_config& c = m->cfg;
+    int n = 0;
+    for (int i = from; i < end; i += n) {
+        n = std::min(PF_MAX_TOK, end - i);
+        if (end - i - n == 1) --n;  // a pass holds two tokens or more
+        L2B_TRY(enqueue_prefill_gemm(s, i, n, i + n == end ? n - 1 : n));
+    }
+    const size_t last = (size_t)n - 1;
+    CU(cudaMemcpyAsync(s->x, s->pf.x + last * c.dim, (size_t)c.dim * 4, cudaMemcpyDeviceToDevice, s->stream));
+    CU(cudaMemcpyAsync(s->q, s->pf.q + last * c.dim, (size_t)c.dim * 4, cudaMemcpyDeviceToDevice, s->stream));
+    CU(cudaMemcpyAsync(s->hb, s->pf.h + last * c.hidden_dim, (size_t)c.hidden_dim * 4, cudaMemcpyDeviceToDevice, s->stream));
+    Control& h = *s->h_ctl;
+    h.token = last_token;
+    h.pos = end - 1;
+    CU(cudaMemcpyAsync(s->ctl, s->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, s->stream));
+    MvLaunch L;
+    memset(&L.p, 0, sizeof(L.p));
+    L.planes = m->planes;
+    L.p.n_in = c.dim;
+    L.p.pos = &s->ctl->pos;
+    L.p.rope_cs = s->rope_cs;
+    L.p.seq_len = c.seq_len;
+    L.p.status = s->status;
+    L.p.seg[L.p.nseg++] = make_segment(m->output, PAIR_ADJACENT, EPI_LOGITS, s->logits, c.dim / c.n_heads);
+    L.kb = m->output.kb;
+    L.p.pro = PRO_RMSNORM;
+    L.p.gain = m->rms_final;
+    L.p.x_in = s->x;
+    L.p.amax_val = s->amax_val;
+    L.p.amax_idx = s->amax_idx;
+    L2B_TRY(plan_matvec(L, s->di));
+    CU(launch_matvec(L, s->stream, false));
+    L2B_TRY(enqueue_finalize(s, L.grid));
+    s->last_launches += 2;
     return L2B_OK;
 }
 
@@ -2169,9 +2216,13 @@ extern "C" int32_t l2b_prefill(l2b_session* s, const int32_t* tokens, int32_t n,
     CU(cudaMemcpyAsync(s->ctl, s->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, s->stream));
     const int end = pos0 + n;
     s->last_launches = 0;
-    L2B_TRY(enqueue_forced_positions(s, pos0, end - 1, tokens));  // every position but the last is followed by a prompt token
-    CU(cudaGraphLaunch(s->graph, s->stream));                     // the last one: its logits are wanted
-    s->last_launches += s->kernels_per_token;
+    bool whole = false;
+    L2B_TRY(enqueue_whole_prompt(s, pos0, end, tokens[n - 1], whole));
+    if (!whole) {
+        L2B_TRY(enqueue_forced_positions(s, pos0, end - 1, tokens));  // every position but the last is followed by a prompt token
+        CU(cudaGraphLaunch(s->graph, s->stream));                     // the last one: its logits are wanted
+        s->last_launches += s->kernels_per_token;
+    }
     CU(cudaMemcpyAsync(&s->h_small[0], s->next_token, 4, cudaMemcpyDeviceToHost, s->stream));
     CU(cudaMemcpyAsync(&s->h_small[1], s->status, 4, cudaMemcpyDeviceToHost, s->stream));
     CU(cudaEventRecord(s->ev1, s->stream));
@@ -2282,9 +2333,12 @@ extern "C" int32_t l2b_generate(l2b_session* s, const int32_t* prompt, int32_t n
     bool mid = false;
     const int forced_end = std::min(n_prompt - 1, n_positions);  // positions below this are followed by a prompt token
     s->last_launches = 0;
-    L2B_TRY(enqueue_forced_positions(s, 0, forced_end, prompt));
-    s->last_launches += (long long)(n_positions - forced_end) * s->kernels_per_token;
-    for (int i = forced_end; i < n_positions; ++i) {
+    bool whole = false;
+    if (forced_end < n_positions) L2B_TRY(enqueue_whole_prompt(s, 0, forced_end + 1, prompt[forced_end], whole));
+    if (!whole) L2B_TRY(enqueue_forced_positions(s, 0, forced_end, prompt));
+    const int first = forced_end + (whole ? 1 : 0);  // the first position that takes the one-position graph
+    s->last_launches += (long long)(n_positions - first) * s->kernels_per_token;
+    for (int i = first; i < n_positions; ++i) {
         if (i >= n_prompt && !mid) {  // the first position that is fed a generated token
             CU(cudaEventRecord(s->ev_mid, s->stream));
             mid = true;
