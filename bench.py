@@ -127,7 +127,7 @@ def kv_bytes(cfg, schedule, tp=1):
 def time_matvec(ggml_type, n_in, n_out, copies, launches, steps, warmup, planes, cols=1):
     """Average device time of one fused_matvec_kernel launch (CUDA events on the launching stream), weights rotated
     through `copies` copies of the matrix so that every launch streams from HBM.  cols > 1: one call of the tensor-core GEMM
-    (quantise + kq_gemm_kernel) over that many activation columns instead."""
+    (split_rows_kernel + kq_gemm_kernel) over that many activation columns instead."""
     import torch
     import __graft_entry__ as g
     g.load_package()
@@ -516,8 +516,8 @@ def run_ours(args):
     forced = max(min(n_prompt - 1, n_pos), 0)  # prompt positions that are followed by a prompt token (no logits needed)
     gemm_min = model.prefill_gemm_min_tokens()
     if gemm_min and forced >= gemm_min:
-        prefill_how = ("%d forced positions through the tensor-core GEMM pass (tcgen05 + TMA, 20 tokens per pass over a weight tile, "
-                       "no logits for forced positions), the last prompt position through the decode kernels" % forced)
+        prefill_how = ("%d forced positions and the last one through the tensor-core GEMM pass (tcgen05 + TMA, up to 128 tokens per pass over a "
+                       "weight tile, no logits for forced positions)" % forced)
     elif pairs:
         prefill_how = "two positions per pass of the decode kernels where both are followed by a prompt token (no logits for forced positions)"
     else:

@@ -216,8 +216,8 @@ int32_t l2b_prefill(l2b_session* session, const int32_t* tokens, int32_t n, int3
 int32_t l2b_session_extend(l2b_session* session, const int32_t* tokens, int32_t n, int32_t pos0, const int32_t* want, int32_t n_want,
                            float* host_logits);
 /* *min_tokens > 0: runs of at least that many prompt positions that are all followed by a prompt token go through the
- * many-token pass (every matrix product one launch of the tensor-core GEMM, tcgen05 + TMA, 20 tokens per pass over a weight
- * tile; up to 240 tokens per pass over the layers).  0: not available for this model (needs q4_K / q5_K layer matrices, three
+ * many-token pass (products on the tensor cores, tcgen05 + TMA, up to 128 tokens per pass over a weight tile; up to 512 tokens
+ * per pass over the layers).  0: not available for this model (needs q4_K / q5_K layer matrices, three
  * activation planes, one GPU; L2B_PREFILL_GEMM=0 switches it off) -- prompts then go through the decode kernels.  The reference
  * feeds prompts token by token (src/inference.jl:349-356). */
 int32_t l2b_session_prefill_gemm(l2b_session* session, int32_t* min_tokens);

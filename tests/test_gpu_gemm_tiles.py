@@ -1,0 +1,57 @@
+"""The tensor-core GEMM (csrc/kq_gemm.cuh) around its tile sizes: 16, 32, 64 and 128 columns, tiles shared between blocks and whole ones, a q6_K
+classifier with every tile width, and prompts around the longest pass."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("t", [12, 13])
+@pytest.mark.parametrize("n_in,n_out", [(256, 2), (4096, 384), (5120, 20000)])
+@pytest.mark.parametrize("ncols", [16, 17, 32, 33, 48, 63, 65, 112, 128, 129, 200])
+def test_columns_around_the_tiles(pkg, orc, synth, t, n_in, n_out, ncols):
+    """Bound as in test_gpu_gemm.py: 4e-6 of the largest result.  Twice, bit for bit: partial results are added in a fixed order."""
+    A = synth.matrix(t, n_in, n_out, seed=n_in + n_out + t)
+    X = synth.normal_f32(ncols * n_in, 3 + ncols, 1.0).reshape(ncols, n_in)
+    X[-1] *= 1e-30  # the factors of a column reach far down
+    X[0, n_in // 2] = 3e4  # one activation that dwarfs the others
+    Y = np.full((ncols, n_out), np.nan, np.float32)
+    again = Y.copy()
+    pkg.matmul_(Y, A, X)
+    pkg.matmul_(again, A, X)
+    assert np.array_equal(Y, again)
+    for c in {0, 1, ncols // 2, ncols - 1}:
+        want = orc.matmul_f64(A, X[c])
+        assert np.abs(Y[c] - want).max() <= 4e-6 * np.abs(want).max(), c
+
+
+@pytest.mark.parametrize("n_seq", [3, 33, 70, 130])
+def test_q6_k_classifier_of_batches(pkg, orc, synth, n_seq):
+    cfg = pkg.ModelConfig(512, 768, 1, 4, 2, 1024, 8, 10000.0, False)
+    w = synth.model_weights(cfg, dict(synth.ALL(12), output=14), seed=n_seq)
+    model = pkg.LanguageModel(cfg, None, w)
+    batch = pkg.BatchRunState(model, n_seq)
+    ids = synth.tokens(n_seq, 9, 3, cfg.vocab_size)
+    batch.decode_next(ids, np.zeros(n_seq, np.int32), want_logits=True)
+    oracle = orc.OracleModel(cfg, w)
+    for i in {0, 1, n_seq // 2, n_seq - 1}:
+        want = oracle.sample_greedy(ids[i:i + 1], 1, want_logits=True)[1][0]
+        assert np.abs(batch.logits[i] - want).max() / float(want.max() - want.min()) < 5e-5, i
+    batch.close()
+    model.close()
+
+
+@pytest.mark.parametrize("n", [10, 512, 513, 514])
+def test_prompts_around_the_longest_pass(pkg, orc, synth, n):
+    """A pass holds 512 tokens and never one alone; the last position is in the pass, and generation goes on behind it."""
+    cfg = pkg.ModelConfig(256, 512, 1, 4, 2, 512, 520, 10000.0, False)
+    w = synth.model_weights(cfg, dict(synth.ALL(12), output=14), seed=77)
+    ids = synth.tokens(n, 21, 3, cfg.vocab_size)
+    tokens, want = orc.OracleModel(cfg, w).sample_greedy(ids, n + 4, want_logits=True)
+    model = pkg.LanguageModel(cfg, None, w)
+    st = pkg.RunState(model)
+    assert pkg.prefill(st, ids, 0) == int(tokens[n - 1])
+    assert np.abs(st.logits - want[n - 1]).max() / float(want[n - 1].max() - want[n - 1].min()) < 5e-5
+    got, _ = pkg.generate(model, ids, n + 4)
+    assert np.array_equal(got, tokens)
+    model.close()
