@@ -43,7 +43,7 @@ def test_q6_k_classifier_of_batches(pkg, orc, synth, n_seq):
 
 @pytest.mark.parametrize("n", [10, 512, 513, 514])
 def test_prompts_around_the_longest_pass(pkg, orc, synth, n):
-    """A pass holds 512 tokens and never one alone; the last position is in the pass, and generation goes on behind it."""
+    """A pass holds 512 tokens; up to there the last position is in it.  Generation goes on behind it."""
     cfg = pkg.ModelConfig(256, 512, 1, 4, 2, 512, 520, 10000.0, False)
     w = synth.model_weights(cfg, dict(synth.ALL(12), output=14), seed=77)
     ids = synth.tokens(n, 21, 3, cfg.vocab_size)
