@@ -7,8 +7,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("t", [12, 13])
-@pytest.mark.parametrize("n_in,n_out", [(256, 2), (4096, 384), (5120, 20000)])
-@pytest.mark.parametrize("ncols", [16, 17, 32, 33, 48, 63, 65, 112, 128, 129, 200])
+@pytest.mark.parametrize("n_in,n_out,ncols", [(256, 2, c) for c in (16, 33, 129)] + [(2048, 384, c) for c in (16, 17, 32, 33, 48, 63, 65, 112, 128, 129, 200)] +
+                         [(2560, 19000, c) for c in (17, 129)])
 def test_columns_around_the_tiles(pkg, orc, synth, t, n_in, n_out, ncols):
     """Bound as in test_gpu_gemm.py: 4e-6 of the largest result.  Twice, bit for bit: partial results are added in a fixed order."""
     A = synth.matrix(t, n_in, n_out, seed=n_in + n_out + t)
