@@ -12,10 +12,11 @@
 //       there in f32 registers: with sums over 256 values the rounding of the tensor core is what the error consists of.
 //   C = centre * d * scale - dmin * min, the part of the weight that a sub-block's values share, as two fp16 terms.
 //
-// Work is counted in super-blocks of (128 weight rows x up to 128 tokens): block c takes units c*U .. c*U + U - 1 of the list
-// (tile, super-block), whatever tile they belong to, so that every SM has the same share.  A tile that several blocks share
-// leaves one partial result per block in a buffer of its own (no atomics: the sum's order is fixed); the kernel that reads
-// the product anyway (norm, SwiGLU, RoPE) adds them.
+// Work is counted in super-blocks of 128 weight rows: chunk c holds units c*U .. c*U + U - 1 of the list (row tile, super-block),
+// whatever tile they belong to, so that every SM has the same share; a block takes a chunk for up to 128 tokens at a time.  A row tile
+// that lies in several chunks leaves one partial result per chunk in a buffer of its own (no atomics: the sum's order is fixed); the
+// kernel that reads the product anyway (norm, SwiGLU, RoPE) adds them.  The cuts come from the matrices alone, never from the number of
+// tokens: buffers grow with the tokens and nothing else.
 //
 //   packed-copy warp  one TMA tiled copy (cp.async.bulk.tensor) per super-block: a 128-row box of the stored blocks
 //   2 operand warps   one bulk copy per 64 values: the tokens' two terms, already in operand layout (split_rows_kernel); a thread takes 750
@@ -45,14 +46,14 @@ constexpr int GM_EPI_WARPS = 8;
 
 // How a product's tiles are shared out; the kernels that read the partial results derive their number from it.
 struct GemmSplit {
-    int U;        // units (super-blocks of a tile) per block
-    int nb;       // units per tile
+    int U;        // units (super-blocks of a row tile) per chunk
+    int nb;       // units per row tile
     int ntile;    // token tiles
     int tok;      // tokens per tile (a multiple of 16)
 };
-__host__ __device__ inline int gm_tile(const GemmSplit& s, int row, int tok) { return (row / GM_ROWS) * s.ntile + tok / s.tok; }
-__host__ __device__ inline int gm_parts(const GemmSplit& s, int tile) {
-    const unsigned lo = (unsigned)tile * s.nb;
+// Parts that the results of this row are in.
+__host__ __device__ inline int gm_parts(const GemmSplit& s, int row) {
+    const unsigned lo = (unsigned)(row / GM_ROWS) * s.nb;
     return (int)((lo + s.nb - 1) / s.U - lo / s.U) + 1;
 }
 
@@ -65,7 +66,7 @@ struct GemmParams {
     GemmSeg seg[GM_MAX_SEG];
     int nseg;
     GemmSplit sp;
-    int total;            // units
+    int total, chunks;    // units; chunks of sp.U of them
     int n_tok, groups;    // tokens; groups of 8 in the operand buffers
     int np;               // slots for packed super-blocks
     const uint8_t* act;   // [nb][4][groups] x GM_GROUP_BYTES
@@ -149,7 +150,7 @@ struct SplitRowsParams {
 };
 
 __device__ __forceinline__ void gm_sum_parts8(const float* y, size_t part_stride, const GemmSplit& sp, int tok, int ldy, int row, float (&v)[8]) {
-    const int parts = gm_parts(sp, gm_tile(sp, row, tok));
+    const int parts = gm_parts(sp, row);
     const float* src = y + (size_t)tok * ldy + row;
     float4 a = __ldcg(reinterpret_cast<const float4*>(src)), b = __ldcg(reinterpret_cast<const float4*>(src) + 1);
     for (int p = 1; p < parts; ++p) {
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const __grid_constant__
 __global__ void sum_parts_kernel(const float* __restrict__ y, size_t part_stride, const __grid_constant__ GemmSplit sp, int ldy, int rows, float* __restrict__ dst) {
     const int tok = blockIdx.y;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
-        const int parts = gm_parts(sp, gm_tile(sp, i, tok));
+        const int parts = gm_parts(sp, i);
         float v = __ldcg(y + (size_t)tok * ldy + i);
         for (int p = 1; p < parts; ++p) v += __ldcg(y + p * part_stride + (size_t)tok * ldy + i);
         dst[(size_t)tok * rows + i] = v;
@@ -374,11 +375,11 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    // the walk over this block's units, the same for every role
-    const int nb = p.sp.nb;
-    const int u0 = blockIdx.x * p.sp.U, u1 = min(u0 + p.sp.U, p.total);
+    // the walk over this block's units, the same for every role: chunks of token tile 0, of token tile 1, ..., every gridDim.x-th of them
+    const int nb = p.sp.nb, items = p.chunks * p.sp.ntile;
     struct Where {
-        int seg, row_tile, ntile, b;  // matrix, its row tile, token tile, super-block
+        int u, end;                  // unit, first one behind the chunk
+        int seg, row_tile, ntile, b; // matrix, its row tile, token tile, super-block
         int type, bb, steps, row_tiles;  // of the matrix (an indexed read of a parameter is slow)
     };
     auto enter = [&](Where& w) {
@@ -387,22 +388,22 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         w.steps = gm_steps<CH>(w.type);
         w.row_tiles = p.seg[w.seg].row_tiles;
     };
-    auto first_unit = [&]() {
+    auto first_unit = [&](int item) {
         Where w;
-        const int tile = u0 / nb;
-        w.b = u0 - tile * nb;
-        w.row_tile = tile / p.sp.ntile;
-        w.ntile = tile - w.row_tile * p.sp.ntile;
+        w.ntile = item / p.chunks;
+        w.u = (item - w.ntile * p.chunks) * p.sp.U;
+        w.end = min(w.u + p.sp.U, p.total);
+        w.row_tile = w.u / nb;
+        w.b = w.u - w.row_tile * nb;
         w.seg = 0;
         while (w.seg + 1 < p.nseg && w.row_tile >= p.seg[w.seg].row_tiles) w.row_tile -= p.seg[w.seg++].row_tiles;
         enter(w);
         return w;
     };
     auto advance = [&](Where& w) {  // (divisions here, once per super-block and role, had cost 2000 cycles of every 5700)
+        ++w.u;
         if (++w.b < nb) return;
         w.b = 0;
-        if (++w.ntile < p.sp.ntile) return;
-        w.ntile = 0;
         if (++w.row_tile < w.row_tiles || w.seg + 1 == p.nseg) return;
         w.row_tile = 0;
         ++w.seg;
@@ -414,11 +415,12 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
     if (warp == 8) {
         // ================= packed weights: one tiled copy per super-block =================
         if (lane == 0) {
-            Where w = first_unit();
             int s = 0;
+            bool first = true;
             uint32_t parity = 1;  // of the use before
-            for (int u = u0; u < u1; ++u, advance(w)) {
-                if (u - u0 >= NP && !mbar_wait_parked(p_free + s, parity)) {
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
+            for (Where w = first_unit(item); w.u < w.end; advance(w)) {
+                if (!first && !mbar_wait_parked(p_free + s, parity)) {
                     ok = false;
                     break;
                 }
@@ -430,6 +432,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                             w.row_tile * GM_ROWS, tail ? 0 : panel, p_full + s);
                 if (++s == NP) {
                     s = 0;
+                    first = false;
                     parity ^= 1u;
                 }
             }
@@ -441,11 +444,11 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
     } else if (warp == 10 || warp == 11) {
         // ================= activation operands: one bulk copy per 64 values =================
         if (lane == 0) {
-            Where w = first_unit();
             int s = 0, turn = warp - 10;
             bool first = true;
             uint32_t parity = 1;
-            for (int u = u0; u < u1 && ok; ++u, advance(w)) {
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
+            for (Where w = first_unit(item); w.u < w.end && ok; advance(w)) {
                 const int steps = w.steps, g0 = (w.ntile * p.sp.tok) >> 3, ng = min(p.sp.tok >> 3, p.groups - g0);
                 const uint8_t* act = p.act + ((size_t)w.b * 4 * p.groups + g0) * GM_GROUP_BYTES;
                 for (int k = 0; k < steps; ++k, turn ^= 1) {
@@ -493,10 +496,10 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         // operand descriptors of slot 0; the others lie a multiple of 16 bytes further
         const uint64_t desc_a = umma_desc(smem + L.off_a, 2048, 128), desc_b = umma_desc(smem + L.off_b, 128, PAIR ? GM_GROUP_BYTES / 2 : GM_GROUP_BYTES);
         const uint64_t desc_xs = umma_desc(smem + L.off_b, 128, GM_XS_BYTES);
-        Where w = first_unit();
         int s = 0, ds = 0;
         uint32_t parity = 0;
-        for (int u = u0; u < u1 && ok; ++u, advance(w)) {
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
+        for (Where w = first_unit(item); w.u < w.end && ok; advance(w)) {
             const int steps = w.steps;
             for (int k = 0; k < steps; ++k) {
                 if (!mbar_wait_parked(ready + s, parity)) {
@@ -547,17 +550,18 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         };
         constexpr int TURNS = UG / GS;
         const int my_turn = group / GS, sub = group % GS;
-        Where w = first_unit();
-        float d6_next = u0 < u1 ? q6_scale(w) : 0.f;
         int s = 0, turn = 0, ps = 0, hs = GM_HDRS - 1;  // slot, whose turn it is, packed slot, set of factors
-        bool first = true;
+        bool first = true, fresh = true;  // fresh: the first super-block of a chunk
+        float d6_next = 0.f;
         uint32_t parity = 1, p_parity = 0;
-        for (int u = u0; u < u1 && ok; ++u) {
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
+        for (Where w = first_unit(item); w.u < w.end && ok;) {
             const int type = w.type, bb = w.bb, steps = w.steps;
             hs = (hs + 1) % GM_HDRS;
-            const float d6 = d6_next;
+            const float d6 = fresh ? q6_scale(w) : d6_next;
             advance(w);
-            if (u + 1 < u1) d6_next = q6_scale(w);  // a super-block ahead: the latency of a global read
+            fresh = w.u == w.end;
+            if (!fresh) d6_next = q6_scale(w);  // a super-block ahead: the latency of a global read
             if (!mbar_wait_parked(p_full + ps, p_parity)) {  // (every group follows every packed slot, with or without a step in it)
                 ok = false;
                 break;
@@ -700,10 +704,10 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
 #pragma unroll
         for (int t = 0; t < NH / 2; ++t) acc[t] = make_float2(0.f, 0.f);
         if (lane < ND) mbar_arrive(ready + lane);  // no accumulators to wait for at first
-        Where w = first_unit();
         int s = 0, hs = 0, ds = 0, next = ND % NS;  // next: the step that will use these accumulators again
         uint32_t parity = 0;
-        for (int u = u0; u < u1 && ok; ++u, advance(w)) {
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
+        for (Where w = first_unit(item); w.u < w.end && ok; advance(w)) {
             const int steps = w.steps;
             float2 f = make_float2(0.f, 0.f);
             for (int k = 0; k < steps; ++k) {
@@ -764,13 +768,12 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 }
             }
             hs = (hs + 1) % GM_HDRS;
-            if (ok && (w.b == nb - 1 || u == u1 - 1)) {  // this block's part of the tile is complete
-                const int tile = u / nb;
-                const int first = tile * nb / p.sp.U;
+            if (ok && (w.b == nb - 1 || w.u == w.end - 1)) {  // this chunk's part of the tile is complete
+                const int part = (w.u / p.sp.U) - (w.u - w.b) / p.sp.U;
                 int row = w.row_tile * GM_ROWS + r;
                 const bool valid = row < p.seg[w.seg].rows;
                 for (int e = 0; e < w.seg; ++e) row += p.seg[e].row_tiles * GM_ROWS;
-                float* dst = p.y + (size_t)(blockIdx.x - first) * p.part_stride + row;
+                float* dst = p.y + (size_t)part * p.part_stride + row;
 #pragma unroll
                 for (int t = 0; t < NH; ++t) {
                     const int tok = w.ntile * p.sp.tok + NH * half + t;

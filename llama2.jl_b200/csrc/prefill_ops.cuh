@@ -47,7 +47,7 @@ __global__ void rope_kv_kernel(const __grid_constant__ RopeKvParams p) {
     float* const kc = p.kc + (p.pos_list ? (size_t)t * p.cache_stride : 0);
     float* const vc = p.vc + (p.pos_list ? (size_t)t * p.cache_stride : 0);
     auto sum = [&](int row) {
-        const int parts = gm_parts(p.sp, gm_tile(p.sp, row, t));
+        const int parts = gm_parts(p.sp, row);
         const float* src = p.y + (size_t)t * p.ldy + row;
         float v = __ldcg(src);
         for (int i = 1; i < parts; ++i) v += __ldcg(src + i * p.part_stride);

@@ -1,0 +1,69 @@
+"""Products of a resident matrix with many columns on device pointers (l2b_matrix_matmul_device): its workspace."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def resident(pkg, synth):
+    """(type, in, out) -> matmul(x, y, columns) on the current stream."""
+    import torch
+    from llama2_jl_b200 import _lib as L
+    handles = []
+
+    def make(t, n_in, n_out):
+        A = synth.matrix(t, n_in, n_out, seed=n_in + n_out)
+        h = C.c_void_p()
+        L.check(L.lib().l2b_matrix_create(t, L.ptr(A.data), n_in, n_out, 1, C.byref(h)))
+        handles.append(h)
+        return A, lambda x, y, n: L.check(L.lib().l2b_matrix_matmul_device(h, 0, x.data_ptr(), n, y.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    yield make
+    torch.cuda.synchronize()
+    for h in handles:
+        L.lib().l2b_matrix_destroy(h)
+
+
+# at both shapes the smaller count falls into more partial results than the larger one when the cuts hang on the columns
+@pytest.mark.parametrize("n_in,n_out,most,fewer", [(4096, 14336, 513, (129, 16)), (4096, 4096, 257, (54, 128, 1)), (2048, 300, 130, (129, 17))])
+def test_only_more_columns_allocate(resident, n_in, n_out, most, fewer):
+    """Calls with fewer columns than an earlier one take no memory, and a graph that holds the earlier one stays good."""
+    import torch
+    A, matmul = resident(12, n_in, n_out)
+    x = torch.randn((most, n_in), generator=torch.Generator(device="cuda").manual_seed(n_out), device="cuda")
+    y, z = torch.zeros((most, n_out), device="cuda"), torch.zeros((most, n_out), device="cuda")
+    matmul(x, y, most)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        matmul(x, z, most)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, z)
+    free = torch.cuda.mem_get_info()[0]
+    for n in fewer:
+        matmul(x, y, n)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
+    for n in fewer:
+        part = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(part):  # (a call that allocated would be refused here)
+            matmul(x, y, n)
+        y.zero_()
+        part.replay()
+        want = x[:n].double() @ torch.from_numpy(_dense(A)).cuda().double().T
+        assert (y[:n] - want).abs().max() <= 4e-6 * want.abs().max()
+        assert (y[n:] == 0).all()
+    x.copy_(-x)
+    z.zero_()
+    graph.replay()
+    matmul(x, y, most)
+    assert torch.equal(y, z)
+
+
+def _dense(A):
+    from llama2_jl_b200 import _lib as L
+    out = np.empty((A.out_dim, A.in_dim), np.float32)
+    L.check(L.lib().l2b_dequantize(A.ggml_type, L.ptr(A.data), out.size, L.ptr(out)))
+    return out
