@@ -515,6 +515,24 @@ static int32_t launch_product(const DevMatrix& w, const GemmInput& in, int n_tok
     return L2B_OK;
 }
 
+// Any number of columns, y[ncols][out] = x[ncols][in] times the matrix: PRODUCT_SLAB columns at a time, whose operands and partial results
+// are all that the workspace holds (eight token tiles: every SM has work, and the launches of a slab are 1 % of it).
+constexpr int PRODUCT_SLAB = 1024;
+static size_t product_operand_bytes(const DevMatrix& w, int n_tok) { return (gemm_input_bytes(w.in, n_tok) + 255) & ~(size_t)255; }
+static size_t columns_workspace(const DevMatrix& w, int ncols, int sms) {
+    const int n = std::min(ncols, PRODUCT_SLAB);
+    return product_operand_bytes(w, n) + gemm_product_bytes(w, n, sms);
+}
+static int32_t launch_columns(const DevMatrix& w, const float* x, int ncols, float* y, uint8_t* workspace, int sms, int* status, cudaStream_t st) {
+    for (int c = 0; c < ncols; c += PRODUCT_SLAB) {
+        const int n = std::min(ncols - c, PRODUCT_SLAB);
+        const GemmInput in = gemm_input(workspace, w.in, n);
+        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(const_cast<float*>(x) + (size_t)c * w.in, nullptr, (int)w.in, n, in), st));
+        L2B_TRY(launch_product(w, in, n, y + (size_t)c * w.out, (float*)(workspace + product_operand_bytes(w, n)), sms, status, st));
+    }
+    return L2B_OK;
+}
+
 // Buffers of a many-token pass: activations of up to PF_MAX_TOK tokens, attention scratch, quantised activations.
 struct GemmBufs {
     float *x = nullptr, *q = nullptr, *att = nullptr, *h = nullptr;  // residual stream, rotated queries, attention output, SwiGLU output
@@ -2903,7 +2921,7 @@ extern "C" int32_t l2b_matrix_matmul_device(l2b_matrix* m, int32_t copy, const f
     const DevMatrix& w = m->copies[copy];
     if (!gemm_supported(w)) return fail(L2B_ERR_UNSUPPORTED_TYPE, "the tensor-core GEMM takes q4_K and q5_K matrices");
     CU(cudaSetDevice(m->device));
-    const size_t in_bytes = (gemm_input_bytes(w.in, ncols) + 255) & ~(size_t)255, need = in_bytes + gemm_product_bytes(w, ncols, m->di.sms);
+    const size_t need = columns_workspace(w, ncols, m->di.sms);
     if (need > m->act_bytes) {
         if (m->act) cudaFree(m->act);
         m->act = nullptr;
@@ -2911,9 +2929,7 @@ extern "C" int32_t l2b_matrix_matmul_device(l2b_matrix* m, int32_t copy, const f
         CU(cudaMalloc(&m->act, need));
         m->act_bytes = need;
     }
-    const GemmInput in = gemm_input(m->act, w.in, ncols);
-    L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(const_cast<float*>(dev_x), nullptr, (int)w.in, ncols, in), (cudaStream_t)stream));
-    return launch_product(w, in, ncols, dev_y, (float*)(m->act + in_bytes), m->di.sms, m->status, (cudaStream_t)stream);
+    return launch_columns(w, dev_x, ncols, dev_y, m->act, m->di.sms, m->status, (cudaStream_t)stream);
 }
 
 extern "C" int32_t l2b_matrix_matvec_device(l2b_matrix* m, int32_t copy, const float* dev_x, float* dev_y, int32_t planes, void* stream) {
@@ -2949,12 +2965,9 @@ extern "C" int32_t l2b_matrix_matvec(l2b_matrix* m, const float* host_x, int32_t
     // instead of one matrix-vector pass per column.  L2B_GEMM_MIN_COLS sets the threshold (default 4; 0 switches it off).
     const long gemm_min = env_long("L2B_GEMM_MIN_COLS", 4);
     if (gemm_min > 0 && ncols >= gemm_min && (planes == 0 || planes == 3) && gemm_supported(w)) {
-        DevBuf act, parts;
-        L2B_TRY(dev_alloc(act, gemm_input_bytes(w.in, ncols)));
-        L2B_TRY(dev_alloc(parts, gemm_product_bytes(w, ncols, m->di.sms)));
-        const GemmInput in = gemm_input(act.as<uint8_t>(), w.in, ncols);
-        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(x.as<float>(), nullptr, (int)w.in, ncols, in), nullptr));
-        L2B_TRY(launch_product(w, in, ncols, y.as<float>(), parts.as<float>(), m->di.sms, m->status, nullptr));
+        DevBuf workspace;
+        L2B_TRY(dev_alloc(workspace, columns_workspace(w, ncols, m->di.sms)));
+        L2B_TRY(launch_columns(w, x.as<float>(), ncols, y.as<float>(), workspace.as<uint8_t>(), m->di.sms, m->status, nullptr));
     } else {
         for (int c = 0; c < ncols; ++c)
             L2B_TRY(l2b_matrix_matvec_device(m, 0, x.as<float>() + (size_t)c * w.in, y.as<float>() + (size_t)c * w.out, planes, nullptr));

@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const __grid_constant__
     }
 }
 
-// A product that is wanted as such: dst[t][i] = the sum of its partial results.  Grid (blocks per row, n_tok).
+// A product that is wanted as such: dst[t][i] = the sum of its partial results.  Grid (blocks per row, n_tok): at most 65535 tokens.
 __global__ void sum_parts_kernel(const float* __restrict__ y, size_t part_stride, const __grid_constant__ GemmSplit sp, int ldy, int rows, float* __restrict__ dst) {
     const int tok = blockIdx.y;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {

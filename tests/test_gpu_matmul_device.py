@@ -62,6 +62,25 @@ def test_only_more_columns_allocate(resident, n_in, n_out, most, fewer):
     assert torch.equal(y, z)
 
 
+def test_more_columns_than_a_grid_holds(resident):
+    """70 000 columns of a matrix whose products are added up from parts, in a workspace of a thousand; columns at the cuts and the ends."""
+    import torch
+    n_in, n_out, n = 2560, 130, 70000
+    A, matmul = resident(13, n_in, n_out)
+    x = torch.randn((n, n_in), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    y = torch.full((n, n_out), float("nan"), device="cuda")
+    matmul(x, y, 16)  # (kernels are loaded by their first call)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    matmul(x, y, n)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 64 << 20
+    assert torch.isfinite(y).all()
+    some = torch.tensor([0, 127, 128, 1023, 1024, 1025, 65535, 65536, 69000, n - 1], device="cuda")
+    want = x[some].double() @ torch.from_numpy(_dense(A)).cuda().double().T
+    assert (y[some] - want).abs().max() <= 4e-6 * want.abs().max()
+
+
 def _dense(A):
     from llama2_jl_b200 import _lib as L
     out = np.empty((A.out_dim, A.in_dim), np.float32)
