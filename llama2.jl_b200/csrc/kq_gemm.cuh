@@ -23,7 +23,8 @@
 //                     cycles to see a slot free and issue a copy, so two take turns
 //   unpack warps      groups of four; thread = row: nibbles -> fp16 times scale, into core matrices (8 rows x 16 bytes)
 //   MMA warp          tcgen05.mma.kind::f16 (M 128, K 16), four or eight per 64 values
-//   8 epilogue warps  thread = weight row, half of the tokens: tensor memory -> times d -> f32 accumulators
+//   8 epilogue warps  thread = weight row, half of the tokens: tensor memory -> times d -> f32 accumulators, and those of four
+//                     super-blocks -> f32 sums in tensor memory (one chain over 14336 values would be 280 roundings long)
 //
 // Every mbarrier wait is bounded; a wait that runs out sets the status word, after which the block drains and still frees
 // its tensor memory.
@@ -103,6 +104,7 @@ struct GmCfg {
     static constexpr bool PAIR = NT == 32;
     static constexpr int CCOLS = PAIR ? 2 * NT : NT;            // accumulator columns per chunk
     static constexpr int DCOLS = CH == 1 ? NT : 2 * CCOLS + NT;  // per slot: 128, 192, 160
+    static_assert(ND * DCOLS + NT <= 512, "the sums stand behind the accumulators");
     static constexpr int THREADS = (GM_EPI_WARPS + 4 + 4 * UG) * 32;  // warps 0-7 epilogue, 8 packed copies, 9 MMA, 10 and 11 operand copies, 12 .. unpack
 };
 constexpr int GM_MAX_PACKED = 5;
@@ -380,13 +382,11 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
     struct Where {
         int u, end;                  // unit, first one behind the chunk
         int seg, row_tile, ntile, b; // matrix, its row tile, token tile, super-block
-        int type, bb, steps, row_tiles;  // of the matrix (an indexed read of a parameter is slow)
+        int type, steps;             // of the matrix (an indexed read of a parameter is slow)
     };
     auto enter = [&](Where& w) {
         w.type = p.seg[w.seg].type;
-        w.bb = dev_block_bytes(w.type);
         w.steps = gm_steps<CH>(w.type);
-        w.row_tiles = p.seg[w.seg].row_tiles;
     };
     auto first_unit = [&](int item) {
         Where w;
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         ++w.u;
         if (++w.b < nb) return;
         w.b = 0;
-        if (++w.row_tile < w.row_tiles || w.seg + 1 == p.nseg) return;
+        if (++w.row_tile < p.seg[w.seg].row_tiles || w.seg + 1 == p.nseg) return;
         w.row_tile = 0;
         ++w.seg;
         enter(w);
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                     break;
                 }
                 const GemmSeg& sg = p.seg[w.seg];
-                const int bb = w.bb, panel = w.b / sg.kb;
+                const int bb = dev_block_bytes(w.type), panel = w.b / sg.kb;
                 mbar_arrive_expect_tx(p_full + s, (uint32_t)(GM_ROWS * bb));
                 const bool tail = (panel + 1) * sg.kb > nb;
                 tma_load_3d(smem + L.off_packed + s * L.slot_packed, tail ? &maps.tail[w.seg] : &maps.main[w.seg], (w.b - panel * sg.kb) * bb,
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         uint32_t parity = 1, p_parity = 0;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
         for (Where w = first_unit(item); w.u < w.end && ok;) {
-            const int type = w.type, bb = w.bb, steps = w.steps;
+            const int type = w.type, bb = dev_block_bytes(type), steps = w.steps;
             hs = (hs + 1) % GM_HDRS;
             const float d6 = fresh ? q6_scale(w) : d6_next;
             advance(w);
@@ -704,6 +704,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
 #pragma unroll
         for (int t = 0; t < NH / 2; ++t) acc[t] = make_float2(0.f, 0.f);
         if (lane < ND) mbar_arrive(ready + lane);  // no accumulators to wait for at first
+        bool held = false;  // sums of this part are in tensor memory
         int s = 0, hs = 0, ds = 0, next = ND % NS;  // next: the step that will use these accumulators again
         uint32_t parity = 0;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
@@ -768,7 +769,27 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 }
             }
             hs = (hs + 1) % GM_HDRS;
-            if (ok && (w.b == nb - 1 || w.u == w.end - 1)) {  // this chunk's part of the tile is complete
+            const bool last = w.b == nb - 1 || w.u == w.end - 1;  // this chunk's part of the tile is complete
+            if (ok && (last || ((w.b + 1) & (w.type == T_Q6_K ? 1 : 3)) == 0)) {  // 20 (q6_K: 16) values have been added up
+                const uint32_t sums = taddr + (uint32_t)(ND * DCOLS + NH * half);
+#pragma unroll
+                for (int c0 = 0; c0 < NH; c0 += 16) {
+                    if (!held || c0 >= mine) break;
+                    float v[16];
+                    tmem_ld16f(sums + (uint32_t)c0, v);
+#pragma unroll
+                    for (int t = 0; t < 16; t += 2) acc[(c0 + t) / 2] = make_float2(v[t] + acc[(c0 + t) / 2].x, v[t + 1] + acc[(c0 + t) / 2].y);
+                }
+                if (!last) {
+#pragma unroll
+                    for (int c0 = 0; c0 < NH; c0 += 16)
+                        if (c0 < mine) tmem_st16f(sums + (uint32_t)c0, reinterpret_cast<const float(&)[16]>(acc[c0 / 2]));
+#pragma unroll
+                    for (int t = 0; t < NH / 2; ++t) acc[t] = make_float2(0.f, 0.f);
+                }
+                held = !last;
+            }
+            if (ok && last) {
                 const int part = (w.u / p.sp.U) - (w.u - w.b) / p.sp.U;
                 int row = w.row_tile * GM_ROWS + r;
                 const bool valid = row < p.seg[w.seg].rows;

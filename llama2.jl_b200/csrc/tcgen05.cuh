@@ -115,7 +115,7 @@ __device__ __forceinline__ void tmem_st1f(uint32_t taddr, float v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "f"(v) : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// 16 consecutive columns of this thread's tensor-memory lane
+// 16 consecutive columns of this thread's tensor-memory lane: load and store
 __device__ __forceinline__ void tmem_ld16f(uint32_t taddr, float (&v)[16]) {
     int r[16];
     asm volatile(
@@ -127,6 +127,14 @@ __device__ __forceinline__ void tmem_ld16f(uint32_t taddr, float (&v)[16]) {
         : "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __int_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_st16f(uint32_t taddr, const float (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n\t"
+        "tcgen05.wait::st.sync.aligned;" ::"r"(taddr),
+        "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]),
+        "f"(v[13]), "f"(v[14]), "f"(v[15])
+        : "memory");
 }
 // 32 consecutive columns of this thread's tensor-memory lane: load and store
 __device__ __forceinline__ void tmem_ld32f(uint32_t taddr, float (&v)[32]) {

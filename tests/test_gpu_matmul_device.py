@@ -81,6 +81,22 @@ def test_more_columns_than_a_grid_holds(resident):
     assert (y[some] - want).abs().max() <= 4e-6 * want.abs().max()
 
 
+@pytest.mark.parametrize("t", [12, 13])
+def test_long_rows_keep_their_precision(resident, t):
+    """56 super-blocks in one sum.  2.05e-7 is the relative error (2-norms, against 64 bits) of such rows with exact integer sums inside each
+    super-block and one f32 addition behind it; a chain over every 64 values (280 additions) is at 2.9e-7."""
+    import torch
+    n_in, n_out, n = 14336, 133 * 128, 128
+    A, matmul = resident(t, n_in, n_out)
+    x = torch.randn((n, n_in), generator=torch.Generator(device="cuda").manual_seed(t), device="cuda")
+    for cols in (16, 48, 128):
+        y = torch.empty((cols, n_out), device="cuda")
+        matmul(x, y, cols)
+        for first in (0, n_out - 512):
+            want = x[:cols].double() @ torch.from_numpy(_dense(A.rows(first, first + 512))).cuda().double().T
+            assert (y[:, first:first + 512] - want).norm() < 2.05e-7 * want.norm(), cols
+
+
 def _dense(A):
     from llama2_jl_b200 import _lib as L
     out = np.empty((A.out_dim, A.in_dim), np.float32)
