@@ -93,17 +93,15 @@ struct GemmMaps {
 // last use by parity, so it must have seen the use before that: its own last step lies at most NS steps back, UG / GS <= NS.  (More groups
 // are no help: all read the scales of every super-block they take part in, 200 instructions a row, which with four groups on the steps
 // of one super-block made the kernel issue-bound.)
-// PAIR: high and low terms are columns of one MMA (half as many instructions, each of which reads the 4 KiB of A again: 32 cycles
-// whatever its columns); with 64 tokens the MMAs themselves take as long, with 128 the sums would not fit tensor memory.
+// Whatever the tile holds, a column's sums are the same ones in the same order: low terms, then high terms of 64 values in one accumulator,
+// added to the f32 sum chunk by chunk, the shared part behind them.  So a column's result does not hang on how many columns came with it.
 template <int NT>
 struct GmCfg {
     static constexpr int CH = NT == 128 ? 1 : 2;
     static constexpr int NS = NT == 64 ? 2 : 3, ND = NS;
     static constexpr int GS = NT == 64 ? 2 : 1, UG = NT == 128 ? 2 : NT == 64 ? 4 : 3;
     static_assert(UG / GS <= NS, "a group would miss a phase");
-    static constexpr bool PAIR = NT == 32;
-    static constexpr int CCOLS = PAIR ? 2 * NT : NT;            // accumulator columns per chunk
-    static constexpr int DCOLS = CH == 1 ? NT : 2 * CCOLS + NT;  // per slot: 128, 192, 160
+    static constexpr int DCOLS = CH == 1 ? NT : 3 * NT;  // accumulator columns per slot: 128, 192, 96
     static_assert(ND * DCOLS + NT <= 512, "the sums stand behind the accumulators");
     static constexpr int THREADS = (GM_EPI_WARPS + 4 + 4 * UG) * 32;  // warps 0-7 epilogue, 8 packed copies, 9 MMA, 10 and 11 operand copies, 12 .. unpack
 };
@@ -283,11 +281,6 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)), "l"(*reinterpret_cast<unsigned long long*>(&c)));
     return *reinterpret_cast<float2*>(&r);
 }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
-    return *reinterpret_cast<float2*>(&r);
-}
 
 // ---- unpacking -------------------------------------------------------------------------------------------
 __device__ __forceinline__ __half2 h2_bits(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
@@ -339,8 +332,7 @@ __device__ __forceinline__ int gm_steps(int type) { return CH == 2 ? (type == T_
 
 template <int NT>
 __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ GemmMaps maps) {
-    constexpr int NS = GmCfg<NT>::NS, ND = GmCfg<NT>::ND, UG = GmCfg<NT>::UG, GS = GmCfg<NT>::GS, DCOLS = GmCfg<NT>::DCOLS, CH = GmCfg<NT>::CH, CCOLS = GmCfg<NT>::CCOLS;
-    constexpr bool PAIR = GmCfg<NT>::PAIR;
+    constexpr int NS = GmCfg<NT>::NS, ND = GmCfg<NT>::ND, UG = GmCfg<NT>::UG, GS = GmCfg<NT>::GS, DCOLS = GmCfg<NT>::DCOLS, CH = GmCfg<NT>::CH;
     const int NP = p.np;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the copies and operands want their alignment
@@ -492,9 +484,9 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         }
     } else if (warp == 9) {
         // ================= MMA issue: the whole warp walks along, one thread issues =================
-        const uint32_t idesc = umma_idesc_f16(GM_ROWS, PAIR ? 2 * p.sp.tok : p.sp.tok), idesc_xs = umma_idesc_f16(GM_ROWS, p.sp.tok);
+        const uint32_t idesc = umma_idesc_f16(GM_ROWS, p.sp.tok);
         // operand descriptors of slot 0; the others lie a multiple of 16 bytes further
-        const uint64_t desc_a = umma_desc(smem + L.off_a, 2048, 128), desc_b = umma_desc(smem + L.off_b, 128, PAIR ? GM_GROUP_BYTES / 2 : GM_GROUP_BYTES);
+        const uint64_t desc_a = umma_desc(smem + L.off_a, 2048, 128), desc_b = umma_desc(smem + L.off_b, 128, GM_GROUP_BYTES);
         const uint64_t desc_xs = umma_desc(smem + L.off_b, 128, GM_XS_BYTES);
         int s = 0, ds = 0;
         uint32_t parity = 0;
@@ -515,17 +507,17 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
 #pragma unroll
                         for (int c = 0; c < CH; ++c)
 #pragma unroll
-                            for (int t = PAIR ? 0 : 1; t >= 0; --t)  // low terms of X first
+                            for (int t = 1; t >= 0; --t)  // low terms of X first
 #pragma unroll
                                 for (int kk = 0; kk < 4; ++kk)
-                                    umma_f16(d + (uint32_t)(c * CCOLS), da + (uint64_t)((c * GM_A_BYTES + kk * 4096) >> 4),
-                                             db + (uint64_t)((c * chunk_b + t * 1024 + kk * 256) >> 4), idesc, t == (PAIR ? 0 : 1) && kk == 0 ? 0u : 1u);
+                                    umma_f16(d + (uint32_t)(c * NT), da + (uint64_t)((c * GM_A_BYTES + kk * 4096) >> 4),
+                                             db + (uint64_t)((c * chunk_b + t * 1024 + kk * 256) >> 4), idesc, t == 1 && kk == 0 ? 0u : 1u);
                     }
                     if (shared_part) {  // low terms of C first
                         const uint64_t ax = da + (uint64_t)(CH == 2 ? (2 * GM_A_BYTES) >> 4 : 0), dx = desc_xs + (uint64_t)((s * L.slot_b + (CH == 2 ? 2 * chunk_b : 0)) >> 4);
-                        const uint32_t dd = d + (uint32_t)(CH == 2 ? 2 * CCOLS : 0);
-                        umma_f16(dd, ax + (4096 >> 4), dx, idesc_xs, 0u);
-                        umma_f16(dd, ax, dx, idesc_xs, 1u);
+                        const uint32_t dd = d + (uint32_t)(CH == 2 ? 2 * NT : 0);
+                        umma_f16(dd, ax + (4096 >> 4), dx, idesc, 0u);
+                        umma_f16(dd, ax, dx, idesc, 1u);
                     }
                     umma_commit(done + s);
                 }
@@ -721,30 +713,16 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 const bool shared_part = k == (CH == 2 ? 1 : 4) && (CH == 2 ? steps == 2 : steps == 5);
                 const float2 md = make_float2(f.x, f.x), mc = make_float2(f.y, f.y);
                 const uint32_t td = taddr + (uint32_t)(ds * DCOLS);
-                if (PAIR) {  // two chunks; columns in eights: high terms of eight tokens, then their low terms
-#pragma unroll
-                    for (int c0 = 0; c0 < NH; c0 += 8) {
-                        if (c0 >= mine) break;
-                        float v[16], w2[16];
-                        tmem_ld16f(td + (uint32_t)(2 * (NH * half + c0)), v);
-                        tmem_ld16f(td + (uint32_t)(CCOLS + 2 * (NH * half + c0)), w2);
-#pragma unroll
-                        for (int t = 0; t < 8; t += 2) {
-                            const float2 hi = add2(make_float2(v[t], v[t + 1]), make_float2(w2[t], w2[t + 1]));
-                            const float2 lo = add2(make_float2(v[8 + t], v[9 + t]), make_float2(w2[8 + t], w2[9 + t]));
-                            acc[(c0 + t) / 2] = fma2(md, add2(hi, lo), acc[(c0 + t) / 2]);
-                        }
-                    }
-                } else if (CH == 2) {
+                if (CH == 2) {
 #pragma unroll
                     for (int c0 = 0; c0 < NH; c0 += 16) {
                         if (c0 >= mine) break;
                         float v[16], w2[16];
                         tmem_ld16f(td + (uint32_t)(NH * half + c0), v);
-                        tmem_ld16f(td + (uint32_t)(CCOLS + NH * half + c0), w2);
+                        tmem_ld16f(td + (uint32_t)(NT + NH * half + c0), w2);
 #pragma unroll
                         for (int t = 0; t < 16; t += 2)
-                            acc[(c0 + t) / 2] = fma2(md, add2(make_float2(v[t], v[t + 1]), make_float2(w2[t], w2[t + 1])), acc[(c0 + t) / 2]);
+                            acc[(c0 + t) / 2] = fma2(md, make_float2(w2[t], w2[t + 1]), fma2(md, make_float2(v[t], v[t + 1]), acc[(c0 + t) / 2]));
                     }
                 }
                 if (CH == 1 || shared_part) {
@@ -753,7 +731,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                     for (int c0 = 0; c0 < NH; c0 += 16) {
                         if (c0 >= mine) break;
                         float v[16];
-                        tmem_ld16f(td + (uint32_t)((CH == 2 ? 2 * CCOLS : 0) + NH * half + c0), v);
+                        tmem_ld16f(td + (uint32_t)((CH == 2 ? 2 * NT : 0) + NH * half + c0), v);
 #pragma unroll
                         for (int t = 0; t < 16; t += 2) acc[(c0 + t) / 2] = fma2(mm, make_float2(v[t], v[t + 1]), acc[(c0 + t) / 2]);
                     }

@@ -41,6 +41,21 @@ def test_q6_k_classifier_of_batches(pkg, orc, synth, n_seq):
     model.close()
 
 
+def test_a_sequence_has_the_same_bits_in_any_batch(pkg, synth):
+    cfg = pkg.ModelConfig(512, 768, 2, 4, 2, 1024, 8, 10000.0, False)
+    model = pkg.LanguageModel(cfg, None, synth.model_weights(cfg, dict(synth.ALL(12), w2=13, output=14), seed=5))
+    ids = synth.tokens(3 * 130, 9, 3, cfg.vocab_size).reshape(3, 130)
+    logits = {}
+    for n_seq in (130, 70, 33, 2):
+        batch = pkg.BatchRunState(model, n_seq)
+        for i in range(3):
+            batch.decode_next(ids[i, :n_seq], np.full(n_seq, i, np.int32), want_logits=i == 2)
+        logits[n_seq] = np.array(batch.logits)
+        batch.close()
+        assert np.array_equal(logits[n_seq], logits[130][:n_seq]), n_seq
+    model.close()
+
+
 @pytest.mark.parametrize("n", [10, 512, 513, 514])
 def test_prompts_around_the_longest_pass(pkg, orc, synth, n):
     """A pass holds 512 tokens; up to there the last position is in it.  Generation goes on behind it."""
