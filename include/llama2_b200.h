@@ -218,7 +218,8 @@ int32_t l2b_session_extend(l2b_session* session, const int32_t* tokens, int32_t 
 /* *min_tokens > 0: runs of at least that many prompt positions that are all followed by a prompt token go through the
  * many-token pass (products on the tensor cores, tcgen05 + TMA, up to 128 tokens per pass over a weight tile; up to 512 tokens
  * per pass over the layers).  0: not available for this model (needs q4_K / q5_K layer matrices, three
- * activation planes, one GPU; L2B_PREFILL_GEMM=0 switches it off) -- prompts then go through the decode kernels.  The reference
+ * activation planes, one GPU; L2B_PREFILL_GEMM=0 switches it off; L2B_PROMPT_ATTENTION, read by a session's first prompt, asks
+ * for its tiled (1) or its split (2) attention kernel instead of the quicker one) -- prompts then go through the decode kernels.  The reference
  * feeds prompts token by token (src/inference.jl:349-356). */
 int32_t l2b_session_prefill_gemm(l2b_session* session, int32_t* min_tokens);
 /* 1 when l2b_generate feeds prompts two positions per pass (k-quant model, three activation planes, one GPU, everything fits in

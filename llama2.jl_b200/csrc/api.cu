@@ -543,6 +543,7 @@ struct GemmBufs {
     uint8_t* act = nullptr;
     int nsplit = 1;
     int sms = 0;
+    int attention = 0;  // of prompt passes: 0 by the rule, 1 the tiled kernel wherever the heads allow it, 2 the split kernel
 };
 
 static void free_gemm_bufs(GemmBufs& B) {
@@ -1896,8 +1897,9 @@ constexpr int STACK_MIN_ROWS = 2;  // layer-stack models
 // Attention of one sequence's tokens at pos0 ..: heads of a multiple of 16 values, at most 128, take the tensor-core kernel.
 // A block of it takes about 10 us and 7.5 us per 64 positions, the split kernel about 5 us and 1 us per 10000 pairs of a query head and a position
 // (measured: 29 queries behind 211 positions, 32 heads: 40 against 25 us; 128 queries: 26 and 25; 512 queries of 2048: 97 against 1280).
-static bool prompt_attention_better(int n, int pos0, int n_heads, int gq, int hs, int sms) {
+static bool prompt_attention_better(int n, int pos0, int n_heads, int gq, int hs, int sms, int asked) {
     if (hs % 16 != 0 || hs > PA_MAX_HS) return false;
+    if (asked) return asked == 1;
     const int tq = PA_ROWS / gq, blocks = (n + tq - 1) / tq * (n_heads / gq), waves = (blocks + sms - 1) / sms;
     const double tiled = 10.0 + 7.5 * waves * ((pos0 + n + PA_KEYS - 1) / PA_KEYS), split = 5.0 + 1e-4 * n_heads * n * (pos0 + 0.5 * n);
     return tiled < split;
@@ -1959,7 +1961,7 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
         r.pos_list = pos_list; r.cache_stride = seq_stride;
         rope_kv_kernel<<<dim3(8, n), 256, 0, st>>>(r);
         CU(cudaGetLastError());
-        if (!pos_list && prompt_attention_better(n, pos0, c.n_heads, gq, hs, B.sms)) {
+        if (!pos_list && prompt_attention_better(n, pos0, c.n_heads, gq, hs, B.sms, B.attention)) {
             PromptAttnParams a;
             a.q = B.q; a.kc = kcl; a.vc = vcl; a.out = B.att; a.n = n; a.pos0 = pos0; a.q_stride = c.dim;
             a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.hs = hs; a.seq_len = c.seq_len; a.status = status;
@@ -2005,6 +2007,7 @@ static bool alloc_gemm_bufs(const l2b_model* m, GemmBufs& B, size_t T, bool batc
     DeviceInfo di;
     if (query_device(di) != L2B_OK) return false;
     B.sms = di.sms;
+    B.attention = (int)env_long("L2B_PROMPT_ATTENTION", 0);
     B.nsplit = c.seq_len >= 2048 ? 4 : 1;
     const LayerW& w = m->layers[0];  // every layer has these shapes
     auto need = [&](std::initializer_list<const DevMatrix*> ws, size_t n) {

@@ -1,14 +1,38 @@
 """Attention of prompt passes on the tensor cores (csrc/prompt_attention.cuh) against the CPU oracle, through the C ABI: prompts around the
-64-position and 128-row tiles, head sizes around its limits, every number of heads per key / value head."""
+64-position and 128-row tiles, head sizes around its limits, every number of heads per key / value head.  Passes as short as these would take
+the split kernel by themselves, so each kernel is asked for."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(params=["tiled", "split"])
+def kernel(request, monkeypatch):
+    monkeypatch.setenv("L2B_PROMPT_ATTENTION", {"tiled": "1", "split": "2"}[request.param])
+    return request.param
+
+
+def test_the_kernel_that_was_asked_for_runs(pkg, synth, monkeypatch):
+    """The two differ in the order of their sums, so their bits differ; a head size that the tiled one does not take leaves no choice."""
+    for dim, heads, same in ((1024, 8, False), (512, 64, True)):
+        cfg = pkg.ModelConfig(dim, 512, 2, heads, heads, 512, 128, 10000.0, False)
+        w = synth.model_weights(cfg, dict(synth.ALL(12), output=14), seed=1)
+        logits = []
+        for asked in ("1", "2", "1"):
+            monkeypatch.setenv("L2B_PROMPT_ATTENTION", asked)
+            model = pkg.LanguageModel(cfg, None, w)
+            st = pkg.RunState(model)
+            pkg.prefill(st, synth.tokens(100, 2, 3, cfg.vocab_size), 0)
+            logits.append(np.array(st.logits))
+            model.close()
+        assert np.array_equal(logits[0], logits[2])
+        assert np.array_equal(logits[0], logits[1]) == same
+
+
 @pytest.mark.parametrize("dim,heads,kv,neox", [(768, 8, 8, True), (1024, 8, 2, False), (512, 16, 16, False), (1024, 8, 1, False), (768, 6, 1, False), (768, 16, 8, False), (256, 16, 8, False)])
 @pytest.mark.parametrize("first,second", [(0, 13), (0, 64), (0, 65), (63, 66), (130, 127)])
-def test_prompt_passes_against_oracle(pkg, orc, synth, dim, heads, kv, neox, first, second):
+def test_prompt_passes_against_oracle(pkg, orc, synth, kernel, dim, heads, kv, neox, first, second):
     """`first` positions, then `second` more in one pass (head sizes 96, 128, 32, 128, 128 with six heads per key head, 48, 16): logits of the
     last position and of one decoded behind the pass.  Bound: that of the other prompt tests, 5e-5 of the logits' range."""
     cfg = pkg.ModelConfig(dim, 512, 2, heads, kv, 512, 320, 10000.0, neox)
