@@ -49,3 +49,29 @@ def test_prompt_passes_against_oracle(pkg, orc, synth, kernel, dim, heads, kv, n
             pkg.transformer_(int(ids[-1]), pos, cfg, st)
         assert np.abs(st.logits - want[pos]).max() / float(want[pos].max() - want[pos].min()) < 5e-5, pos
     model.close()
+
+
+def test_positions_behind_do_not_matter(pkg, synth, kernel):
+    """Two prompts that differ from position 60 on, the second with an id there whose embedding is infinite: the rows before it in the cache have
+    the same bits, which position 59, fed once more, shows in its logits."""
+    cfg = pkg.ModelConfig(1024, 512, 3, 8, 2, 512, 160, 10000.0, False)
+    w = synth.model_weights(cfg, dict(synth.ALL(12), output=14), seed=3)
+    emb = w.token_embedding_table
+    row = emb.data.size // cfg.vocab_size
+    data = np.array(emb.data)
+    data[7 * row:7 * row + 2] = np.array([0x7C00], np.uint16).view(np.uint8)  # d of the id's first super-block
+    w.token_embedding_table = pkg.QuantMatrix(emb.ggml_type, data, emb.in_dim, emb.out_dim)
+    model = pkg.LanguageModel(cfg, None, w)
+    ids = synth.tokens(100, 4, 8, cfg.vocab_size)
+    logits = []
+    for tail in (ids[60:], np.concatenate([[7], ids[60:99][::-1]]).astype(ids.dtype)):
+        st = pkg.RunState(model)
+        try:
+            pkg.prefill(st, np.concatenate([ids[:60], tail]), 0)
+        except pkg.L2BError:
+            assert tail[0] == 7  # its own logits, and those behind, are not numbers
+        pkg.transformer_(int(ids[59]), 59, cfg, st)
+        logits.append(np.array(st.logits))
+    assert np.isfinite(logits[0]).all()
+    assert np.array_equal(logits[0], logits[1])
+    model.close()
