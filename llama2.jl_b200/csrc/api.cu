@@ -541,6 +541,7 @@ struct GemmBufs {
     float *pm = nullptr, *pl = nullptr, *pacc = nullptr;
     int* tickets = nullptr;
     uint8_t* act = nullptr;
+    int tokens = 0;  // that they hold
     int nsplit = 1;
     int sms = 0;
     int attention = 0;  // of prompt passes: 0 by the rule, 1 the tiled kernel wherever the heads allow it, 2 the split kernel
@@ -644,7 +645,7 @@ struct l2b_session {
     // logits of chosen rows of a many-token pass (l2b_session_extend): row numbers and results, allocated on first use
     int* want_index = nullptr;
     float* want_logits = nullptr;
-    // many-token prompt pass through the tensor-core GEMM (kq_gemm.cuh): buffers for PF_MAX_TOK tokens, allocated on first use
+    // many-token prompt pass through the tensor-core GEMM (kq_gemm.cuh): buffers for up to PF_MAX_TOK tokens, allocated on first use
     bool pf_checked = false, pf_ok = false;
     GemmBufs pf;
     // one persistent kernel per token (token_kernel.cuh): k-quant models on one GPU
@@ -2006,6 +2007,7 @@ static bool alloc_gemm_bufs(const l2b_model* m, GemmBufs& B, size_t T, bool batc
     const int hs = c.dim / c.n_heads;
     DeviceInfo di;
     if (query_device(di) != L2B_OK) return false;
+    B.tokens = (int)T;
     B.sms = di.sms;
     B.attention = (int)env_long("L2B_PROMPT_ATTENTION", 0);
     B.nsplit = c.seq_len >= 2048 ? 4 : 1;
@@ -2035,8 +2037,11 @@ static bool prefill_gemm_eligible(l2b_session* s) {
     if (s->stack) return true;
     if (s->pf_checked) return s->pf_ok;
     s->pf_checked = true;
-    // (a pass that cannot get its buffers leaves prompts to the decode passes)
-    s->pf_ok = env_long("L2B_PREFILL_GEMM", 1) != 0 && gemm_layers_supported(s->model) && alloc_gemm_bufs(s->model, s->pf, std::min(PF_MAX_TOK, std::max(2, s->model->cfg.seq_len)), false);
+    if (env_long("L2B_PREFILL_GEMM", 1) == 0 || !gemm_layers_supported(s->model)) return false;
+    // Buffers for 512 tokens are 211 MB at the 8B shape, 473 MB at the 70B shape (seq_len 4096); where there is no room for them, passes of fewer tokens, down to
+    // 32 (13 and 30 MB), and only then the decode passes.
+    const int most = std::min(PF_MAX_TOK, std::max(2, s->model->cfg.seq_len));
+    for (int T = most; !s->pf_ok && (T == most || T >= 32); T /= 2) s->pf_ok = alloc_gemm_bufs(s->model, s->pf, T, false);
     return s->pf_ok;
 }
 
@@ -2044,7 +2049,7 @@ static bool prefill_gemm_eligible(l2b_session* s) {
 static int min_pass_tokens(const l2b_session* s) { return s->stack ? STACK_MIN_ROWS : PF_MIN_TOK; }
 
 // `forced` of them are followed by a prompt token.
-// Positions pos0 .. pos0 + n - 1 of the prompt already in s->prompt (device), 2 <= n <= PF_MAX_TOK; all enqueued on the session stream.
+// Positions pos0 .. pos0 + n - 1 of the prompt already in s->prompt (device), 2 <= n <= s->pf.tokens; all enqueued on the session stream.
 static int32_t enqueue_prefill_gemm(l2b_session* s, int pos0, int n, int forced) {
     const l2b_model* m = s->model;
     const l2b_config& c = m->cfg;
@@ -2072,7 +2077,7 @@ static int32_t enqueue_forced_positions(l2b_session* s, int from, int to, const 
     int i = from;
     if (to - from >= min_pass_tokens(s) && prefill_gemm_eligible(s)) {
         while (i < to && (s->stack || to - i > 1)) {  // (a llama pass holds two tokens or more; one that is left over takes the graph)
-            const int n = std::min(s->stack ? stack_session_max_rows(s->stack) : PF_MAX_TOK, to - i);
+            const int n = std::min(s->stack ? stack_session_max_rows(s->stack) : s->pf.tokens, to - i);
             L2B_TRY(enqueue_prefill_gemm(s, i, n, n));
             i += n;
         }
@@ -2097,7 +2102,7 @@ static int32_t enqueue_whole_prompt(l2b_session* s, int from, int end, int32_t l
     // Prompts of one pass: there one more reading of the matrices would weigh (1.3 of 8 ms at 128 positions of the 8B shape).  Behind longer ones it
     // is 2 % (1.3 of 61 ms, Phi-3 shape, 2048 positions), and the decode attention's f32 products keep the last row's error against 64 bits
     // where it was: 4.4e-6 with it, 4.6e-6 and 8.3e-6 in the pass, 2.7e-6 to 5.4e-6 before there was one.
-    taken = !s->stack && end - from >= PF_MIN_ALL && end - from <= PF_MAX_TOK && prefill_gemm_eligible(s);
+    taken = !s->stack && end - from >= PF_MIN_ALL && prefill_gemm_eligible(s) && end - from <= s->pf.tokens;
     if (!taken) return L2B_OK;
     const l2b_model* m = s->model;
     const l2b_config& c = m->cfg;

@@ -70,3 +70,27 @@ def test_prompts_around_the_longest_pass(pkg, orc, synth, n):
     got, _ = pkg.generate(model, ids, n + 4)
     assert np.array_equal(got, tokens)
     model.close()
+
+
+def test_prompt_passes_take_the_room_there_is(pkg, synth):
+    """With 100 MB left, a prompt of 400 goes through passes of fewer tokens (512 would take 118 MB), not through 200 decode passes."""
+    import ctypes as C
+    import torch
+    from llama2_jl_b200 import _lib as L
+    cfg = pkg.ModelConfig(2048, 8192, 1, 16, 16, 512, 600, 10000.0, False)
+    w = synth.model_weights(cfg, synth.ALL(12), seed=6)
+    models = [pkg.LanguageModel(cfg, None, w) for _ in range(2)]
+    roomy, tight = (pkg.RunState(m) for m in models)
+    ids = synth.tokens(400, 22, 3, cfg.vocab_size)
+    pkg.prefill(roomy, ids, 0)
+    torch.cuda.synchronize()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (100 << 20), dtype=torch.uint8, device="cuda")
+    pkg.prefill(tight, ids, 0)
+    launches = C.c_int64()
+    L.check(L.lib().l2b_session_last_launches(tight.session, C.byref(launches)))
+    del filler
+    torch.cuda.empty_cache()
+    assert 13 < launches.value < 100
+    assert np.abs(tight.logits - roomy.logits).max() < 2e-5 * float(roomy.logits.max() - roomy.logits.min())
+    for m in models:
+        m.close()
