@@ -1888,6 +1888,8 @@ static int32_t run_one(l2b_session* s, int token, int pos, float temperature, do
 // [tokens][dim] arrays, attention serves every token's query against the cache (causal: token t sees positions <= pos0 + t).
 // Needs q4_K / q5_K layer matrices, three activation planes, one GPU; otherwise the caller uses the decode passes.
 constexpr int PF_MAX_TOK = 512;
+// Shortest run of forced positions (their last one is followed by a prompt token) that takes a pass: where l2b_generate stops inside the prompt, and in
+// front of the last position of a prompt of several passes.  From the integer form of the product; not measured anew.
 constexpr int PF_MIN_TOK = 12;
 // Shortest prompt whose last position goes through the pass too, so that the matrices are read once for all of it.  At the 8B shape a pass of a
 // few tokens takes 6.4 ms and the decode kernels 1.6 ms per position or pair of forced positions: even at about eight.
@@ -1896,13 +1898,15 @@ constexpr int BATCH_MAX_SEQ = 240;
 constexpr int STACK_MIN_ROWS = 2;  // layer-stack models
 
 // Attention of one sequence's tokens at pos0 ..: heads of a multiple of 16 values, at most 128, take the tensor-core kernel.
-// A block of it takes about 10 us and 7.5 us per 64 positions, the split kernel about 5 us and 1 us per 10000 pairs of a query head and a position
-// (measured: 29 queries behind 211 positions, 32 heads: 40 against 25 us; 128 queries: 26 and 25; 512 queries of 2048: 97 against 1280).
+// A block of it takes 12.5 us and per 64 positions 1.1 us and 0.0445 us per dim; the split kernel 11 us and per 10000 pairs of a query head and a
+// position 0.55 us, 0.88 us where no query heads share a key head (fits to 27, 68 us: 128 and 512 queries, 32 heads of 128 on 8; 155: 256 behind 1500,
+// 32 of 96; 35: 300 behind 21, 16 of 64 on 2; 19: 100 behind 77, 8 of 32 on 4; split: 25, 224, 1177, 58, 17; within 15 %).
 static bool prompt_attention_better(int n, int pos0, int n_heads, int gq, int hs, int sms, int asked) {
     if (hs % 16 != 0 || hs > PA_MAX_HS) return false;
     if (asked) return asked == 1;
     const int tq = PA_ROWS / gq, blocks = (n + tq - 1) / tq * (n_heads / gq), waves = (blocks + sms - 1) / sms;
-    const double tiled = 10.0 + 7.5 * waves * ((pos0 + n + PA_KEYS - 1) / PA_KEYS), split = 5.0 + 1e-4 * n_heads * n * (pos0 + 0.5 * n);
+    const double tiled = 12.5 + (1.1 + 0.0445 * hs) * waves * ((pos0 + n + PA_KEYS - 1) / PA_KEYS);
+    const double split = 11.0 + (gq > 1 ? 0.55e-4 : 0.88e-4) * n_heads * n * (pos0 + 0.5 * n);
     return tiled < split;
 }
 static int32_t launch_prompt_attention(const PromptAttnParams& a, int gq, cudaStream_t st) {
@@ -2100,8 +2104,7 @@ static int32_t enqueue_forced_positions(l2b_session* s, int from, int to, const 
 // one-position graph leaves them (and its row in the buffers that l2b_session_read shows).  False: not taken, nothing enqueued.
 static int32_t enqueue_whole_prompt(l2b_session* s, int from, int end, int32_t last_token, bool& taken) {
     // Prompts of one pass: there one more reading of the matrices would weigh (1.3 of 8 ms at 128 positions of the 8B shape).  Behind longer ones it
-    // is 2 % (1.3 of 61 ms, Phi-3 shape, 2048 positions), and the decode attention's f32 products keep the last row's error against 64 bits
-    // where it was: 4.4e-6 with it, 4.6e-6 and 8.3e-6 in the pass, 2.7e-6 to 5.4e-6 before there was one.
+    // is 2 % (1.3 of 61 ms, Phi-3 shape, 2048 positions), and the row takes the decode kernels as in every other model.
     taken = !s->stack && end - from >= PF_MIN_ALL && prefill_gemm_eligible(s) && end - from <= s->pf.tokens;
     if (!taken) return L2B_OK;
     const l2b_model* m = s->model;
@@ -2227,7 +2230,8 @@ extern "C" int32_t l2b_decode_next(l2b_session* s, int32_t token, int32_t pos, f
 }
 
 // Feed n prompt tokens at positions pos0 .. pos0+n-1 (teacher-forced; two positions per pass where both are followed by a
-// prompt token).  The last position goes through the one-position graph, so its logits are in the session afterwards and
+// prompt token).  The last position goes through the one-position graph, or along in the pass (enqueue_whole_prompt), so its logits are
+// in the session afterwards and
 // *next (if given) is their argmax; the caller continues with l2b_decode_next(session, chosen token, pos0 + n, ...).
 extern "C" int32_t l2b_prefill(l2b_session* s, const int32_t* tokens, int32_t n, int32_t pos0, int32_t* next) {
     if (!s || !tokens) return fail(L2B_ERR_BAD_ARG, "null argument");
