@@ -515,9 +515,10 @@ def run_ours(args):
     launches_per_step = model.last_launches()  # of the l2b_generate call above, counted by the library as it enqueues
     forced = max(min(n_prompt - 1, n_pos), 0)  # prompt positions that are followed by a prompt token (no logits needed)
     gemm_min = model.prefill_gemm_min_tokens()
-    if gemm_min and forced >= gemm_min:
-        prefill_how = ("%d forced positions and the last one through the tensor-core GEMM pass (tcgen05 + TMA, up to 128 tokens per pass over a "
-                       "weight tile, no logits for forced positions)" % forced)
+    whole = bool(gemm_min) and forced < n_pos and 10 <= forced + 1 <= 512  # the last prompt position is in the pass too
+    if whole or (gemm_min and forced >= gemm_min):
+        prefill_how = ("%d forced positions%s through the tensor-core GEMM pass (tcgen05 + TMA, up to 128 tokens per pass over a "
+                       "weight tile, no logits for forced positions)%s" % (forced, " and the last one" if whole else "", "" if whole else ", the last one through the decode kernels"))
     elif pairs:
         prefill_how = "two positions per pass of the decode kernels where both are followed by a prompt token (no logits for forced positions)"
     else:

@@ -206,7 +206,8 @@ int32_t l2b_session_last_device_ms(l2b_session* session, float* ms);
  * (src/inference.jl:354-356): positions 0 .. n_prompt-1 (fed prompt tokens) and positions n_prompt .. (fed generated tokens). */
 int32_t l2b_session_last_phase_ms(l2b_session* session, float* prompt_ms, float* decode_ms);
 /* The prompt phase of `sample` (src/inference.jl:349-356, where the reference runs transformer! once per prompt token) as one
- * call: feeds tokens[0..n-1] at positions pos0 .. pos0+n-1, two positions per pass where both are followed by a prompt token.
+ * call: feeds tokens[0..n-1] at positions pos0 .. pos0+n-1, many positions per pass over the weights (l2b_session_prefill_gemm) or two
+ * where both are followed by a prompt token (l2b_session_prefill_pairs).
  * Afterwards the session holds the logits of the last prompt position (l2b_session_logits); *next (may be NULL) is their argmax.
  * Continue with l2b_decode_next(session, chosen_token, pos0 + n, ...). */
 int32_t l2b_prefill(l2b_session* session, const int32_t* tokens, int32_t n, int32_t pos0, int32_t* next);
@@ -217,7 +218,8 @@ int32_t l2b_session_extend(l2b_session* session, const int32_t* tokens, int32_t 
                            float* host_logits);
 /* *min_tokens > 0: runs of at least that many prompt positions that are all followed by a prompt token go through the
  * many-token pass (products on the tensor cores, tcgen05 + TMA, up to 128 tokens per pass over a weight tile; up to 512 tokens
- * per pass over the layers).  0: not available for this model (needs q4_K / q5_K layer matrices, three
+ * per pass over the layers, fewer where device memory has no room for their buffers); prompts of 10 positions up to one pass go through
+ * it whole, the last position, whose logits are wanted, included.  0: not available for this model (needs q4_K / q5_K layer matrices, three
  * activation planes, one GPU; L2B_PREFILL_GEMM=0 switches it off; L2B_PROMPT_ATTENTION, read by a session's first prompt, asks
  * for its tiled (1) or its split (2) attention kernel instead of the quicker one) -- prompts then go through the decode kernels.  The reference
  * feeds prompts token by token (src/inference.jl:349-356). */
@@ -234,7 +236,7 @@ int32_t l2b_session_kernels_per_token(l2b_session* session, int32_t* n);
 
 /* ---- batched decode (no counterpart in the reference, whose `sample` serves one prompt) ----------------------
  * n_seq independent sequences (2 .. 240), each with its own zeroed KV cache of seq_len positions, advanced one position per
- * call: every matrix is streamed once per 20 sequences by the tensor-core GEMM instead of once per sequence.  Needs q4_K /
+ * call: every matrix is streamed once per 128 sequences by the tensor-core GEMM instead of once per sequence.  Needs q4_K /
  * q5_K layer matrices (the classifier may be q6_K), three activation planes, one GPU, or a layer-stack model; otherwise
  * L2B_ERR_UNSUPPORTED_TYPE.
  * l2b_batch_decode_next: tokens[i] is fed at position positions[i] of sequence i (transformer!, src/inference.jl:222-315, for
@@ -295,8 +297,9 @@ int32_t l2b_matrix_destroy(l2b_matrix* m);
 /* y = A' x on device pointers (x: [in] f32, y: [out] f32), copy index `copy`, on `stream` (cudaStream_t; NULL = default). */
 int32_t l2b_matrix_matvec_device(l2b_matrix* m, int32_t copy, const float* dev_x, float* dev_y, int32_t act_planes, void* stream);
 /* ncols columns at once on device pointers (x: [ncols][in], y: [ncols][out]) through the tensor-core GEMM (q4_K / q5_K): the
- * weights are streamed once per 20 columns.  The first call (and any call with more columns than before) allocates the buffer
- * of quantised columns. */
+ * weights are streamed once per 128 columns.  The first call (and any call with more columns than before, up to 1024) allocates the
+ * workspace: the columns as operand terms and the partial results.  It belongs to the matrix, all copies and streams alike: the caller
+ * orders calls on one matrix.  dev_x lies on a 16-byte boundary. */
 int32_t l2b_matrix_matmul_device(l2b_matrix* m, int32_t copy, const float* dev_x, int32_t ncols, float* dev_y, void* stream);
 /* The same through host buffers (x: [ncols][in], y: [ncols][out]); 4 or more columns of a q4_K / q5_K matrix take the GEMM. */
 int32_t l2b_matrix_matvec(l2b_matrix* m, const float* host_x, int32_t ncols, float* host_y, int32_t act_planes);
