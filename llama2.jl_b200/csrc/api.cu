@@ -427,7 +427,8 @@ static GemmInput gemm_input(uint8_t* buf, int64_t n_in, int n_tok) {
 // Tokens per tile and super-blocks per chunk.  The super-blocks of `tiles` row tiles are dealt out evenly, but never so thinly that a tile falls
 // into more than eight parts or a block's start-up outweighs its work; `whole`: every row tile in one chunk (no partial results).
 // Where the token tiles are not dealt out along with them (`by_tokens`), the cuts hang on the matrices alone, and the
-// workspace grows with the tokens and nothing else.  Where they are, there are as few parts as the SMs allow (Phi-3 shape, prompt of 2048: 62.8 against 71.3 ms).
+// workspace grows with the tokens and nothing else.  Where they are, there are as few parts as the SMs allow (Phi-3 shape, prompt of 2048: 64.0 against
+// 71.3 ms).
 static GemmSplit gemm_split(int row_tiles, int nb, int n_tok, int sms, bool whole, bool by_tokens) {
     GemmSplit s;
     const int t16 = (n_tok + 15) / 16 * 16;
@@ -2231,8 +2232,7 @@ extern "C" int32_t l2b_decode_next(l2b_session* s, int32_t token, int32_t pos, f
 
 // Feed n prompt tokens at positions pos0 .. pos0+n-1 (teacher-forced; two positions per pass where both are followed by a
 // prompt token).  The last position goes through the one-position graph, or along in the pass (enqueue_whole_prompt), so its logits are
-// in the session afterwards and
-// *next (if given) is their argmax; the caller continues with l2b_decode_next(session, chosen token, pos0 + n, ...).
+// in the session afterwards and *next (if given) is their argmax; the caller continues with l2b_decode_next(session, chosen token, pos0 + n, ...).
 extern "C" int32_t l2b_prefill(l2b_session* s, const int32_t* tokens, int32_t n, int32_t pos0, int32_t* next) {
     if (!s || !tokens) return fail(L2B_ERR_BAD_ARG, "null argument");
     const l2b_config& c = s->model->cfg;
