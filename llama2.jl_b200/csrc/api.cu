@@ -446,9 +446,9 @@ static int gemm_max_parts(const GemmSplit& s) { return s.U % s.nb == 0 ? 1 : s.n
 static int gemm_row_tiles(const DevMatrix& w) { return (int)((w.out + GM_ROWS - 1) / GM_ROWS); }
 
 template <int MODE>
-static int32_t launch_split_rows(const SplitRowsParams& q, cudaStream_t st) {
-    split_rows_kernel<MODE><<<q.n_tok, 512, 0, st>>>(q);
-    CU(cudaGetLastError());
+static int32_t launch_split_rows(const SplitRowsParams& q, cudaStream_t st, bool pdl = true) {
+    const SplitRowsShape sh = split_rows_shape(q.n, q.n_tok);
+    CU(launch_kernel(split_rows_kernel<MODE>, dim3(sh.cluster, q.n_tok), dim3(sh.warps * 32), (size_t)(q.n / QK_K) * 4, st, pdl, q, sh.cluster));
     return L2B_OK;
 }
 static SplitRowsParams split_rows_params(float* x, const float* gain, int n, int n_tok, const GemmInput& in) {
@@ -485,12 +485,11 @@ static int32_t launch_kq_gemm(const DevMatrix* const* ws, int nw, const GemmInpu
     auto go = [&](auto kernel, auto layout, int threads) {
         g.np = GM_MAX_PACKED;
         while (layout(max_bb, g.np, shared).total + 1024 > GM_SMEM) --g.np;  // + room to align the base to 1024 bytes
-        kernel<<<grid, threads, layout(max_bb, g.np, shared).total + 1024, st>>>(g, maps);
+        return launch_kernel_args(kernel, dim3(grid), dim3(threads), layout(max_bb, g.np, shared).total + 1024, st, true, 1, g, maps);
     };
-    if (sp.tok <= 32) go(kq_gemm_kernel<32>, gm_smem_layout<32>, GmCfg<32>::THREADS);
-    else if (sp.tok <= 64) go(kq_gemm_kernel<64>, gm_smem_layout<64>, GmCfg<64>::THREADS);
-    else go(kq_gemm_kernel<128>, gm_smem_layout<128>, GmCfg<128>::THREADS);
-    CU(cudaGetLastError());
+    if (sp.tok <= 32) CU(go(kq_gemm_kernel<32>, gm_smem_layout<32>, GmCfg<32>::THREADS));
+    else if (sp.tok <= 64) CU(go(kq_gemm_kernel<64>, gm_smem_layout<64>, GmCfg<64>::THREADS));
+    else CU(go(kq_gemm_kernel<128>, gm_smem_layout<128>, GmCfg<128>::THREADS));
     return L2B_OK;
 }
 
@@ -511,8 +510,8 @@ static int32_t launch_product(const DevMatrix& w, const GemmInput& in, int n_tok
     if (gemm_max_parts(sp) == 1) return launch_kq_gemm(ws, 1, in, n_tok, sp, y, 0, (int)w.out, sms, status, st);
     const size_t stride = (size_t)n_tok * w.out;
     L2B_TRY(launch_kq_gemm(ws, 1, in, n_tok, sp, parts, stride, (int)w.out, sms, status, st));
-    sum_parts_kernel<<<dim3((unsigned)std::min<int64_t>(16, (w.out + 255) / 256), n_tok), 256, 0, st>>>(parts, stride, sp, (int)w.out, (int)w.out, y);
-    CU(cudaGetLastError());
+    CU(launch_kernel_args(sum_parts_kernel, dim3((unsigned)std::min<int64_t>(16, (w.out + 255) / 256), n_tok), dim3(256), 0, st, true, 1, (const float*)parts, stride, sp,
+                          (int)w.out, (int)w.out, y));
     return L2B_OK;
 }
 
@@ -528,7 +527,7 @@ static int32_t launch_columns(const DevMatrix& w, const float* x, int ncols, flo
     for (int c = 0; c < ncols; c += PRODUCT_SLAB) {
         const int n = std::min(ncols - c, PRODUCT_SLAB);
         const GemmInput in = gemm_input(workspace, w.in, n);
-        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(const_cast<float*>(x) + (size_t)c * w.in, nullptr, (int)w.in, n, in), st));
+        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(const_cast<float*>(x) + (size_t)c * w.in, nullptr, (int)w.in, n, in), st, false));
         L2B_TRY(launch_product(w, in, n, y + (size_t)c * w.out, (float*)(workspace + product_operand_bytes(w, n)), sms, status, st));
     }
     return L2B_OK;
@@ -1915,12 +1914,11 @@ static int32_t launch_prompt_attention(const PromptAttnParams& a, int gq, cudaSt
     const int tq = PA_ROWS / gq;
     const dim3 grid((a.n + tq - 1) / tq, a.n_heads / gq);
     switch (gq) {
-        case 8: prompt_attention_kernel<8><<<grid, PA_THREADS, smem, st>>>(a); break;
-        case 4: prompt_attention_kernel<4><<<grid, PA_THREADS, smem, st>>>(a); break;
-        case 2: prompt_attention_kernel<2><<<grid, PA_THREADS, smem, st>>>(a); break;
-        default: prompt_attention_kernel<1><<<grid, PA_THREADS, smem, st>>>(a); break;
+        case 8: CU(launch_kernel(prompt_attention_kernel<8>, grid, dim3(PA_THREADS), smem, st, true, a)); break;
+        case 4: CU(launch_kernel(prompt_attention_kernel<4>, grid, dim3(PA_THREADS), smem, st, true, a)); break;
+        case 2: CU(launch_kernel(prompt_attention_kernel<2>, grid, dim3(PA_THREADS), smem, st, true, a)); break;
+        default: CU(launch_kernel(prompt_attention_kernel<1>, grid, dim3(PA_THREADS), smem, st, true, a)); break;
     }
-    CU(cudaGetLastError());
     return L2B_OK;
 }
 
@@ -1952,7 +1950,7 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
     GemmSplit sp;
     size_t stride = 0;
     int ldy = 0;
-    L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.x, m->layers[0].rms_att, c.dim, n, in_dim), st));
+    L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.x, m->layers[0].rms_att, c.dim, n, in_dim), st, false));
     for (int l = 0; l < c.n_layers; ++l) {
         const LayerW& w = m->layers[l];
         float* kcl = kc + (size_t)l * layer_stride;
@@ -1965,8 +1963,7 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
         r.q = B.q; r.kc = kcl; r.vc = vcl; r.rope_cs = rope_cs;
         r.n_tok = n; r.q_dim = c.dim; r.kv_dim = kv_dim; r.hs = hs; r.seq_len = c.seq_len; r.pos0 = pos0; r.neox = c.rope_is_neox;
         r.pos_list = pos_list; r.cache_stride = seq_stride;
-        rope_kv_kernel<<<dim3(8, n), 256, 0, st>>>(r);
-        CU(cudaGetLastError());
+        CU(launch_kernel(rope_kv_kernel, dim3(std::max(1, std::min((c.dim / 2 + kv_dim / 2 + kv_dim + 255) / 256, 8 * B.sms / n)), n), dim3(256), 0, st, true, r));
         if (!pos_list && prompt_attention_better(n, pos0, c.n_heads, gq, hs, B.sms, B.attention)) {
             PromptAttnParams a;
             a.q = B.q; a.kc = kcl; a.vc = vcl; a.out = B.att; a.n = n; a.pos0 = pos0; a.q_stride = c.dim;
@@ -1983,7 +1980,7 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
             a.q_stride = c.dim;
             a.min_chunk = 256;  // many queries already fill the GPU: split a query's positions only when there are many
             if (n < 2) return fail(L2B_ERR_BAD_ARG, "a many-token pass needs at least two tokens");
-            CU(launch_attention(a, gq, st, false));
+            CU(launch_attention(a, gq, st, true));
         }
         L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.att, nullptr, c.dim, n, in_dim), st));
         L2B_TRY(product({&w.wo}, in_dim, sp, stride, ldy));

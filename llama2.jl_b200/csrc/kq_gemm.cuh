@@ -129,13 +129,14 @@ __host__ __device__ inline GmSmem gm_smem_layout(int max_block_bytes, int np, bo
 }
 
 // ---- activations: f32 rows -> two fp16 terms in operand layout --------------------------------------------
-// One block per token.  Where the values come from:
+// A token is one cluster of blocks (split_rows_shape), a warp one super-block.  Where the values come from:
 //   SR_PLAIN    x[t][i]
 //   SR_RESIDUAL x[t][i] + the product's partial results, stored back to x: the residual update of src/inference.jl:285, :305
-//   SR_SWIGLU   silu(gate) * up of the product's partial results (src/inference.jl:295-299), stored to x
+//   SR_SWIGLU   silu(gate) * up of the product's partial results (src/inference.jl:295-299), the last token's stored to x as well
 // then, where `gain` is given, rmsnorm (src/inference.jl:102-110): terms of gain .* x, 1/rms in the token's factor.
 // Value k of a super-block: chunk k / 64, MMA step 2 * (k / 16 % 2) + (k / 32 % 2), half k / 8 % 2, and inside four values the order 0 2 1 3:
-// the order in which the unpack warps meet the nibbles.  Bound by latency (n_tok blocks, two passes over a row held in L2).
+// the order in which the unpack warps meet the nibbles.  Bound by latency: a read from L2, the row's maximum and sum across the cluster, a write.
+// SwiGLU rows of 14336 values: 24 tokens 15.3 -> 7.5 us, 128 tokens 15.9 -> 14.3 us against one block of 16 warps per token and two passes over the row.
 enum : int { SR_PLAIN = 0, SR_RESIDUAL = 1, SR_SWIGLU = 2 };
 struct SplitRowsParams {
     float* x;            // [n_tok][n]
@@ -145,80 +146,126 @@ struct SplitRowsParams {
     int ldy, up_row;     // SR_SWIGLU: rows of the up projection begin here
     GemmSplit sp;
     int n, n_tok, groups;
-    uint8_t *act, *xs;   // null: only the values are wanted (x)
+    uint8_t *act, *xs;   // null: only the values are wanted (x; not with SR_SWIGLU)
     float* scale;
 };
+constexpr int SR_MAX_CLUSTER = 8, SR_MAX_WARPS = 16, SR_KEEP = 2, SR_MAX_BLOCKS = 2 * 148;  // SR_KEEP: super-blocks that a warp keeps in registers
+// Blocks per token (a cluster) and warps per block.  The sum of squares is added up super-block by super-block, whatever the shape is.  As many
+// blocks as give every SM two: beyond that clusters cost more than they bring (512 tokens of 8192 values, SwiGLU: 45 us with eight blocks each, 21 with one).
+struct SplitRowsShape {
+    int cluster, warps;
+};
+inline SplitRowsShape split_rows_shape(int n, int n_tok) {
+    const int nb = n / QK_K;
+    int cl = SR_MAX_CLUSTER;
+    while (cl > 1 && (cl * n_tok > SR_MAX_BLOCKS || nb < 2 * cl)) cl /= 2;
+    const int per = (nb + cl - 1) / cl;
+    return {cl, per < SR_MAX_WARPS ? per : SR_MAX_WARPS};
+}
 
 __device__ __forceinline__ void gm_sum_parts8(const float* y, size_t part_stride, const GemmSplit& sp, int tok, int ldy, int row, float (&v)[8]) {
     const int parts = gm_parts(sp, row);
     const float* src = y + (size_t)tok * ldy + row;
     float4 a = __ldcg(reinterpret_cast<const float4*>(src)), b = __ldcg(reinterpret_cast<const float4*>(src) + 1);
-    for (int p = 1; p < parts; ++p) {
+    for (int p = 1; p < parts; p += 2) {  // two parts' reads in flight together
+        const bool two = p + 1 < parts;
         const float4* s = reinterpret_cast<const float4*>(src + p * part_stride);
-        const float4 c = __ldcg(s), d = __ldcg(s + 1);
+        const float4* s2 = reinterpret_cast<const float4*>(src + (two ? p + 1 : p) * part_stride);
+        const float4 c = __ldcg(s), d = __ldcg(s + 1), e = __ldcg(s2), f = __ldcg(s2 + 1);
         a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
         b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
+        if (two) {
+            a.x += e.x; a.y += e.y; a.z += e.z; a.w += e.w;
+            b.x += f.x; b.y += f.y; b.z += f.z; b.w += f.w;
+        }
     }
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(512) split_rows_kernel(const __grid_constant__ SplitRowsParams p) {
-    __shared__ float s_sum[16], s_max[16];
-    const int tok = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(SR_MAX_WARPS * 32) split_rows_kernel(const __grid_constant__ SplitRowsParams p) {
+    extern __shared__ float s_sum[];  // [nb] sums of squares of the token's super-blocks
+    __shared__ float s_max[SR_MAX_WARPS], s_all[SR_MAX_CLUSTER];  // largest magnitudes of this block's warps, of the cluster's blocks
+    const int tok = blockIdx.y, rank = blockIdx.x, cl = gridDim.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
+    const int nb = p.n / QK_K, per = (nb + cl - 1) / cl, b0 = rank * per, b1 = min(nb, b0 + per);
+    const bool operands = p.act != nullptr, kept = per <= SR_KEEP * W;
     float* x = p.x + (size_t)tok * p.n;
-    float ss = 0.f, mx = 0.f;
-    auto load = [&](int i, float (&v)[8]) {
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldcg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
-        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    pdl_launch_dependents();
+    cluster_arrive();  // (the cluster's blocks have to have started before one writes to another)
+    float mx = 0.f, v[SR_KEEP][8];
+    auto load8 = [](const float* src, float (&d)[8]) {
+        const float4* s = reinterpret_cast<const float4*>(src);
+        const float4 a = __ldcg(s), b = __ldcg(s + 1);
+        d[0] = a.x; d[1] = a.y; d[2] = a.z; d[3] = a.w; d[4] = b.x; d[5] = b.y; d[6] = b.z; d[7] = b.w;
     };
-    for (int i = threadIdx.x; i < p.n / 8; i += blockDim.x) {
-        float v[8];
-        if (MODE == SR_SWIGLU) {
-            float u[8];
-            gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, 8 * i, v);
-            gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, p.up_row + 8 * i, u);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = (v[k] * (1.0f / (1.0f + expf(-v[k])))) * u[k];
-        } else {
-            load(i, v);
-            if (MODE == SR_RESIDUAL) {
-                float u[8];
-                gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, 8 * i, u);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] += u[k];
-            }
-        }
-        if (MODE != SR_PLAIN) {
-            __stcg(reinterpret_cast<float4*>(x) + 2 * i, make_float4(v[0], v[1], v[2], v[3]));
-            __stcg(reinterpret_cast<float4*>(x) + 2 * i + 1, make_float4(v[4], v[5], v[6], v[7]));
-        }
+    auto times_gain = [&](int e, const float (&a)[8], float (&d)[8]) {
         if (p.gain) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i + 1);
-            const float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            const float4* s = reinterpret_cast<const float4*>(p.gain + e);
+            const float4 g = __ldg(s), h = __ldg(s + 1);
+            d[0] = a[0] * g.x; d[1] = a[1] * g.y; d[2] = a[2] * g.z; d[3] = a[3] * g.w;
+            d[4] = a[4] * h.x; d[5] = a[5] * h.y; d[6] = a[6] * h.z; d[7] = a[7] * h.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) d[k] = a[k];
+        }
+    };
+    cluster_wait();
+    pdl_wait();
+    // (the loop over the kept ones is unrolled, so that they are registers; what is not kept is stored and read again)
+    for (int c0 = b0 + warp; c0 < b1; c0 += SR_KEEP * W) {
+#pragma unroll
+        for (int c = 0; c < SR_KEEP; ++c) {
+            const int b = c0 + c * W, e = 256 * b + 8 * lane;
+            if (b >= b1) break;
+            if (MODE == SR_SWIGLU) {
+                float u[8];
+                gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, e, v[c]);
+                gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, p.up_row + e, u);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[c][k] = (v[c][k] * (1.0f / (1.0f + expf(-v[c][k])))) * u[k];
+            } else {
+                load8(x + e, v[c]);
+                if (MODE == SR_RESIDUAL) {
+                    float u[8];
+                    gm_sum_parts8(p.y, p.part_stride, p.sp, tok, p.ldy, e, u);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[c][k] += u[k];
+                }
+            }
+            if (MODE == SR_RESIDUAL || (MODE == SR_SWIGLU && (!kept || tok == p.n_tok - 1))) {
+                __stcg(reinterpret_cast<float4*>(x + e), make_float4(v[c][0], v[c][1], v[c][2], v[c][3]));
+                __stcg(reinterpret_cast<float4*>(x + e) + 1, make_float4(v[c][4], v[c][5], v[c][6], v[c][7]));
+            }
+            if (!operands) continue;
+            float ss = 0.f, d[8];
+            times_gain(e, v[c], d);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                ss = fmaf(v[k], v[k], ss);
-                mx = fmaxf(mx, fabsf(v[k] * g[k]));
+                ss = fmaf(v[c][k], v[c][k], ss);
+                mx = fmaxf(mx, fabsf(d[k]));
             }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) mx = fmaxf(mx, fabsf(v[k]));
+            if (p.gain) {
+                ss = warp_sum(ss);
+                if (lane < cl) st_cluster_f32(cluster_map(s_sum + b, lane), ss);
+            }
         }
     }
-    if (!p.act) return;
-    ss = warp_sum(ss);
+    if (!operands) return;
     mx = warp_max(mx);
-    if (lane == 0) {
-        s_sum[warp] = ss;
-        s_max[warp] = mx;
-    }
+    if (lane == 0) s_max[warp] = mx;
     __syncthreads();
-    ss = 0.f;
+    if (threadIdx.x < cl) {  // this block's maximum to every block of the cluster
+        mx = 0.f;
+        for (int i = 0; i < W; ++i) mx = fmaxf(mx, s_max[i]);
+        st_cluster_f32(cluster_map(s_all + rank, threadIdx.x), mx);
+    }
+    cluster_sync_all();
+    float ss = 0.f;
     mx = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
-        ss += s_sum[i];
-        mx = fmaxf(mx, s_max[i]);
+    for (int i = 0; i < cl; ++i) mx = fmaxf(mx, s_all[i]);
+    if (p.gain) {
+#pragma unroll 4
+        for (int b = 0; b < nb; ++b) ss += s_sum[b];
     }
     // power of two that brings the largest value into [2^13, 2^14): a value 2^-16 of the largest still has 24 significant bits in its
     // two terms, and sums of 32 values, over 32, stay below 2^14 too
@@ -226,40 +273,39 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const __grid_constant__
     const int up = ex == 0 || ex == 255 ? 127 : min(267 - ex, 252);  // 127 + 13 - (ex - 127)
     const float s = __uint_as_float((uint32_t)up << 23), inv = __uint_as_float((uint32_t)(254 - up) << 23);
     const float rms = p.gain ? 1.0f / sqrtf(ss / (float)p.n + 1e-5f) : 1.f;
-    if (threadIdx.x == 0) p.scale[tok] = inv * rms;
+    if (rank == 0 && threadIdx.x == 0) p.scale[tok] = inv * rms;
     const int group = tok >> 3, row = tok & 7;
-    for (int i = threadIdx.x; i < p.n / 8; i += blockDim.x) {  // p.n / 8 is a multiple of 32: whole warps stay together
-        float v[8];
-        load(i, v);
-        if (p.gain) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(p.gain) + 2 * i + 1);
-            const float g[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    for (int c0 = b0 + warp; c0 < b1; c0 += SR_KEEP * W) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] *= g[k];
-        }
-        float sum = 0.f;
-        __half h[8], l[8];
+        for (int cc = 0; cc < SR_KEEP; ++cc) {
+            const int b = c0 + cc * W;
+            if (b >= b1) break;
+            if (!kept) load8(x + 256 * b + 8 * lane, v[cc]);
+            float sum = 0.f, d[8];
+            times_gain(256 * b + 8 * lane, v[cc], d);
+            __half h[8], l[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            v[k] *= s;
-            h[k] = __float2half_rn(v[k]);
-            l[k] = __float2half_rn(v[k] - __half2float(h[k]));
-            sum += v[k];
-        }
-        auto pack = [](__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); };
-        const int b = i >> 5, q = i & 31;  // super-block, which eight values of it
-        const int c = q >> 3, step = 2 * ((q >> 1) & 1) + ((q >> 2) & 1), half = q & 1;
-        uint8_t* dst = p.act + ((size_t)(b * 4 + c) * p.groups + group) * GM_GROUP_BYTES + step * 256 + half * 128 + row * 16;
-        *reinterpret_cast<uint4*>(dst) = make_uint4(pack(h[0], h[2]), pack(h[1], h[3]), pack(h[4], h[6]), pack(h[5], h[7]));
-        *reinterpret_cast<uint4*>(dst + 1024) = make_uint4(pack(l[0], l[2]), pack(l[1], l[3]), pack(l[4], l[6]), pack(l[5], l[7]));
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        if ((q & 3) == 0) {
-            sum *= 0.03125f;
-            const __half sh = __float2half_rn(sum), sl = __float2half_rn(sum - __half2float(sh));
-            uint8_t* xd = p.xs + ((size_t)b * p.groups + group) * GM_XS_BYTES + row * 16 + (q >> 2) * 2;
-            *reinterpret_cast<__half*>(xd) = sh;
-            *reinterpret_cast<__half*>(xd + 128) = sl;
+            for (int k = 0; k < 8; ++k) {
+                d[k] *= s;
+                h[k] = __float2half_rn(d[k]);
+                l[k] = __float2half_rn(d[k] - __half2float(h[k]));
+                sum += d[k];
+            }
+            auto pack = [](__half a, __half b) { return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16); };
+            const int q = lane;  // which eight values of the super-block
+            const int c = q >> 3, step = 2 * ((q >> 1) & 1) + ((q >> 2) & 1), half = q & 1;
+            uint8_t* dst = p.act + ((size_t)(b * 4 + c) * p.groups + group) * GM_GROUP_BYTES + step * 256 + half * 128 + row * 16;
+            *reinterpret_cast<uint4*>(dst) = make_uint4(pack(h[0], h[2]), pack(h[1], h[3]), pack(h[4], h[6]), pack(h[5], h[7]));
+            *reinterpret_cast<uint4*>(dst + 1024) = make_uint4(pack(l[0], l[2]), pack(l[1], l[3]), pack(l[4], l[6]), pack(l[5], l[7]));
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            if ((q & 3) == 0) {
+                sum *= 0.03125f;
+                const __half sh = __float2half_rn(sum), sl = __float2half_rn(sum - __half2float(sh));
+                uint8_t* xd = p.xs + ((size_t)b * p.groups + group) * GM_XS_BYTES + row * 16 + (q >> 2) * 2;
+                *reinterpret_cast<__half*>(xd) = sh;
+                *reinterpret_cast<__half*>(xd + 128) = sl;
+            }
         }
     }
 }
@@ -267,6 +313,8 @@ __global__ void __launch_bounds__(512) split_rows_kernel(const __grid_constant__
 // A product that is wanted as such: dst[t][i] = the sum of its partial results.  Grid (blocks per row, n_tok): at most 65535 tokens.
 __global__ void sum_parts_kernel(const float* __restrict__ y, size_t part_stride, const __grid_constant__ GemmSplit sp, int ldy, int rows, float* __restrict__ dst) {
     const int tok = blockIdx.y;
+    pdl_launch_dependents();
+    pdl_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
         const int parts = gm_parts(sp, i);
         float v = __ldcg(y + (size_t)tok * ldy + i);
@@ -435,6 +483,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         }
     } else if (warp == 10 || warp == 11) {
         // ================= activation operands: one bulk copy per 64 values =================
+        pdl_wait();  // (weights are constant: the copies and the unpacking of the first ones do not wait)
         if (lane == 0) {
             int s = 0, turn = warp - 10;
             bool first = true;
@@ -687,6 +736,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
     } else {
         // ================= epilogue: thread = weight row; warps e and e + 4 split the tokens =================
+        pdl_wait();
         constexpr int NH = NT / 2;
         const int q = warp & 3, half = warp >> 2;
         const int r = 32 * q + lane;
@@ -785,6 +835,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
     }
     // every path ends here; the tensor memory is freed by the warp that allocated it
+    pdl_launch_dependents();  // (here: blocks of the next kernel that start earlier would all share the few SMs this grid leaves free)
     tc_fence_before();
     __syncthreads();
     if (warp == 9) tmem_dealloc(tmem_base, 512);

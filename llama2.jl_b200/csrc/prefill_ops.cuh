@@ -44,6 +44,8 @@ struct RopeKvParams {
 };
 __global__ void rope_kv_kernel(const __grid_constant__ RopeKvParams p) {
     const int t = blockIdx.y, pos = p.pos_list ? __ldg(p.pos_list + t) : p.pos0 + t;
+    pdl_launch_dependents();
+    pdl_wait();
     float* const kc = p.kc + (p.pos_list ? (size_t)t * p.cache_stride : 0);
     float* const vc = p.vc + (p.pos_list ? (size_t)t * p.cache_stride : 0);
     auto sum = [&](int row) {

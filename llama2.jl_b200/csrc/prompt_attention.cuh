@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
         fence_proxy_async();
     }
     if (warp == 8) tmem_alloc(tmem_slot, 512);
+    pdl_wait();
     float q_inv = 1.f;
     if (warp < 8) {  // two threads per query row: its two terms (all loads in flight at once: one after the other they had taken 10 us)
         const int r = threadIdx.x & 127, half = threadIdx.x >> 7, t = min(tok0 + r % TQ, p.n - 1), h = hg * GQ + r / TQ, oct = hs >> 4;
@@ -481,6 +482,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
         }
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
     }
+    pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
     if (warp == 8) tmem_dealloc(tmem, 512);
