@@ -474,9 +474,7 @@ static int32_t set_stack_kernel_attrs() {
         set((const void*)head_prefill_kernel);
         set((const void*)mlstm_state_kernel);
         set((const void*)mlstm_chunk_kernel);
-        set((const void*)bf16_gemm_kernel<32, 1>); set((const void*)bf16_gemm_kernel<32, 2>);
-        set((const void*)bf16_gemm_kernel<64, 1>); set((const void*)bf16_gemm_kernel<64, 2>);
-        set((const void*)bf16_gemm_kernel<128, 1>); set((const void*)bf16_gemm_kernel<128, 2>);
+        set((const void*)bf16_gemm_kernel<false>); set((const void*)bf16_gemm_kernel<true>);
         set((const void*)cache_scan_kernel<float, 1>); set((const void*)cache_scan_kernel<float, 2>);
         set((const void*)cache_scan_kernel<float, 3>); set((const void*)cache_scan_kernel<float, 4>);
         set((const void*)cache_scan_mma_kernel<1>); set((const void*)cache_scan_mma_kernel<2>); set((const void*)cache_scan_mma_kernel<3>);
@@ -894,6 +892,19 @@ static int32_t bf16_map(CUtensorMap& map, const bf16* base, int64_t inner, int64
     return L2B_OK;
 }
 
+// Tokens per tile.  A round of all pairs takes, per 64 values of K, the larger of 2 N cycles (the products) and 2.67 (128 + N / 2) cycles (the
+// operands' way from L2; fits 256: 376 ns, 224 - 128 within 10 %): what takes least for all rounds.
+static int gemm_tile_tokens(int mtiles, int n, int sms) {
+    int best = 0;
+    double least = 0.0;
+    for (int N = 256; N >= 32; N -= 32) {
+        const int tiles = mtiles * ((n + N - 1) / N), pairs = sms / 2;
+        const double t = (tiles + pairs - 1) / pairs * std::max(2.0 * N, 2.667 * (128 + N / 2));
+        if (!best || t < least * 0.99) least = t, best = N;
+    }
+    return best;
+}
+
 // W x for n rows of x ([n][ldx], bf16 or f32 by the model's compute type), then `epi`.
 static int32_t launch_gemm(const StackSession* s, const StackMatrix& w, const void* x, int ldx, int n, const DenseEpilogue& epi, int* status, cudaStream_t st) {
     const int rows = w.results();
@@ -908,35 +919,23 @@ static int32_t launch_gemm(const StackSession* s, const StackMatrix& w, const vo
         CU(cudaGetLastError());
         return L2B_OK;
     }
-    // Token tile: as wide as the rows there are, narrower while the tiles do not fill the GPU.  Weight tiles per block: what takes fewer
-    // rounds of the GPU, a round of two weight tiles costing about 1.55 rounds of one (2 when short products leave the epilogue exposed).
-    auto up_div = [](long a, long b) { return (a + b - 1) / b; };
-    const long sms = s->di.sms;
-    int bn = n <= 32 ? 32 : n <= 64 ? 64 : 128;
-    while (bn > 32 && up_div(rows, 128) * up_div(n, bn) < sms) bn /= 2;
-    const double one = (double)up_div(up_div(rows, 128) * up_div(n, bn), sms), two = (w.k < 1024 ? 2.0 : 1.55) * (double)up_div(up_div(rows, 256) * up_div(n, bn), sms);
-    const int na = w.pair == 2 || two < one ? 2 : 1;
+    const bool dual = w.pair == 2;
     GemmDenseParams g;
     memset(&g, 0, sizeof(g));
     g.rows = rows; g.n_tok = n; g.k = w.k; g.epi = epi; g.status = status;
-    g.row2 = w.pair == 2 || na == 1 ? 0 : 128;
-    const int stage = bg_stage_bytes(bn, na);
-    g.stages = std::min(BG_MAX_STAGES, (s->di.max_smem_optin - 4096) / stage);
+    g.mtiles = dual ? (rows + 127) / 128 : (rows + 255) / 256;
+    g.N = gemm_tile_tokens(g.mtiles, n, s->di.sms);
+    g.ntiles = (n + g.N - 1) / g.N;
+    const int stage = bg_stage_bytes(g.N), swap = dual ? BG_SWAP_BYTES : 0;
+    g.stages = std::min(BG_MAX_STAGES, (s->di.max_smem_optin - 4096 - swap) / stage);
     CUtensorMap ma, ma2, mb;
-    L2B_TRY(bf16_map(ma, w.w, w.k, rows, (int64_t)w.stride(), 128));
+    L2B_TRY(bf16_map(ma, w.w, w.k, rows, (int64_t)w.stride(), dual ? 64 : 128));
     ma2 = ma;
-    if (w.pair == 2) L2B_TRY(bf16_map(ma2, w.second(), w.k, rows, (int64_t)w.stride(), 128));
-    L2B_TRY(bf16_map(mb, static_cast<const bf16*>(x), w.k, n, ldx, bn));
-    const int per = w.pair == 2 ? 128 : 128 * na;
-    g.mtiles = (rows + per - 1) / per;
-    g.ntiles = (n + bn - 1) / bn;
-    const dim3 grid((unsigned)std::min<long>((long)g.mtiles * g.ntiles, s->di.sms)), block(BG_THREADS);
-    const size_t smem = (size_t)g.stages * stage + 1024;
-    auto go = [&](auto k) { return launch_kernel_args(k, grid, block, smem, st, false, 1, g, ma, ma2, mb); };
-    cudaError_t e;
-    if (na == 1) e = bn == 32 ? go(bf16_gemm_kernel<32, 1>) : bn == 64 ? go(bf16_gemm_kernel<64, 1>) : go(bf16_gemm_kernel<128, 1>);
-    else e = bn == 32 ? go(bf16_gemm_kernel<32, 2>) : bn == 64 ? go(bf16_gemm_kernel<64, 2>) : go(bf16_gemm_kernel<128, 2>);
-    CU(e);
+    if (dual) L2B_TRY(bf16_map(ma2, w.second(), w.k, rows, (int64_t)w.stride(), 64));
+    L2B_TRY(bf16_map(mb, static_cast<const bf16*>(x), w.k, n, ldx, g.N / 2));
+    const dim3 grid(2u * (unsigned)std::min(g.mtiles * g.ntiles, s->di.sms / 2)), block(BG_THREADS);
+    const size_t smem = (size_t)g.stages * stage + swap + 1024;
+    CU(launch_kernel_args(dual ? bf16_gemm_kernel<true> : bf16_gemm_kernel<false>, grid, block, smem, st, false, 2, g, ma, ma2, mb));
     return L2B_OK;
 }
 

@@ -128,6 +128,17 @@ def test_prompt_decode_and_portions(pkg, case, compute):
     model.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("width, ff, n", [(200, 330, 33), (72, 129, 257), (264, 520, 513), (64, 8200, 600)])
+def test_products_at_tile_edges(pkg, width, ff, n):
+    """Rows, tokens and inner lengths around the tiles of the bf16 products (256 or 2 x 64 rows, 32 .. 256 tokens, 128 values), and several tiles per block."""
+    cfg = sc.config([(sc.mixer(heads=2), ff)], width=width, vocab=130, side=40)
+    w, t = sc.weights(cfg, 41), sc.tokens(cfg, n, 42)
+    model = build(pkg, cfg, w, n, "bfloat16")
+    check(feed(pkg, pkg.RunState(model), t, [n]), expected(cfg, w, t), "bfloat16")
+    model.close()
+
+
 def only(cfg, w, keep):
     """Weights whose other mechanisms are silent: residual contributions not named in `keep` are zero."""
     w = {k: v.copy() for k, v in w.items()}
