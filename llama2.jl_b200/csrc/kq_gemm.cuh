@@ -21,7 +21,8 @@
 //   packed-copy warp  one TMA tiled copy (cp.async.bulk.tensor) per super-block: a 128-row box of the stored blocks
 //   2 operand warps   one bulk copy per 64 values: the tokens' two terms, already in operand layout (split_rows_kernel); a thread takes 750
 //                     cycles to see a slot free and issue a copy, so two take turns
-//   unpack warps      groups of four; thread = row: nibbles -> fp16 times scale, into core matrices (8 rows x 16 bytes)
+//   unpack warps      groups of four; thread = row: nibbles -> fp16 times scale, into core matrices (8 rows x 16 bytes) or, for tiles of more
+//                     than 64 tokens, into tensor memory (lane = row)
 //   MMA warp          tcgen05.mma.kind::f16 (M 128, K 16), four or eight per 64 values
 //   8 epilogue warps  thread = weight row, half of the tokens: tensor memory -> times d -> f32 accumulators, and those of four
 //                     super-blocks -> f32 sums in tensor memory (one chain over 14336 values would be 280 roundings long)
@@ -93,16 +94,24 @@ struct GemmMaps {
 // last use by parity, so it must have seen the use before that: its own last step lies at most NS steps back, UG / GS <= NS.  (More groups
 // are no help: all read the scales of every super-block they take part in, 200 instructions a row, which with four groups on the steps
 // of one super-block made the kernel issue-bound.)
+// AT: with 128 tokens the products read 64 KB of shared memory per 64 values when the weights come from there too (each of the two terms
+// reads them again), as much as an SM delivers while they run, and copies and unpacking want another 57 KB.  From tensor memory the weights cost
+// nothing of it, and there is room for four slots of activations: 1240 -> 930 cycles per 64 values (q4_K 28672 x 4096 times 128).  That leaves two
+// sets of accumulators instead of three.  (Blocks in pairs that share the activations, cta_group::2: 1270 - 1350 cycles; 16 epilogue warps: no
+// faster.)  Narrower tiles spend their time on the unpack warps' instructions and keep the deeper accumulators.
 // Whatever the tile holds, a column's sums are the same ones in the same order: low terms, then high terms of 64 values in one accumulator,
 // added to the f32 sum chunk by chunk, the shared part behind them.  So a column's result does not hang on how many columns came with it.
 template <int NT>
 struct GmCfg {
     static constexpr int CH = NT == 128 ? 1 : 2;
-    static constexpr int NS = NT == 64 ? 2 : 3, ND = NS;
+    static constexpr bool AT = NT == 128;  // weights go through tensor memory
+    static constexpr int NS = NT == 64 ? 2 : NT == 32 ? 3 : 4, ND = NT == 32 ? 3 : 2;
     static constexpr int GS = NT == 64 ? 2 : 1, UG = NT == 128 ? 2 : NT == 64 ? 4 : 3;
     static_assert(UG / GS <= NS, "a group would miss a phase");
     static constexpr int DCOLS = CH == 1 ? NT : 3 * NT;  // accumulator columns per slot: 128, 192, 96
-    static_assert(ND * DCOLS + NT <= 512, "the sums stand behind the accumulators");
+    static constexpr int SUMS = ND * DCOLS, A_COLS = SUMS + NT;  // columns where the sums and the weights stand
+    static_assert(ND <= NS, "a step's accumulators are waited for at its own slot");
+    static_assert(A_COLS + (AT ? 32 * NS : 0) <= 512, "accumulators, sums, weights");
     static constexpr int THREADS = (GM_EPI_WARPS + 4 + 4 * UG) * 32;  // warps 0-7 epilogue, 8 packed copies, 9 MMA, 10 and 11 operand copies, 12 .. unpack
 };
 constexpr int GM_MAX_PACKED = 5;
@@ -115,11 +124,11 @@ template <int NT>
 __host__ __device__ inline GmSmem gm_smem_layout(int max_block_bytes, int np, bool shared) {
     constexpr int CH = GmCfg<NT>::CH;
     GmSmem s;
-    s.off_bar = 0;  // done[3] ready[3] p_full[5] p_free[5]
-    s.off_tmem = 16 * 8;
+    s.off_bar = 0;  // done[4] ready[4] p_full[5] p_free[5]
+    s.off_tmem = 18 * 8;
     s.off_hdr = 256;  // [GM_HDRS][128] {d, factor of the shared part}
     s.off_a = (s.off_hdr + GM_HDRS * GM_ROWS * 8 + 1023) & ~1023;
-    s.slot_a = CH * GM_A_BYTES + (CH == 2 && shared ? GM_A_BYTES / 2 : 0);
+    s.slot_a = GmCfg<NT>::AT ? 0 : CH * GM_A_BYTES + (CH == 2 && shared ? GM_A_BYTES / 2 : 0);
     s.slot_b = CH * NT * 256 + (CH == 2 && shared ? NT * 32 : 0);
     s.off_b = s.off_a + GmCfg<NT>::NS * s.slot_a;
     s.off_packed = s.off_b + GmCfg<NT>::NS * s.slot_b;
@@ -355,10 +364,9 @@ __device__ __forceinline__ GmScale gm_scale(__half2 S, float centre) {
 // 16 values of one MMA step from the nibbles of q (HIGH: the upper ones); f: words whose bits `top_mask` of every byte stand above the
 // nibble, with the factor `top`.  Pairs are bytes (0, 2) and (1, 3) of a word.
 template <bool HIGH, bool TOP>
-__device__ __forceinline__ void gm_store16(uint8_t* dst, const uint4& q, const uint4& f, uint32_t top_mask, __half2 top, const GmScale& g) {
+__device__ __forceinline__ void gm_values16(const uint4& q, const uint4& f, uint32_t top_mask, __half2 top, const GmScale& g, uint32_t (&o)[8]) {
     const uint32_t qw[4] = {q.x, q.y, q.z, q.w}, fw[4] = {f.x, f.y, f.z, f.w};
     const uint32_t m = HIGH ? 0x00F000F0u : 0x000F000Fu;
-    uint32_t o[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
@@ -369,9 +377,21 @@ __device__ __forceinline__ void gm_store16(uint8_t* dst, const uint4& q, const u
             o[2 * i + e] = h2_raw(v);
         }
     }
-    *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
-    *reinterpret_cast<uint4*>(dst + 2048) = make_uint4(o[4], o[5], o[6], o[7]);
 }
+// Where a row's operand values go: the 16 of MMA step kk of a slot, into core matrices in shared memory or eight columns of tensor memory.
+template <bool AT>
+struct GmDest {
+    uint8_t* smem;
+    uint32_t tmem;
+    __device__ __forceinline__ void put(int kk, const uint32_t (&o)[8]) const {
+        if (AT) {
+            tmem_st8(tmem + (uint32_t)(8 * kk), o);
+        } else {
+            *reinterpret_cast<uint4*>(smem + kk * 4096) = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4*>(smem + kk * 4096 + 2048) = make_uint4(o[4], o[5], o[6], o[7]);
+        }
+    }
+};
 
 // ---- the GEMM ----------------------------------------------------------------------------------------
 // Steps per super-block: q6_K has eight chunks (its two passes) and no shared part.
@@ -380,6 +400,7 @@ __device__ __forceinline__ int gm_steps(int type) { return CH == 2 ? (type == T_
 
 template <int NT>
 __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ GemmMaps maps) {
+    constexpr bool AT = GmCfg<NT>::AT;
     constexpr int NS = GmCfg<NT>::NS, ND = GmCfg<NT>::ND, UG = GmCfg<NT>::UG, GS = GmCfg<NT>::GS, DCOLS = GmCfg<NT>::DCOLS, CH = GmCfg<NT>::CH;
     const int NP = p.np;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -395,7 +416,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
     uint64_t* done = reinterpret_cast<uint64_t*>(smem + L.off_bar);
     // ready: weights unpacked, activations landed and the accumulators of the slot's last use read.  One barrier for all three, because the
     // MMA thread's own instructions bound this kernel: with a barrier each it took 1450 cycles per step of 64 values, whatever the tile.
-    uint64_t *ready = done + 3, *p_full = done + 6, *p_free = done + 11;
+    uint64_t *ready = done + 4, *p_full = done + 8, *p_free = done + 13;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.off_tmem);
     float2* hdr = reinterpret_cast<float2*>(smem + L.off_hdr);
 
@@ -537,6 +558,11 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         // operand descriptors of slot 0; the others lie a multiple of 16 bytes further
         const uint64_t desc_a = umma_desc(smem + L.off_a, 2048, 128), desc_b = umma_desc(smem + L.off_b, 128, GM_GROUP_BYTES);
         const uint64_t desc_xs = umma_desc(smem + L.off_b, 128, GM_XS_BYTES);
+        // a: slot of the weights; ka, kb: bytes further in it and in the operand of the activations
+        auto mma = [&](uint32_t d, int a, int ka, uint64_t b, uint32_t accumulate) {
+            if (AT) umma_f16_at(d, tmem_base + (uint32_t)(GmCfg<NT>::A_COLS + 32 * a + (ka >> 9)), b, idesc, accumulate);  // (4096 bytes: 8 columns)
+            else umma_f16(d, desc_a + (uint64_t)((a * L.slot_a + ka) >> 4), b, idesc, accumulate);
+        };
         int s = 0, ds = 0;
         uint32_t parity = 0;
         for (int item = blockIdx.x; item < items && ok; item += gridDim.x)
@@ -549,7 +575,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 }
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(ds * DCOLS);
-                const uint64_t da = desc_a + (uint64_t)(s * (L.slot_a >> 4)), db = desc_b + (uint64_t)(s * (L.slot_b >> 4));
+                const uint64_t db = desc_b + (uint64_t)(s * (L.slot_b >> 4));
                 const bool shared_part = k == (CH == 2 ? 1 : 4) && (CH == 2 ? steps == 2 : steps == 5);
                 if (elect_one()) {
                     if (CH == 2 || !shared_part) {
@@ -559,14 +585,15 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                             for (int t = 1; t >= 0; --t)  // low terms of X first
 #pragma unroll
                                 for (int kk = 0; kk < 4; ++kk)
-                                    umma_f16(d + (uint32_t)(c * NT), da + (uint64_t)((c * GM_A_BYTES + kk * 4096) >> 4),
-                                             db + (uint64_t)((c * chunk_b + t * 1024 + kk * 256) >> 4), idesc, t == 1 && kk == 0 ? 0u : 1u);
+                                    mma(d + (uint32_t)(c * NT), s, c * GM_A_BYTES + kk * 4096, db + (uint64_t)((c * chunk_b + t * 1024 + kk * 256) >> 4),
+                                        t == 1 && kk == 0 ? 0u : 1u);
                     }
                     if (shared_part) {  // low terms of C first
-                        const uint64_t ax = da + (uint64_t)(CH == 2 ? (2 * GM_A_BYTES) >> 4 : 0), dx = desc_xs + (uint64_t)((s * L.slot_b + (CH == 2 ? 2 * chunk_b : 0)) >> 4);
+                        constexpr int ax = CH == 2 ? 2 * GM_A_BYTES : 0;
+                        const uint64_t dx = desc_xs + (uint64_t)((s * L.slot_b + (CH == 2 ? 2 * chunk_b : 0)) >> 4);
                         const uint32_t dd = d + (uint32_t)(CH == 2 ? 2 * NT : 0);
-                        umma_f16(dd, ax + (4096 >> 4), dx, idesc, 0u);
-                        umma_f16(dd, ax, dx, idesc, 1u);
+                        mma(dd, s, ax + 4096, dx, 0u);
+                        mma(dd, s, ax, dx, 1u);
                     }
                     umma_commit(done + s);
                 }
@@ -649,14 +676,17 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                     ok = false;
                     break;
                 }
+                if (AT) tc_fence_after();
                 // (the epilogue may still be at the super-block before the last one: four sets of factors are enough)
                 if (k == 0 && sub == 0) hdr[hs * GM_ROWS + r] = make_float2(d * (float)(1 << GM_A_EXP), 32.f * s_dn);
                 uint8_t* const a_slot = smem + L.off_a + slot * L.slot_a + row_off;
+                const uint32_t a_cols = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(GmCfg<NT>::A_COLS + 32 * slot);
                 if (CH == 2 || type == T_Q6_K || k < 4) {
 #pragma unroll 1
                     for (int e = sub; e < CH; e += GS) {
                         const int kc = CH * k + e;
-                        uint8_t* const dst = a_slot + e * GM_A_BYTES;
+                        const GmDest<AT> dst = {a_slot + e * GM_A_BYTES, a_cols};
+                        uint32_t o[8];
                         if (type == T_Q6_K) {
                             const int c = kc & 3, hh = c >> 1, odd = c & 1;
                             const uint32_t scw = c == 0 ? top0.x : c == 1 ? top0.y : c == 2 ? top0.z : top0.w;
@@ -671,8 +701,9 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                                     const uint4 q = *reinterpret_cast<const uint4*>(blk + 64 * hh + 32 * hi + 16 * part);
                                     const int idx = 2 * odd + hi;  // which two bits of the byte: value 16 at bit 2 * idx
                                     const __half2 up = __hmul2(S, h2_bits(((uint32_t)(23 - 2 * idx) << 10) * 0x00010001u));  // 2^(8 - 2 idx)
-                                    if (odd) gm_store16<true, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
-                                    else gm_store16<false, true>(dst + (2 * part + hi) * 4096, q, f, 0x00030003u << (2 * idx), up, g);
+                                    if (odd) gm_values16<true, true>(q, f, 0x00030003u << (2 * idx), up, g, o);
+                                    else gm_values16<false, true>(q, f, 0x00030003u << (2 * idx), up, g, o);
+                                    dst.put(2 * part + hi, o);
                                 }
                             }
                         } else {
@@ -685,23 +716,27 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
 #pragma unroll
                                 for (int part = 0; part < 2; ++part) {
                                     const uint4 q = *reinterpret_cast<const uint4*>(blk + 48 + 32 * kc + 16 * part);
-                                    gm_store16<false, true>(dst + 2 * part * 4096, q, part ? top1 : top0, bit, up0, g0);
-                                    gm_store16<true, true>(dst + (2 * part + 1) * 4096, q, part ? top1 : top0, bit << 1, up1, g1);
+                                    gm_values16<false, true>(q, part ? top1 : top0, bit, up0, g0, o);
+                                    dst.put(2 * part, o);
+                                    gm_values16<true, true>(q, part ? top1 : top0, bit << 1, up1, g1, o);
+                                    dst.put(2 * part + 1, o);
                                 }
                             } else {
 #pragma unroll
                                 for (int part = 0; part < 2; ++part) {
                                     const uint4 q = *reinterpret_cast<const uint4*>(blk + 16 + 32 * kc + 16 * part);
-                                    gm_store16<false, false>(dst + 2 * part * 4096, q, q, 0u, g0.high, g0);
-                                    gm_store16<true, false>(dst + (2 * part + 1) * 4096, q, q, 0u, g1.high, g1);
+                                    gm_values16<false, false>(q, q, 0u, g0.high, g0, o);
+                                    dst.put(2 * part, o);
+                                    gm_values16<true, false>(q, q, 0u, g1.high, g1, o);
+                                    dst.put(2 * part + 1, o);
                                 }
                             }
                         }
                     }
                 }
                 if (type != T_Q6_K && k == (CH == 2 ? 1 : 4) && sub == GS - 1) {
-                    uint8_t* const dst = a_slot + (CH == 2 ? 2 * GM_A_BYTES : 0);
-                    uint32_t o[4], o2[4];
+                    const GmDest<AT> dst = {a_slot + (CH == 2 ? 2 * GM_A_BYTES : 0), a_cols};
+                    uint32_t o[8], o2[8];
 #pragma unroll
                     for (int j2 = 0; j2 < 4; ++j2) {
                         float f2[2];
@@ -713,16 +748,18 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                         }
                         const __half2 hi = __floats2half2_rn(f2[0], f2[1]);
                         const float2 back = __half22float2(hi);
-                        o[j2] = h2_raw(hi);
-                        o2[j2] = h2_raw(__floats2half2_rn(f2[0] - back.x, f2[1] - back.y));
+                        o[j2] = o[j2 + 4] = h2_raw(hi);
+                        o2[j2] = o2[j2 + 4] = h2_raw(__floats2half2_rn(f2[0] - back.x, f2[1] - back.y));
                     }
-                    const uint4 v = make_uint4(o[0], o[1], o[2], o[3]), v2 = make_uint4(o2[0], o2[1], o2[2], o2[3]);
-                    *reinterpret_cast<uint4*>(dst) = v;  // each term times the high and the low terms of the sums
-                    *reinterpret_cast<uint4*>(dst + 2048) = v;
-                    *reinterpret_cast<uint4*>(dst + 4096) = v2;
-                    *reinterpret_cast<uint4*>(dst + 4096 + 2048) = v2;
+                    dst.put(0, o);  // each term times the high and the low terms of the sums
+                    dst.put(1, o2);
                 }
-                fence_proxy_async();  // the tensor core reads shared memory through the asynchronous proxy
+                if (AT) {
+                    tmem_wait_st();
+                    tc_fence_before();
+                } else {
+                    fence_proxy_async();  // the tensor core reads shared memory through the asynchronous proxy
+                }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(ready + slot);
             }
@@ -799,7 +836,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
             hs = (hs + 1) % GM_HDRS;
             const bool last = w.b == nb - 1 || w.u == w.end - 1;  // this chunk's part of the tile is complete
             if (ok && (last || ((w.b + 1) & (w.type == T_Q6_K ? 1 : 3)) == 0)) {  // 20 (q6_K: 16) values have been added up
-                const uint32_t sums = taddr + (uint32_t)(ND * DCOLS + NH * half);
+                const uint32_t sums = taddr + (uint32_t)(GmCfg<NT>::SUMS + NH * half);
 #pragma unroll
                 for (int c0 = 0; c0 < NH; c0 += 16) {
                     if (!held || c0 >= mine) break;
