@@ -194,6 +194,10 @@ struct MvLaunch {
     size_t smem = 0;
 };
 
+// f32 rows that a warp of f32_matvec_kernel keeps in registers.
+constexpr int F32_MAX_NV = 12;
+static int f32_nv(int n_in) { return n_in <= 3 * 128 ? 3 : n_in <= 6 * 128 ? 6 : n_in <= F32_MAX_NV * 128 ? F32_MAX_NV : 0; }  // 0: too long
+
 // Decide grid, consumer warps, ring slots and shared memory for a launch whose segments, n_in, prologue and
 // epilogue fields are already filled in, and precompute the schedule constants the kernel would otherwise
 // derive with serial integer arithmetic.
@@ -226,7 +230,7 @@ static int32_t plan_matvec(MvLaunch& L, const DeviceInfo& di) {
     p.units_rem = units % L.grid;
     if (!L.kq) {
         const int per_block = p.units_lo + (p.units_rem ? 1 : 0);
-        const int W = std::max(4, std::min(MV_MAX_CONSUMERS, per_block));
+        const int nv = f32_nv(p.n_in), W = std::max(nv ? 1 : 4, std::min(nv ? f32_max_warps(nv) : MV_MAX_CONSUMERS, per_block));
         p.consumers = W;
         p.cgroups = 1;
         p.turns = (p.n_in / 8 + 32 * W - 1) / (32 * W);
@@ -342,6 +346,9 @@ static cudaError_t launch_matvec(const MvLaunch& L, cudaStream_t st, bool pdl) {
         if (!L.kq || L.planes != 3 || L.p.tp) return cudaErrorNotSupported;
         return launch_kernel(fused_matvec_kernel<true, 3, false, false, 2>, grid, block, L.smem, st, pdl, L.p);
     }
+    if (!L.kq)
+        if (const int nv = f32_nv(L.p.n_in))
+            return launch_kernel(nv == 3 ? f32_matvec_kernel<3> : nv == 6 ? f32_matvec_kernel<6> : f32_matvec_kernel<F32_MAX_NV>, grid, block, 0, st, pdl, L.p);
     if (!L.kq) return launch_kernel(fused_matvec_kernel<false, 1>, grid, block, L.smem, st, pdl, L.p);
     if (L.p.tp)  // the variants that carry the tensor-parallel exchange
         switch (L.planes) {

@@ -171,6 +171,20 @@ def test_matvec_rejects_bad_arguments(L, pkg):
 
 
 # ---- small operators ------------------------------------------------------------------------------
+@pytest.mark.parametrize("n_in", [8, 128, 376, 384, 392, 768, 776, 1528, 1536, 1544])
+@pytest.mark.parametrize("n_out", [2, 300, 5000])
+def test_matvec_f32_row_lengths(pkg, orc, synth, n_in, n_out):
+    """Around the lengths at which another kernel takes over (384, 768, 1536), from one row pair in all to several per warp.  A result has gone
+    through one rounding per product of its lane (four of every 128) and five on the way round the lanes, each at most 2^-24 of the sum of
+    magnitudes."""
+    A = synth.normal_f32(n_in * n_out, n_in + n_out, 0.02).reshape(n_out, n_in)
+    x = synth.normal_f32(n_in, 81, 1.0)
+    y = np.zeros(n_out, np.float32)
+    pkg.matmul_(y, A, x)
+    bound = (4 * -(-n_in // 128) + 5) * 2.0 ** -24 * (np.abs(A.astype(np.float64)) @ np.abs(x.astype(np.float64)))
+    assert (np.abs(y - A.astype(np.float64) @ x.astype(np.float64)) <= bound).all()
+
+
 @pytest.mark.parametrize("n", [288, 4096, 8192, 14336])
 def test_rmsnorm(L, orc, n):
     rng = np.random.default_rng(40)
