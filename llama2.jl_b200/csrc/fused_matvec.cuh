@@ -738,6 +738,13 @@ __device__ __forceinline__ void epilogue_pair(const MvParams& p, const MvSegment
     }
 }
 
+// Kernel parameters come through a cache that is cold at every launch, a line at a time: read one after the other where they are used, the
+// producer's cost half a microsecond before the first copy.  This reads one of every line at once.
+__device__ __forceinline__ void touch_params(const MvParams& p) {
+    asm volatile("" ::"l"(p.seg[0].w), "r"(p.seg[0].npairs), "r"(p.seg[0].rowb), "l"(p.seg[1].w), "r"(p.seg[1].rowb), "l"(p.seg[2].w), "r"(p.seg[2].rowb), "r"(p.nseg),
+                 "r"(p.units_lo), "r"(p.cgroups), "r"(p.pro), "l"(p.pos), "l"(p.amax_val), "l"(p.status));
+}
+
 // ---- the kernel --------------------------------------------------------------------------------
 // DBG = true compiles in the measurement aids (timeline stamps, skip-arithmetic / skip-copies switches); the production
 // instantiations carry none of them: even a predicated-off stamp in the producer's loop cost 2 % of a token.
@@ -771,20 +778,25 @@ __global__ void __launch_bounds__((MV_MAX_CONSUMERS + 2) * 32, 1) fused_matvec_k
     };
 
     if (KQ) {
-        if (threadIdx.x < NS) {
-            mbar_init(full + threadIdx.x, 1);
-            mbar_init(empty + threadIdx.x, W / p.cgroups);
-        }
-        if (threadIdx.x >= 32 && threadIdx.x < 32 + MV_RED_BUFS) {
-            mbar_init(red_full + (threadIdx.x - 32), W / p.cgroups);
-            mbar_init(red_empty + (threadIdx.x - 32), 1);
-        }
-        if (threadIdx.x == 31) mbar_init(ss_ready, W);
-        if (threadIdx.x < 32 + MV_RED_BUFS) {
+        // The producer's first copy is what an HBM-bound launch waits for: that warp sets up its barriers itself and goes on; the others wait for it.
+        if (warp == W) {
+            touch_params(p);
+            if (lane < NS) {
+                mbar_init(full + lane, 1);
+                mbar_init(empty + lane, W / p.cgroups);
+            }
+            if (lane < MV_RED_BUFS) {
+                mbar_init(red_full + lane, W / p.cgroups);
+                mbar_init(red_empty + lane, 1);
+            }
+            if (lane == 31) mbar_init(ss_ready, W);
             fence_barrier_init();
             fence_proxy_async();
+            __syncwarp();
+            asm volatile("bar.arrive 2, %0;" ::"r"((W + 2) * 32) : "memory");
+        } else {
+            asm volatile("bar.sync 2, %0;" ::"r"((W + 2) * 32) : "memory");
         }
-        __syncthreads();
     }
     MV_TRACE(7);
 
@@ -1031,6 +1043,21 @@ __global__ void __launch_bounds__((MV_MAX_CONSUMERS + 2) * 32, 1) fused_matvec_k
     // kernel): fetched now, behind the previous kernel's tail, instead of as two dependent round trips after the wait.
     unsigned tp_epoch = 0;
     if (TP && p.tp && p.tp->part_src != nullptr) tp_epoch = __ldcg(p.tp->tp_epoch);
+    // (everything that does not hang on the vector comes before the wait)
+    const int grp = KQ && p.cgroups == 2 ? (warp >= (W >> 1) ? 1 : 0) : 0;
+    int unit = (int)blockIdx.x + grp * (int)gridDim.x, seg_i = -1, seg_end = 0, seg_first = 0;
+    MvSegment sg = p.seg[0];
+    int bb = 0, offA = 0, offB = 0;
+    const int pj = ((lane >> 2 & 3) << 1) | (lane >> 4);  // the pair of the tile this lane group works on: (0,2,4,6,1,3,5,7)[lane / 4]
+    auto enter_segment = [&]() {
+        seg_i = find_unit<true>(p, unit).seg;
+        sg = get_segment(p, seg_i);
+        seg_first = (seg_i == 0) ? 0 : (seg_i == 1 ? p.seg_start[1] : p.seg_start[2]);
+        seg_end = (seg_i == 0) ? p.seg_start[1] : (seg_i == 1 ? p.seg_start[2] : p.seg_start[3]);
+        bb = dev_block_bytes(sg.type);
+        pair_offsets(sg, sg.rowb, pj, offA, offB);
+    };
+    if (KQ && !TP) enter_segment();  // (with TP the summing prologue needs the registers)
     pdl_wait();
     MV_TRACE(2);
 
@@ -1058,30 +1085,18 @@ __global__ void __launch_bounds__((MV_MAX_CONSUMERS + 2) * 32, 1) fused_matvec_k
         cx.xs16 = reinterpret_cast<const float*>(smem + L.off_xs);
         tile_ctx_columns<NB, P>(cx, smem + L.off_act, L.plane_stride, lane);
         if (NB == 2) cx.xs16 = reinterpret_cast<const float*>(smem + L.off_xs) + (cx.t >> 1) * (p.n_in / QK_K) * 16;  // this lane's vector
-        const int pj = ((cx.g & 3) << 1) | (cx.g >> 2);  // the pair of the tile this lane group works on: (0,2,4,6,1,3,5,7)[g]
         float* red = reinterpret_cast<float*>(smem + L.off_red);
         bool dead = false;
         // counters kept incrementally (no run-time divisions in the loop): weight slot and its phase parity,
         // reduction buffer and its phase parity, and the warp whose turn it is to finish a tile
         const int CG = p.cgroups, WG = W / CG, NSG = NS / CG;
-        const int grp = warp / WG, wl = warp - grp * WG;  // this warp's group and its index inside the group
+        const int wl = warp - grp * WG;  // this warp's index inside its group
         int slot_i = grp * NSG, rb = grp, red_wrap = 0;
         uint32_t full_par = 0;
         // Per-tile bookkeeping is incremental: the segment descriptor and everything derived from it change only
         // when the unit number crosses into the next segment (serial code here runs at ~20 cycles per instruction).
-        int unit = (int)blockIdx.x + grp * (int)gridDim.x, seg_i = -1, seg_end = 0, seg_first = 0;
-        MvSegment sg = p.seg[0];
-        int bb = 0, offA = 0, offB = 0;
         for (int j = grp; j < my_units; j += CG, unit += CG * (int)gridDim.x) {
-            if (seg_i < 0 || unit >= seg_end) {
-                const UnitInfo u0 = find_unit<true>(p, unit);
-                seg_i = u0.seg;
-                sg = get_segment(p, seg_i);
-                seg_first = (seg_i == 0) ? 0 : (seg_i == 1 ? p.seg_start[1] : p.seg_start[2]);
-                seg_end = (seg_i == 0) ? p.seg_start[1] : (seg_i == 1 ? p.seg_start[2] : p.seg_start[3]);
-                bb = dev_block_bytes(sg.type);
-                pair_offsets(sg, sg.rowb, pj, offA, offB);
-            }
+            if (unit >= seg_end) enter_segment();  // (TP: the first one as well, seg_end = 0)
             UnitInfo u;
             u.seg = seg_i;
             u.pair0 = (unit - seg_first) * MV_TILE_PAIRS;
