@@ -1,5 +1,6 @@
 // Matrix-vector product of the decode path of layer-stack models: bf16 weights, f32 activations and accumulation.  The counterpart
-// of fused_matvec_kernel for matrices stored in bf16.
+// of fused_matvec_kernel for matrices stored in bf16.  dense_matvec_kernel takes rows of any length, dense_rows_kernel (below) rows that fit
+// into a warp's registers.
 //
 // One block per SM, 8 consumer warps and a producer warp, every block a contiguous range of rows.
 //   producer : a stage is 4 * gs rows x cs 256-value chunks (16 KiB at most); stages come into a ring with bulk asynchronous copies
@@ -266,6 +267,145 @@ __global__ void __launch_bounds__(DMV_THREADS, 2) dense_matvec_kernel(const __gr
     if (threadIdx.x == 0) {
         for (int w = 1; w < DMV_WARPS; ++w)
             if (better(s_red[w], s_idx[w], best, best_i)) best = s_red[w], best_i = s_idx[w];
+        p.amax_val[b] = best;
+        p.amax_idx[b] = best_i;
+    }
+}
+
+// ---- rows of up to 4096 values -----------------------------------------------------------------------
+// A launch of the decode chain lasts at least as long as its dependent latencies, which is all that a small matrix costs.  Here a warp
+// works on a result by itself: its first row (or pair of rows) is in registers before the wait on the previous kernel, the vector meets
+// the block in shared memory once, and the next row's words are asked for as soon as this one's have been used, so that what is in flight
+// stays at 16 rows per SM.  No ring, no mbarriers, no sums across warps.  Product of 5700 x 2048, 16384 x 2048 (pairs): about 1 and 2 us less
+// a launch than through the ring; of 128 rows or 128 columns: the same.
+constexpr int DRW_WARPS = 16, DRW_THREADS = DRW_WARPS * 32;
+__device__ __forceinline__ uint4 ld_weights(const bf16* p) {  // read once: not kept in L1
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+// NC: 256-value chunks of a row at most; R: rows per result (1, 2).
+template <bool RMS, unsigned KINDS, int NC, int R>
+__global__ void __launch_bounds__(DRW_THREADS, 1) dense_rows_kernel(const __grid_constant__ DmvParams p) {
+    extern __shared__ __align__(16) float drw_x[];  // [nchunk * 256], as read_lane_major reads it
+    __shared__ float s_red[DRW_WARPS], s_ss[DRW_WARPS];
+    __shared__ int s_idx[DRW_WARPS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = (int)blockDim.x >> 5, b = (int)blockIdx.x;
+    const int u0 = b * p.per_lo + min(b, p.per_rem), nu = p.per_lo + (b < p.per_rem ? 1 : 0);
+    const bool logits = p.epi.kind == DE_LOGITS || ((KINDS >> DE_AFFINE_LOGITS & 1) && p.epi.kind == DE_AFFINE_LOGITS);
+    uint4 w[R][NC];
+    const bf16* row = p.w + (size_t)(u0 + warp) * R * p.kp + lane * 8;
+    const size_t next = (size_t)W * R * p.kp;
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int r = 0; r < R; ++r) w[r][c] = warp < nu && c * 256 + lane * 8 < p.kp ? ld_weights(row + r * p.kp + c * 256) : make_uint4(0u, 0u, 0u, 0u);
+    pdl_launch_dependents();
+    pdl_wait();
+    {
+        constexpr int U = 4;  // values of a thread whose reads are under way together
+        const int k = p.k, kc = p.nchunk * 256, T = (int)blockDim.x;
+        float scale = 0.f;
+        auto sum_all = [&](float v) {
+            v = warp_sum(v);
+            if (lane == 0) s_red[warp] = v;
+            __syncthreads();
+            float t = 0.f;
+            for (int i = 0; i < W; ++i) t += s_red[i];
+            return t;
+        };
+        if (p.upd.y) {
+            float ss = 0.f;
+            for (int i0 = threadIdx.x; i0 < k; i0 += U * T) {
+                float v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = i0 + u * T < k ? __ldcg(p.upd.y + i0 + u * T) : 0.f;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    ss = fmaf(v[u], v[u], ss);
+                    if (i0 + u * T < k) drw_x[lane_major(i0 + u * T)] = v[u];
+                }
+            }
+            scale = 1.f / sqrtf(sum_all(ss) / (float)k + p.upd.eps);
+        }
+        float xs = 0.f;
+        for (int i0 = threadIdx.x; i0 < kc; i0 += U * T) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = i0 + u * T < k ? __ldcg(p.x + i0 + u * T) : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * T, at = lane_major(i);
+                if (i < k) {
+                    float t = v[u];
+                    if (p.upd.y) t = fmaf(drw_x[at] * scale, __ldg(p.upd.w + i), t);
+                    if (p.upd.step) t += __ldg(p.upd.step + i);
+                    if (p.x_out && b == 0) p.x_out[i] = t;
+                    if (RMS) xs = fmaf(t, t, xs);
+                    drw_x[at] = apply_norm<RMS>(p.norm, t, i);
+                } else if (i < kc) {
+                    drw_x[at] = 0.f;
+                }
+            }
+        }
+        if (RMS) {
+            xs = warp_sum(xs);
+            if (lane == 0) s_ss[warp] = xs;
+        }
+    }
+    __syncthreads();
+    float rms_scale = 1.f;
+    if (RMS) {
+        float ss = 0.f;
+        for (int i = 0; i < W; ++i) ss += s_ss[i];
+        rms_scale = 1.f / sqrtf(ss / (float)p.k + p.norm.eps);
+    }
+    float best = -INFINITY;
+    int best_i = 0x7fffffff;
+    for (int u = warp; u < nu; u += W) {
+        const float old = p.epi.kind == DE_RESIDUAL && lane == 0 ? p.epi.y[u0 + u] : 0.f;
+        row += next;
+        f32x2 acc[R][2];  // two sums a row: the chain of additions is half as long
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0ull;
+        const bool more = u + W < nu;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (c >= p.nchunk) break;
+            const Pairs8 x = read_lane_major(drw_x, c, lane);
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const uint4 q = w[r][c];
+                acc[r][0] = fma2(widen2(q.x), x.p[0], acc[r][0]);
+                acc[r][1] = fma2(widen2(q.y), x.p[1], acc[r][1]);
+                acc[r][0] = fma2(widen2(q.z), x.p[2], acc[r][0]);
+                acc[r][1] = fma2(widen2(q.w), x.p[3], acc[r][1]);
+                if (more && c * 256 + lane * 8 < p.kp) w[r][c] = ld_weights(row + r * p.kp + c * 256);
+            }
+        }
+        float a[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) a[r] = sum2(acc[r][0]) + sum2(acc[r][1]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int r = 0; r < R; ++r) a[r] += __shfl_xor_sync(0xffffffffu, a[r], o);
+        if (lane) continue;
+        float v = a[0] * rms_scale;
+        if (p.epi.kind == DE_RESIDUAL) p.epi.y[u0 + u] = old + v;
+        else dense_epilogue<float, KINDS>(p.epi, 0, u0 + u, v, a[R - 1] * rms_scale);
+        if ((KINDS >> DE_AFFINE_LOGITS & 1) && p.epi.kind == DE_AFFINE_LOGITS) v = affine(p.epi, u0 + u, v);
+        if (v > best) {
+            best = v;
+            best_i = u0 + u;
+        }
+    }
+    if (!logits) return;
+    if (lane == 0) s_red[warp] = best, s_idx[warp] = best_i;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < W; ++i)
+            if (s_red[i] > best || (s_red[i] == best && s_idx[i] < best_i)) best = s_red[i], best_i = s_idx[i];
         p.amax_val[b] = best;
         p.amax_idx[b] = best_i;
     }
