@@ -113,6 +113,8 @@ __device__ __forceinline__ void normed_rotated_quads(const float* src, const flo
 // Grid (parts of the items, rows): the operands of a prompt portion.  Needs dim a multiple of 8 that is its own stored size, vdim a
 // multiple of 8, `lanes` = rdims / 8 a power of two up to 32, ld and offsets multiples of 4.
 __global__ void __launch_bounds__(HA_WARPS * 32) head_rows_quads_kernel(const __grid_constant__ HeadAttnParams p, int lanes) {
+    pdl_launch_dependents();
+    pdl_wait();
     const HeadShape& S = p.s;
     const int row = (int)blockIdx.y, pos = scan_position(p.c, row), per = HA_WARPS * 32 / lanes;  // vectors at a time
     const float2* const cs = p.rope + (size_t)pos * (S.rdims >> 1);

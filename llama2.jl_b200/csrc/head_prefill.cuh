@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(HP_THREADS, 2) head_prefill_kernel(const __gri
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
     const uint32_t tmem = s_tmem, tmem_o = tmem + (uint32_t)(nsb * 128);
 
     if (warp == 0) {
@@ -301,6 +302,7 @@ __global__ void __launch_bounds__(HP_THREADS, 2) head_prefill_kernel(const __gri
             }
         }
     }
+    pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, nsb * 256);

@@ -62,6 +62,8 @@ __device__ __forceinline__ void store_latent_row(const LatentAttnParams& p, int 
 template <typename CT>
 __global__ void __launch_bounds__(128) latent_rows_kernel(const __grid_constant__ LatentAttnParams p) {
     __shared__ float s_red[4];
+    pdl_launch_dependents();
+    pdl_wait();
     store_latent_row<CT, 4>(p, (int)blockIdx.x, scan_position(p.c, (int)blockIdx.x), s_red);
 }
 

@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prefill_kernel(const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
     const uint32_t tmem = s_tmem, tmem_o = tmem + 256;
 
     if (warp == 0) {
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prefill_kernel(const __grid
             }
         }
     }
+    pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);
@@ -289,6 +291,8 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prefill_kernel(const __grid
 // Grid (rows, heads); a thread makes two values.
 __global__ void __launch_bounds__(128) latent_queries_kernel(const float* __restrict__ qdg, int ld, const float2* __restrict__ rope, int pos0, LatentShape s, int dq,
                                                             bf16* __restrict__ out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int row = (int)blockIdx.x, h = (int)blockIdx.y;
     const float2* cs = rope + (size_t)(pos0 + row) * (s.rdims >> 1);
     const float* q = qdg + (size_t)row * ld + h * (s.dim + s.rot);

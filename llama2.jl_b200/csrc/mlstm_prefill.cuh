@@ -35,6 +35,8 @@ struct MlstmPrefillParams {
 
 // Grid (n): one token's operands.
 __global__ void __launch_bounds__(256) mlstm_operands_kernel(const __grid_constant__ MlstmPrefillParams p) {
+    pdl_launch_dependents();
+    pdl_wait();
     const MlstmShape& S = p.m.s;
     const int t = (int)blockIdx.x;
     const float* const in = p.m.in + (size_t)t * p.m.ld;
@@ -54,6 +56,8 @@ __global__ void __launch_bounds__(256) mlstm_operands_kernel(const __grid_consta
 // Grid (heads), a warp per chunk, a lane four consecutive tokens.
 __global__ void __launch_bounds__(MP_MAX_CHUNKS * 32) mlstm_gates_kernel(const __grid_constant__ MlstmPrefillParams p) {
     __shared__ float s_f[MP_MAX_CHUNKS], s_a[MP_MAX_CHUNKS];
+    pdl_launch_dependents();
+    pdl_wait();
     const MlstmShape& S = p.m.s;
     const int h = (int)blockIdx.x, c = (int)threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* const gm = p.m.state + S.m_at() + (size_t)h * S.cl;
@@ -150,6 +154,7 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_state_kernel(const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
     const uint32_t tmem = s_tmem;
 
     if (warp == 0) {
@@ -278,6 +283,7 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_state_kernel(const __grid
         }
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
     }
+    pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 128);
@@ -335,6 +341,7 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_chunk_kernel(const __grid
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_wait();
     const uint32_t tmem = s_tmem, tmem_a = tmem, tmem_o = tmem + 128, tmem_r = tmem + 256;
     if (p.vt > 1) cluster_arrive();  // (waited for before the first store into another block's shared memory)
     float o[2][32];                  // this thread's results (columns 32 half + 64 i ..)
@@ -531,6 +538,7 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_chunk_kernel(const __grid
             }
         }
     }
+    pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);

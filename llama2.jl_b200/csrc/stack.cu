@@ -954,15 +954,14 @@ static int32_t launch_gemm(const StackSession* s, const StackMatrix& w, const vo
     L2B_TRY(bf16_map(mb, static_cast<const bf16*>(x), w.k, n, ldx, g.N / 2));
     const dim3 grid(2u * (unsigned)std::min(g.mtiles * g.ntiles, s->di.sms / 2)), block(BG_THREADS);
     const size_t smem = (size_t)g.stages * stage + swap + 1024;
-    CU(launch_kernel_args(dual ? bf16_gemm_kernel<true> : bf16_gemm_kernel<false>, grid, block, smem, st, false, 2, g, ma, ma2, mb));
+    CU(launch_kernel_args(dual ? bf16_gemm_kernel<true> : bf16_gemm_kernel<false>, grid, block, smem, st, true, 2, g, ma, ma2, mb));
     return L2B_OK;
 }
 
 static int32_t launch_residual_rows(const StackSession* s, const RowsParams& r, int n, cudaStream_t st) {
     const bool wide = r.width % 4 == 0;
-    if (s->m->f32) wide ? residual_rows_kernel<float, 4><<<n, 256, 0, st>>>(r) : residual_rows_kernel<float, 1><<<n, 256, 0, st>>>(r);
-    else wide ? residual_rows_kernel<bf16, 4><<<n, 256, 0, st>>>(r) : residual_rows_kernel<bf16, 1><<<n, 256, 0, st>>>(r);
-    CU(cudaGetLastError());
+    auto go = [&](auto k) { return launch_kernel(k, dim3(n), dim3(256), 0, st, true, r); };
+    CU(s->m->f32 ? wide ? go(residual_rows_kernel<float, 4>) : go(residual_rows_kernel<float, 1>) : wide ? go(residual_rows_kernel<bf16, 4>) : go(residual_rows_kernel<bf16, 1>));
     return L2B_OK;
 }
 
@@ -993,9 +992,7 @@ static int32_t enqueue_latent_rows(StackSession* s, int run, int n, int pos0, co
     a.c.status = status;
     a.out = s->act2;
     a.ldo = ldo;
-    if (m->f32) latent_rows_kernel<float><<<n, 128, 0, st>>>(a);
-    else latent_rows_kernel<bf16><<<n, 128, 0, st>>>(a);
-    CU(cudaGetLastError());
+    CU(launch_kernel(m->f32 ? latent_rows_kernel<float> : latent_rows_kernel<bf16>, dim3(n), dim3(128), 0, st, true, a));
     ++*launches;
     const int kstages = prefill_kstages(sh, s->di);
     if (!s->pq || pos_list || n < EXPAND_MIN_ROWS || kstages == 0 || !(sh.scale2 > 0.f))
@@ -1008,8 +1005,7 @@ static int32_t enqueue_latent_rows(StackSession* s, int run, int n, int pos0, co
     const bf16* cache = static_cast<const bf16*>(a.c.cache);
     L2B_TRY(launch_gemm(s, w.uk, cache, sh.row, npos, dense_epilogue_of(DE_STORE_ACT, nullptr, s->pk, sh.heads * sh.dp), status, st));
     L2B_TRY(launch_gemm(s, w.uv, cache, sh.row, npos, dense_epilogue_of(DE_STORE_T, nullptr, s->pv, s->pv_ld), status, st));
-    latent_queries_kernel<<<dim3(n, sh.heads), 128, 0, st>>>(s->in, a.ld, a.rope, pos0, sh, dq, s->pq);
-    CU(cudaGetLastError());
+    CU(launch_kernel_args(latent_queries_kernel, dim3(n, sh.heads), dim3(128), 0, st, true, 1, (const float*)s->in, a.ld, a.rope, pos0, sh, dq, s->pq));
     LatentPrefillParams f;
     memset(&f, 0, sizeof(f));
     f.n = n; f.pos0 = pos0; f.dim = sh.dim; f.rot = sh.rot; f.vdim = sh.vdim; f.dp = sh.dp; f.dq = dq; f.vp = sh.vp; f.kstages = kstages;
@@ -1020,7 +1016,7 @@ static int32_t enqueue_latent_rows(StackSession* s, int run, int n, int pos0, co
     L2B_TRY(bf16_map(mkr, cache + sh.rp, sh.rot, npos, sh.row, LP_TILE));
     L2B_TRY(bf16_map(mv, s->pv, npos, (int64_t)sh.heads * sh.vp, s->pv_ld, sh.vp));
     const size_t smem = (size_t)lp_smem_layout(sh.dim, sh.rot, sh.vp, kstages).total + 1024;
-    CU(launch_kernel_args(latent_prefill_kernel, dim3((n + LP_TILE - 1) / LP_TILE, sh.heads), dim3(LP_THREADS), smem, st, false, 1, f, mq, mk, mkr, mv));
+    CU(launch_kernel_args(latent_prefill_kernel, dim3((n + LP_TILE - 1) / LP_TILE, sh.heads), dim3(LP_THREADS), smem, st, true, 1, f, mq, mk, mkr, mv));
     *launches += 4;
     return L2B_OK;
 }
@@ -1050,7 +1046,7 @@ static int32_t enqueue_head_rows(StackSession* s, int run, int n, int pos0, cons
     a.pg = s->pg;
     const int lanes = sh.rdims / 8, vectors = 2 * sh.heads + (a.own_kv ? 2 * sh.kv_heads : 0), per = lanes ? HA_WARPS * 32 / lanes : 1;
     if (sh.rdims % 8 == 0 && lanes && (lanes & (lanes - 1)) == 0 && lanes <= 32 && sh.dim % 16 == 0 && sh.vdim % 8 == 0)
-        head_rows_quads_kernel<<<dim3((vectors + per - 1) / per, n), HA_WARPS * 32, 0, st>>>(a, lanes);
+        CU(launch_kernel_args(head_rows_quads_kernel, dim3((vectors + per - 1) / per, n), dim3(HA_WARPS * 32), 0, st, true, 1, a, lanes));
     else launch_head_rows<bf16>(a, n, false, st);
     CU(cudaGetLastError());
     HeadPrefillParams f;
@@ -1063,7 +1059,7 @@ static int32_t enqueue_head_rows(StackSession* s, int run, int n, int pos0, cons
     L2B_TRY(bf16_map(mkv, static_cast<const bf16*>(a.c.cache), sh.row, pos0 + n, sh.row, HP_TILE, sh.kv_heads, (int64_t)a.c.group_stride));
     L2B_TRY(bf16_map(mg, s->pg, (int64_t)sh.heads * sh.vp, n, (int64_t)sh.heads * sh.vp, HP_TILE));
     const size_t smem = (size_t)hp_smem_layout(sh.dim, f.vn, kstages).total + 1024;
-    CU(launch_kernel_args(head_prefill_kernel, dim3(blocks), dim3(HP_THREADS), smem, st, false, 1, f, mq, mkv, mg));
+    CU(launch_kernel_args(head_prefill_kernel, dim3(blocks), dim3(HP_THREADS), smem, st, true, 1, f, mq, mkv, mg));
     *launches += 2;
     return L2B_OK;
 }
@@ -1099,13 +1095,11 @@ static int32_t enqueue_mlstm_rows(StackSession* s, int run, int n, int pos0, con
         L2B_TRY(bf16_map(mg, p.g, nv, n, nv, MP_L));
         L2B_TRY(bf16_map(msh, p.sh, p.vs, rows, p.vs, MC_ROWS));
         L2B_TRY(bf16_map(msl, p.sl, p.vs, rows, p.vs, MC_ROWS));
-        mlstm_operands_kernel<<<n, 256, 0, st>>>(p);
-        CU(cudaGetLastError());
-        mlstm_gates_kernel<<<sh.heads, 32 * p.nchunk, 0, st>>>(p);
-        CU(cudaGetLastError());
+        CU(launch_kernel(mlstm_operands_kernel, dim3(n), dim3(256), 0, st, true, p));
+        CU(launch_kernel(mlstm_gates_kernel, dim3(sh.heads), dim3(32 * p.nchunk), 0, st, true, p));
         const dim3 sgrid((sh.vdim + MP_STATE_COLS - 1) / MP_STATE_COLS, (sh.dim + 127) / 128, sh.heads), cgrid(p.vt, p.nchunk, sh.heads);
-        CU(launch_kernel_args(mlstm_state_kernel, sgrid, dim3(MP_THREADS), (size_t)MsSmem::total + 1024, st, false, 1, p, mk));
-        CU(launch_kernel_args(mlstm_chunk_kernel, cgrid, dim3(MP_THREADS), (size_t)mc_smem_layout(p.dp, stages).total + 1024, st, false, p.vt, p, mq, mk, mv, msh, msl, mg));
+        CU(launch_kernel_args(mlstm_state_kernel, sgrid, dim3(MP_THREADS), (size_t)MsSmem::total + 1024, st, true, 1, p, mk));
+        CU(launch_kernel_args(mlstm_chunk_kernel, cgrid, dim3(MP_THREADS), (size_t)mc_smem_layout(p.dp, stages).total + 1024, st, true, p.vt, p, mq, mk, mv, msh, msl, mg));
         *launches += 4;
         return L2B_OK;
     }

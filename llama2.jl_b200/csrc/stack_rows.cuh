@@ -66,6 +66,8 @@ struct RowsParams {
 template <typename AT, int V>
 __global__ void __launch_bounds__(256) residual_rows_kernel(const __grid_constant__ RowsParams p) {
     __shared__ float s_red[8], s_red2[8];
+    pdl_launch_dependents();
+    pdl_wait();
     struct alignas(4 * V) F { float v[V]; };
     struct alignas(sizeof(AT) * V) A { AT v[V]; };
     const int src = p.index ? __ldg(p.index + blockIdx.x) : (int)blockIdx.x;
