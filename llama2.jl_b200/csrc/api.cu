@@ -1906,16 +1906,21 @@ constexpr int STACK_MIN_ROWS = 2;  // layer-stack models
 
 // Attention of one sequence's tokens at pos0 ..: heads of a multiple of 16 values, at most 128, take the tensor-core kernel.
 // A block of it takes 12.5 us and per 64 positions 1.1 us and 0.0445 us per dim; the split kernel 11 us and per 10000 pairs of a query head and a
-// position 0.55 us, 0.88 us where no query heads share a key head (fits to 27, 68 us: 128 and 512 queries, 32 heads of 128 on 8; 155: 256 behind 1500,
-// 32 of 96; 35: 300 behind 21, 16 of 64 on 2; 19: 100 behind 77, 8 of 32 on 4; split: 25, 224, 1177, 58, 17; within 15 %).
+// position 0.37 us, 0.7 us where no query heads share a key head (fits to 27, 68 us: 128 and 512 queries, 32 heads of 128 on 8; 155: 256 behind 1500,
+// 32 of 96; 35: 300 behind 21, 16 of 64 on 2; 19: 100 behind 77, 8 of 32 on 4; split: 19, 37, 66, 159: 128, 211, 300 and 500 queries, 32 heads of 128
+// on 8; 141, 654: 300, and 200 behind 1500, 32 of 96; within 20 %).
 static bool prompt_attention_better(int n, int pos0, int n_heads, int gq, int hs, int sms, int asked) {
     if (hs % 16 != 0 || hs > PA_MAX_HS) return false;
     if (asked) return asked == 1;
     const int tq = PA_ROWS / gq, blocks = (n + tq - 1) / tq * (n_heads / gq), waves = (blocks + sms - 1) / sms;
     const double tiled = 12.5 + (1.1 + 0.0445 * hs) * waves * ((pos0 + n + PA_KEYS - 1) / PA_KEYS);
-    const double split = 11.0 + (gq > 1 ? 0.55e-4 : 0.88e-4) * n_heads * n * (pos0 + 0.5 * n);
+    const double split = 11.0 + (gq > 1 ? 0.37e-4 : 0.7e-4) * n_heads * n * (pos0 + 0.5 * n);
     return tiled < split;
 }
+// Parts that a query's positions are in, for the split kernel: so many that few queries still make about four blocks per SM (29 queries behind 211, 32
+// heads on 8: 25 us with one part each, 14 us with eight).
+constexpr int SPLIT_BLOCKS = 600, SPLIT_MOST = 8;
+static int prompt_splits(int n, int groups, const GemmBufs& B) { return std::max(B.nsplit, std::min(SPLIT_MOST, SPLIT_BLOCKS / std::max(1, n * groups))); }
 static int32_t launch_prompt_attention(const PromptAttnParams& a, int gq, cudaStream_t st) {
     const size_t smem = (size_t)pa_smem_layout(a.hs).total + 1024;
     const int tq = PA_ROWS / gq;
@@ -1982,10 +1987,12 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
             a.q = B.q; a.kc = kcl; a.vc = vcl; a.out = B.att; a.tickets = B.tickets;
             a.part_m = B.pm; a.part_l = B.pl; a.part_acc = B.pacc;
             a.pos = nullptr; a.pos_base = pos0; a.pos_list = pos_list; a.cache_stride_q = seq_stride;
-            a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.hs = hs; a.seq_len = c.seq_len; a.nsplit = B.nsplit;
+            a.n_heads = c.n_heads; a.n_kv = c.n_kv_heads; a.hs = hs; a.seq_len = c.seq_len;
+            a.nsplit = pos_list ? B.nsplit : prompt_splits(n, c.n_heads / gq, B);
             a.nq = std::max(n, 2);  // (a one-token pass takes the many-query form of the kernel too: the second query copy leaves at once)
             a.q_stride = c.dim;
-            a.min_chunk = 256;  // many queries already fill the GPU: split a query's positions only when there are many
+            // many queries already fill the GPU: split a query's positions only when there are many; few do not
+            a.min_chunk = a.nsplit > B.nsplit ? 32 : 256;
             if (n < 2) return fail(L2B_ERR_BAD_ARG, "a many-token pass needs at least two tokens");
             CU(launch_attention(a, gq, st, true));
         }
@@ -2030,9 +2037,10 @@ static bool alloc_gemm_bufs(const l2b_model* m, GemmBufs& B, size_t T, bool batc
         B.y_bytes = std::max({B.y_bytes, need({&w.wq, &w.wk, &w.wv}, n), need({&w.wo}, n), need({&w.w1, &w.w3}, n), need({&w.w2}, n)});
     if (batch && m->output.type != T_F32) B.y_bytes = std::max(B.y_bytes, gemm_product_bytes(m->output, (int)T, B.sms));
     auto alloc = [&](auto*& ptr, size_t bytes) { return cudaMalloc((void**)&ptr, bytes) == cudaSuccess; };
+    // partial results of the split attention kernel: prompt_splits() of a few queries' heads are at most SPLIT_BLOCKS blocks of up to 8 heads each
+    const size_t parts = std::max(T * c.n_heads * B.nsplit, batch ? (size_t)0 : (size_t)SPLIT_BLOCKS * 8);
     bool ok = alloc(B.x, T * c.dim * 4) && alloc(B.q, T * c.dim * 4) && alloc(B.att, T * c.dim * 4) && alloc(B.h, T * c.hidden_dim * 4) && alloc(B.y, B.y_bytes) &&
-              alloc(B.pm, T * c.n_heads * B.nsplit * 4) && alloc(B.pl, T * c.n_heads * B.nsplit * 4) &&
-              alloc(B.pacc, T * c.n_heads * B.nsplit * hs * 4) && alloc(B.tickets, T * c.n_heads * 4) &&
+              alloc(B.pm, parts * 4) && alloc(B.pl, parts * 4) && alloc(B.pacc, parts * hs * 4) && alloc(B.tickets, T * c.n_heads * 4) &&
               alloc(B.act, gemm_input_bytes(std::max(c.dim, c.hidden_dim), (int)T));
     if (ok) ok = cudaMemset(B.tickets, 0, T * c.n_heads * 4) == cudaSuccess;
     if (!ok) {

@@ -51,6 +51,22 @@ def test_prompt_passes_against_oracle(pkg, orc, synth, kernel, dim, heads, kv, n
     model.close()
 
 
+@pytest.mark.parametrize("heads,kv", [(8, 8), (8, 4), (8, 2), (8, 1)])
+@pytest.mark.parametrize("n", [10, 19])
+def test_few_queries_behind_many_positions(pkg, orc, synth, heads, kv, n):
+    """Few queries' positions are shared out among up to eight blocks each (the split kernel, one to eight heads per key head).  Bound as above."""
+    cfg = pkg.ModelConfig(512, 256, 1, heads, kv, 512, 320, 10000.0, False)
+    w = synth.model_weights(cfg, dict(synth.ALL(12), output=14), seed=heads + kv)
+    ids = synth.tokens(261 + n, 7 + n, 3, cfg.vocab_size)
+    _, want = orc.OracleModel(cfg, w).sample_greedy(ids, len(ids), want_logits=True)
+    model = pkg.LanguageModel(cfg, None, w)
+    st = pkg.RunState(model)
+    pkg.prefill(st, ids[:261], 0)
+    pkg.prefill(st, ids[261:], 261)
+    assert np.abs(st.logits - want[-1]).max() / float(want[-1].max() - want[-1].min()) < 5e-5
+    model.close()
+
+
 def test_positions_behind_do_not_matter(pkg, synth, kernel):
     """Two prompts that differ from position 60 on, the second with an id there whose embedding is infinite: the rows before it in the cache have
     the same bits, which position 59, fed once more, shows in its logits."""
