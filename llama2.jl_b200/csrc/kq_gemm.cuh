@@ -21,8 +21,8 @@
 //   packed-copy warp  one TMA tiled copy (cp.async.bulk.tensor) per super-block: a 128-row box of the stored blocks
 //   2 operand warps   one bulk copy per 64 values: the tokens' two terms, already in operand layout (split_rows_kernel); a thread takes 750
 //                     cycles to see a slot free and issue a copy, so two take turns
-//   unpack warps      groups of four; thread = row: nibbles -> fp16 times scale, into core matrices (8 rows x 16 bytes) or, for tiles of more
-//                     than 64 tokens, into tensor memory (lane = row)
+//   unpack warps      groups of four; thread = row: nibbles -> fp16 times scale, into tensor memory (lane = row) or, for tiles of 33 - 64
+//                     tokens, into core matrices (8 rows x 16 bytes)
 //   MMA warp          tcgen05.mma.kind::f16 (M 128, K 16), four or eight per 64 values
 //   8 epilogue warps  thread = weight row, half of the tokens: tensor memory -> times d -> f32 accumulators, and those of four
 //                     super-blocks -> f32 sums in tensor memory (one chain over 14336 values would be 280 roundings long)
@@ -98,20 +98,23 @@ struct GemmMaps {
 // reads them again), as much as an SM delivers while they run, and copies and unpacking want another 57 KB.  From tensor memory the weights cost
 // nothing of it, and there is room for four slots of activations: 1240 -> 930 cycles per 64 values (q4_K 28672 x 4096 times 128).  That leaves two
 // sets of accumulators instead of three.  (Blocks in pairs that share the activations, cta_group::2: 1270 - 1350 cycles; 16 epilogue warps: no
-// faster.)  Narrower tiles spend their time on the unpack warps' instructions and keep the deeper accumulators.
+// faster.)  With 32 tokens an MMA takes 46 cycles instead of 16 for the weights' sake, and the unpack warps, whose instructions bound the kernel
+// there, wait behind it: 24 sequences of the 8B shape 10.6 -> 10.1 ms, 29 tokens 2.46 -> 2.31 ms.  With 64 there is no room beside two slots of
+// accumulators; a chunk per step, which leaves some, costs more in hand-overs (56 against 53 us, q5_K 14336 x 4096 times 37).
 // Whatever the tile holds, a column's sums are the same ones in the same order: low terms, then high terms of 64 values in one accumulator,
 // added to the f32 sum chunk by chunk, the shared part behind them.  So a column's result does not hang on how many columns came with it.
 template <int NT>
 struct GmCfg {
     static constexpr int CH = NT == 128 ? 1 : 2;
-    static constexpr bool AT = NT == 128;  // weights go through tensor memory
-    static constexpr int NS = NT == 64 ? 2 : NT == 32 ? 3 : 4, ND = NT == 32 ? 3 : 2;
+    static constexpr bool AT = NT != 64;  // weights go through tensor memory
+    static constexpr int NS = NT == 64 ? 2 : NT == 32 ? 3 : 4, ND = 2;
     static constexpr int GS = NT == 64 ? 2 : 1, UG = NT == 128 ? 2 : NT == 64 ? 4 : 3;
     static_assert(UG / GS <= NS, "a group would miss a phase");
     static constexpr int DCOLS = CH == 1 ? NT : 3 * NT;  // accumulator columns per slot: 128, 192, 96
     static constexpr int SUMS = ND * DCOLS, A_COLS = SUMS + NT;  // columns where the sums and the weights stand
     static_assert(ND <= NS, "a step's accumulators are waited for at its own slot");
-    static_assert(A_COLS + (AT ? 32 * NS : 0) <= 512, "accumulators, sums, weights");
+    static constexpr int A_SLOT = CH == 2 ? 80 : 32;  // 32 a chunk, 16 for the shared part
+    static_assert(A_COLS + (AT ? A_SLOT * NS : 0) <= 512, "accumulators, sums, weights");
     static constexpr int THREADS = (GM_EPI_WARPS + 4 + 4 * UG) * 32;  // warps 0-7 epilogue, 8 packed copies, 9 MMA, 10 and 11 operand copies, 12 .. unpack
 };
 constexpr int GM_MAX_PACKED = 5;
@@ -560,7 +563,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         const uint64_t desc_xs = umma_desc(smem + L.off_b, 128, GM_XS_BYTES);
         // a: slot of the weights; ka, kb: bytes further in it and in the operand of the activations
         auto mma = [&](uint32_t d, int a, int ka, uint64_t b, uint32_t accumulate) {
-            if (AT) umma_f16_at(d, tmem_base + (uint32_t)(GmCfg<NT>::A_COLS + 32 * a + (ka >> 9)), b, idesc, accumulate);  // (4096 bytes: 8 columns)
+            if (AT) umma_f16_at(d, tmem_base + (uint32_t)(GmCfg<NT>::A_COLS + GmCfg<NT>::A_SLOT * a + (ka >> 9)), b, idesc, accumulate);  // (4096 bytes: 8 columns)
             else umma_f16(d, desc_a + (uint64_t)((a * L.slot_a + ka) >> 4), b, idesc, accumulate);
         };
         int s = 0, ds = 0;
@@ -680,12 +683,12 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 // (the epilogue may still be at the super-block before the last one: four sets of factors are enough)
                 if (k == 0 && sub == 0) hdr[hs * GM_ROWS + r] = make_float2(d * (float)(1 << GM_A_EXP), 32.f * s_dn);
                 uint8_t* const a_slot = smem + L.off_a + slot * L.slot_a + row_off;
-                const uint32_t a_cols = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(GmCfg<NT>::A_COLS + 32 * slot);
+                const uint32_t a_cols = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(GmCfg<NT>::A_COLS + GmCfg<NT>::A_SLOT * slot);
                 if (CH == 2 || type == T_Q6_K || k < 4) {
 #pragma unroll 1
                     for (int e = sub; e < CH; e += GS) {
                         const int kc = CH * k + e;
-                        const GmDest<AT> dst = {a_slot + e * GM_A_BYTES, a_cols};
+                        const GmDest<AT> dst = {a_slot + e * GM_A_BYTES, a_cols + (uint32_t)(32 * e)};
                         uint32_t o[8];
                         if (type == T_Q6_K) {
                             const int c = kc & 3, hh = c >> 1, odd = c & 1;
@@ -735,7 +738,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                     }
                 }
                 if (type != T_Q6_K && k == (CH == 2 ? 1 : 4) && sub == GS - 1) {
-                    const GmDest<AT> dst = {a_slot + (CH == 2 ? 2 * GM_A_BYTES : 0), a_cols};
+                    const GmDest<AT> dst = {a_slot + (CH == 2 ? 2 * GM_A_BYTES : 0), a_cols + (CH == 2 ? 64u : 0u)};
                     uint32_t o[8], o2[8];
 #pragma unroll
                     for (int j2 = 0; j2 < 4; ++j2) {
