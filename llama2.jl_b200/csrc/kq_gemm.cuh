@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(SR_MAX_WARPS * 32) split_rows_kernel(const __g
 }
 
 // A product that is wanted as such: dst[t][i] = the sum of its partial results.  Grid (blocks per row, n_tok): at most 65535 tokens.
-__global__ void sum_parts_kernel(const float* __restrict__ y, size_t part_stride, const __grid_constant__ GemmSplit sp, int ldy, int rows, float* __restrict__ dst) {
+__global__ void sum_parts_kernel(const float* y, size_t part_stride, const __grid_constant__ GemmSplit sp, int ldy, int rows, float* __restrict__ dst) {
     const int tok = blockIdx.y;
     pdl_launch_dependents();
     pdl_wait();
@@ -863,10 +863,17 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                 const bool valid = row < p.seg[w.seg].rows;
                 for (int e = 0; e < w.seg; ++e) row += p.seg[e].row_tiles * GM_ROWS;
                 float* dst = p.y + (size_t)part * p.part_stride + row;
+                float scale[(NH + 31) / 32];  // the tokens' factors, a lane each: read from L2 in front of every store, they would be NH reads in a row
+#pragma unroll
+                for (int i = 0; i < (NH + 31) / 32; ++i) {
+                    const int t = 32 * i + lane, tok = w.ntile * p.sp.tok + NH * half + t;
+                    scale[i] = t < mine && tok < p.n_tok ? __ldcg(p.scale + tok) : 0.f;
+                }
 #pragma unroll
                 for (int t = 0; t < NH; ++t) {
                     const int tok = w.ntile * p.sp.tok + NH * half + t;
-                    if (valid && t < mine && tok < p.n_tok) dst[(size_t)tok * p.ldy] = (t & 1 ? acc[t / 2].y : acc[t / 2].x) * __ldg(p.scale + tok);
+                    const float of_tok = __shfl_sync(0xffffffffu, scale[t / 32], t & 31);
+                    if (valid && t < mine && tok < p.n_tok) dst[(size_t)tok * p.ldy] = (t & 1 ? acc[t / 2].y : acc[t / 2].x) * of_tok;
                 }
 #pragma unroll
                 for (int t = 0; t < NH / 2; ++t) acc[t] = make_float2(0.f, 0.f);

@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prefill_kernel(const __grid
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
                     const int t = q0 + 32 * qd + i;
-                    o[i] = t < p.n && c + lane < p.vdim ? __ldg(p.gate + (size_t)t * p.ld + h * p.vdim + c + lane) : 0.f;
+                    o[i] = t < p.n && c + lane < p.vdim ? __ldcg(p.gate + (size_t)t * p.ld + h * p.vdim + c + lane) : 0.f;
                 }
 #pragma unroll
                 for (int i = 0; i < 32; ++i) sg[i * 33 + lane] = sigmoid(o[i]);
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prefill_kernel(const __grid
 
 // Query operand of the kernel above: [row][head][dq] = unrotated part rounded up to 16 (zeros), rotated part rounded up to 16.
 // Grid (rows, heads); a thread makes two values.
-__global__ void __launch_bounds__(128) latent_queries_kernel(const float* __restrict__ qdg, int ld, const float2* __restrict__ rope, int pos0, LatentShape s, int dq,
+__global__ void __launch_bounds__(128) latent_queries_kernel(const float* qdg, int ld, const float2* rope, int pos0, LatentShape s, int dq,
                                                             bf16* __restrict__ out) {
     pdl_launch_dependents();
     pdl_wait();
@@ -300,13 +300,13 @@ __global__ void __launch_bounds__(128) latent_queries_kernel(const float* __rest
     for (int d = 2 * threadIdx.x; d < dq; d += 256) {
         float v0 = 0.f, v1 = 0.f;
         if (d < s.dp) {
-            v0 = d < s.dim ? q[d] : 0.f;
-            v1 = d + 1 < s.dim ? q[d + 1] : 0.f;
+            v0 = d < s.dim ? __ldcg(q + d) : 0.f;
+            v1 = d + 1 < s.dim ? __ldcg(q + d + 1) : 0.f;
         } else {
             const int r = d - s.dp;  // even: a whole pair, or two unrotated values
             if (r < s.rot) {
-                v0 = rotary_element(r, s.rdims, cs, [&](int j) { return q[s.dim + j]; });
-                v1 = rotary_element(r + 1, s.rdims, cs, [&](int j) { return q[s.dim + j]; });
+                v0 = rotary_element(r, s.rdims, cs, [&](int j) { return __ldcg(q + s.dim + j); });
+                v1 = rotary_element(r + 1, s.rdims, cs, [&](int j) { return __ldcg(q + s.dim + j); });
             }
         }
         *reinterpret_cast<__nv_bfloat162*>(dst + d) = __floats2bfloat162_rn(v0, v1);

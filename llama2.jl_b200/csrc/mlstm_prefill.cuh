@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_state_kernel(const __grid
             const bf16* src = p.v + (size_t)(c * MP_L + tok) * S.heads * p.vp + (size_t)h * p.vp + cc;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                v[i] = c < p.nchunk && c * MP_L + tok < p.n && cc + 8 * i < p.vp ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
-            u = c < p.nchunk ? __ldg(p.u + ((size_t)h * p.nchunk + c) * MP_L + tok) : 0.f;
+                v[i] = c < p.nchunk && c * MP_L + tok < p.n && cc + 8 * i < p.vp ? __ldcg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
+            u = c < p.nchunk ? __ldcg(p.u + ((size_t)h * p.nchunk + c) * MP_L + tok) : 0.f;
         };
         auto weigh = [&](int c) {  // u V of chunk c in two terms; rows are tokens
             uint8_t* const wh = smem + MsSmem::w + (c & 1) * MsSmem::wbytes;
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_state_kernel(const __grid
         bool ok = true;
         for (int c = 0; c <= p.nchunk; ++c) {
             float st[32], n = 0.f;
-            if (c < p.nchunk) decay = __ldg(p.decay + (size_t)h * p.nchunk + c);
+            if (c < p.nchunk) decay = __ldcg(p.decay + (size_t)h * p.nchunk + c);
             if (c == 0) {
 #pragma unroll
                 for (int k = 0; k < 32; ++k) st[k] = !fresh && row_in && cc + k < S.vdim ? gs[k] : 0.f;
@@ -423,10 +423,10 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_chunk_kernel(const __grid
         const int qd = warp & 3, half = (warp - 2) >> 2, r = 32 * qd + lane, tid = (int)threadIdx.x - 64;
         const uint32_t lane_off = (uint32_t)(32 * qd) << 16;
         const size_t at = ((size_t)h * p.nchunk + c) * MP_L;
-        if (tid < MP_L) s_g[tid] = __ldg(p.a + at + tid);
+        if (tid < MP_L) s_g[tid] = __ldcg(p.a + at + tid);
         if (state)
-            for (int i = tid; i < p.dp; i += MP_WARPS * 32) s_n[i] = __ldg(p.sn + ((size_t)c * S.heads + h) * p.dp + i);
-        const float M = __ldg(p.mx + at + r), w = __ldg(p.w + at + r), floor = __ldg(p.floor + at + r);
+            for (int i = tid; i < p.dp; i += MP_WARPS * 32) s_n[i] = __ldcg(p.sn + ((size_t)c * S.heads + h) * p.dp + i);
+        const float M = __ldcg(p.mx + at + r), w = __ldcg(p.w + at + r), floor = __ldcg(p.floor + at + r);
         bool ok = true;
         float den = 0.f;
         partial_sync_2(MP_WARPS * 32);

@@ -1,0 +1,70 @@
+"""Rules that the kernels' text has to keep because a run on a GPU shows a break only by chance."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llama2.jl_b200", "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"/\*.*?\*/", "", f.read(), flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def closing(text, at):
+    """Index of the bracket that closes the one at `at`."""
+    pairs = {"(": ")", "{": "}"}
+    opened, closed, depth = text[at], pairs[text[at]], 0
+    for i in range(at, len(text)):
+        depth += (text[i] == opened) - (text[i] == closed)
+        if depth == 0:
+            return i
+    raise ValueError("unbalanced")
+
+
+def kernels(text):
+    """(name, parameters, body) of every __global__ function."""
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(", text):
+        end = closing(text, m.end() - 1)
+        start = text.index("{", end)
+        yield m.group(1), text[m.end():end], text[start:closing(text, start) + 1]
+
+
+FILES = sorted(f for f in os.listdir(CSRC) if f.endswith(".cuh"))
+
+# What the kernels of a file read through the read-only path: weights, gains, biases, tables, and index lists that the host
+# uploaded before the chain of launches began.
+CONSTANTS = {
+    "attention.cuh": {"p.pos_list"},
+    "dense_gemm.cuh": {"e.bias"},
+    "dense_matvec.cuh": {"p.upd.w", "p.upd.step"},
+    "dense_ops.cuh": {"cs", "e.bias", "e.tokens", "n.w", "n.b"},
+    "fused_matvec.cuh": {"p.gain", "p.rope_cs", "d6A", "d6B", "wa", "wb"},
+    "head_attention.cuh": {"w", "cs"},
+    "kq_gemm.cuh": {"s", "sg.d6"},  # s: the gains
+    "latent_attention.cuh": {"p.dnorm", "p.sink"},
+    "latent_prefill.cuh": {"p.sink"},
+    "mlstm.cuh": {"p.norm"},
+    "mlstm_prefill.cuh": {"p.m.norm"},
+    "prefill_ops.cuh": {"tokens", "p.pos_list", "p.rope_cs"},
+    "stack_rows.cuh": {"tv", "pv", "p.index", "p.upd.w", "p.upd.step"},
+    "token_kernel.cuh": {"s4", "tp.ops", "d6A", "d6B"},
+}
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_read_only_path_for_constants(name):
+    """Kernels start while their predecessor still writes, and the read-only path (__ldg, const __restrict__) is defined only for memory that nobody
+    writes while the kernel runs: such a load may be moved above the wait, and its line may be an old one."""
+    text = source(name)
+    for m in re.finditer(r"\b__ldg\(", text):
+        arg = text[m.end():closing(text, m.end() - 1)]
+        arg = re.sub(r"reinterpret_cast<[^>]*>\(", "", arg).lstrip("&(")
+        root = re.match(r"[\w.]*\w", arg).group(0)
+        assert root in CONSTANTS.get(name, set()), f"{name}: __ldg({arg})"
+    for kernel, params, body in kernels(text):
+        if "pdl_wait()" in body:
+            inputs = set(re.findall(r"const [\w:]+\*\s*__restrict__\s+(\w+)", params))
+            assert inputs <= {"table", "d6", "rope"}, f"{name}: {kernel}"
