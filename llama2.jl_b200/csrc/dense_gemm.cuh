@@ -241,10 +241,8 @@ __global__ void __launch_bounds__(BG_THREADS, 1) bf16_gemm_kernel(const __grid_c
         for (int tile = first; tile < tiles; tile += pairs, ++n) {
             const int buf = n & 1, tok0 = tile % p.ntiles * p.N;
             const int f = DUAL ? tile / p.ntiles * 128 + rank * 64 + (r & 63) : tile / p.ntiles * 256 + rank * 128 + r;
-            if (!__all_sync(0xffffffffu, mbar_wait_bounded(s_acc + buf, (uint32_t)((n >> 1) & 1)))) {
-                ok = false;
-                break;
-            }
+            // (the warps of a group meet at the barriers below, so a wait that runs out is carried along and not left by; nothing is stored then)
+            if (ok && !__all_sync(0xffffffffu, mbar_wait_bounded(s_acc + buf, (uint32_t)((n >> 1) & 1)))) ok = false;
             tc_fence_after();
             const uint32_t ta = tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(buf * 256);
 #pragma unroll 1
@@ -268,16 +266,16 @@ __global__ void __launch_bounds__(BG_THREADS, 1) bf16_gemm_kernel(const __grid_c
                     for (int k = 0; k < 16; ++k) {
                         const float other = from[64 * k], own = is_up ? v[16 + k] : v[k];
                         const float g = is_up ? other : own, u = is_up ? own : other;
-                        if (k < mine && f < p.rows) put(act + (size_t)(t0 + k) * p.epi.ld + f, (p.epi.kind == DE_SWIGLU ? silu(g) : gelu_tanh(g)) * u);
+                        if (ok && k < mine && f < p.rows) put(act + (size_t)(t0 + k) * p.epi.ld + f, (p.epi.kind == DE_SWIGLU ? silu(g) : gelu_tanh(g)) * u);
                     }
                     asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory");
-                } else if (f < p.rows) {
+                } else if (ok && f < p.rows) {
                     epilogue_tokens(p.epi, tok0 + c, left, f, v);
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(cluster_map(s_acc_free + buf, 0));
+            if (ok && lane == 0) mbar_arrive_cluster(cluster_map(s_acc_free + buf, 0));
         }
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
     }

@@ -68,3 +68,35 @@ def test_read_only_path_for_constants(name):
         if "pdl_wait()" in body:
             inputs = set(re.findall(r"const [\w:]+\*\s*__restrict__\s+(\w+)", params))
             assert inputs <= {"table", "d6", "rope"}, f"{name}: {kernel}"
+
+
+BARRIER = re.compile(r"bar\.sync|\bpa_bar_sync\(|\bpartial_sync(?:_2)?\(|\bconsumer_sync\(|\bblock_sum(?:_all)?\b")
+
+
+def loops(text):
+    """Body of every loop with braces."""
+    for m in re.finditer(r"\bfor\s*\(|\bwhile\s*\(", text):
+        end = closing(text, m.end() - 1)
+        start = re.match(r"\s*(?:for\s*\([^{]*\)\s*)?", text[end + 1:]).end() + end + 1  # (two headers over one body)
+        if text[start] == "{":
+            yield text[start:closing(text, start) + 1]
+
+
+def conditions(text):
+    """(condition, what is done) of every if with braces."""
+    for m in re.finditer(r"\bif\s*\(", text):
+        end = closing(text, m.end() - 1)
+        start = re.match(r"\s*", text[end + 1:]).end() + end + 1
+        stop = closing(text, start) + 1 if text[start] == "{" else text.index(";", start) + 1
+        yield text[m.end():end], text[start:stop]
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_no_warp_leaves_a_loop_with_a_barrier(name):
+    """A bounded wait may run out for one warp and not for the next.  Where warps meet at a named barrier, which has no bound, the verdict is carried along
+    to the loop's end: a warp that left would be waited for without end."""
+    for kernel, _, body in kernels(source(name)):
+        for loop in loops(body):
+            if BARRIER.search(loop):
+                for cond, then in conditions(loop):
+                    assert not ("mbar_wait" in cond and re.search(r"\b(break|return)\b", then)), f"{name}: {kernel}: {cond}"
