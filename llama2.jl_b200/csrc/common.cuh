@@ -88,6 +88,10 @@ __device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity)
     return false;
 }
 
+// The same by a whole warp that goes on together (tensor memory, votes and shuffles need all of its threads): its threads could see the budget run
+// out in different polls.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_parked(bar, parity)); }
+
 // The same wait bounded by TIME (nanoseconds of %globaltimer) instead of by polls: for warps whose partner may itself be
 // inside a long, legitimate wait (the tensor-parallel wait for another GPU's partial results).
 __device__ __forceinline__ bool mbar_wait_bounded_ns(uint64_t* bar, uint32_t parity, unsigned long long limit_ns) {

@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         for (Where w = first_unit(item); w.u < w.end && ok; advance(w)) {
             const int steps = w.steps;
             for (int k = 0; k < steps; ++k) {
-                if (!mbar_wait_parked(ready + s, parity)) {
+                if (!mbar_wait_warp(ready + s, parity)) {
                     ok = false;
                     break;
                 }
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
             advance(w);
             fresh = w.u == w.end;
             if (!fresh) d6_next = q6_scale(w);  // a super-block ahead: the latency of a global read
-            if (!mbar_wait_parked(p_full + ps, p_parity)) {  // (every group follows every packed slot, with or without a step in it)
+            if (!mbar_wait_warp(p_full + ps, p_parity)) {  // (every group follows every packed slot, with or without a step in it)
                 ok = false;
                 break;
             }
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
                     parity ^= 1u;
                 }
                 if (!mine) continue;
-                if (reused && !mbar_wait_parked(done + slot, use_parity)) {
+                if (reused && !mbar_wait_warp(done + slot, use_parity)) {
                     ok = false;
                     break;
                 }
@@ -794,7 +794,7 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
             const int steps = w.steps;
             float2 f = make_float2(0.f, 0.f);
             for (int k = 0; k < steps; ++k) {
-                if (!mbar_wait_parked(done + s, parity)) {
+                if (!mbar_wait_warp(done + s, parity)) {
                     ok = false;
                     break;
                 }

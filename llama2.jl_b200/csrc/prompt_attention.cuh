@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
         const uint64_t dv = umma_desc(smem + L.off_v, hs * 16, 128), dp = umma_desc(smem + L.off_p, PA_ROWS * 16, 128);
         const uint32_t q_lo = q_term >> 4, kv_lo = kv_term >> 4, p_lo = p_term >> 4;
         auto scores = [&](int j) {
-            if (!mbar_wait_parked(k_ready, (uint32_t)(j & 1))) return false;
+            if (!mbar_wait_warp(k_ready, (uint32_t)(j & 1))) return false;
             tc_fence_after();
             if (elect_one()) {
 #pragma unroll 1
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
         };
         ok = scores(0);
         for (int j = 0; j < tiles && ok; ++j) {
-            if (!mbar_wait_parked(p_ready, (uint32_t)(j & 1)) || !mbar_wait_parked(v_ready + (j & 1), (uint32_t)((j >> 1) & 1))) {
+            if (!mbar_wait_warp(p_ready, (uint32_t)(j & 1)) || !mbar_wait_warp(v_ready + (j & 1), (uint32_t)((j >> 1) & 1))) {
                 ok = false;
                 break;
             }
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
             }
             pa_bar_sync(2, CT);
             const float ks = conv.key_scale[key];
-            if (ok && j > 0 && !mbar_wait_parked(s_full + ((j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1))) ok = false;  // the last scores have read the keys
+            if (ok && j > 0 && !mbar_wait_warp(s_full + ((j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1))) ok = false;  // the last scores have read the keys
             if (ok) {
 #pragma unroll
                 for (int u = 0; u < ITEMS; ++u) {
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
             __syncwarp();
             if (ok && lane == 0) mbar_arrive(k_ready);
             if (j + 1 < tiles) fetch_k(j + 1);
-            if (ok && j > 1 && !mbar_wait_parked(pv_full + (j & 1), (uint32_t)(((j - 2) >> 1) & 1))) ok = false;
+            if (ok && j > 1 && !mbar_wait_warp(pv_full + (j & 1), (uint32_t)(((j - 2) >> 1) & 1))) ok = false;
             if (ok) {
 #pragma unroll
                 for (int u = 0; u < ITEMS; ++u) {
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
         };
         for (int j = 0; j < tiles; ++j) {
             // (both halves' warps meet at the barrier below, so a wait that runs out is carried along and not left by)
-            if (ok && !mbar_wait_parked(s_full + (j & 1), (uint32_t)((j >> 1) & 1))) ok = false;
+            if (ok && !mbar_wait_warp(s_full + (j & 1), (uint32_t)((j >> 1) & 1))) ok = false;
             float s[32];
             if (ok) {
                 tc_fence_after();
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
             // weights take the scales of their values along; a power of two per row brings the largest of them to 2^12 .. 2^13
             const int ie = (int)fminf(fmaxf(ceilf(fmaxf(tx, other.y) - mn), -100.f), 126.f);
             const float w_scale = __uint_as_float((uint32_t)(140 - ie) << 23);
-            if (ok && j > 0 && !mbar_wait_parked(pv_full + ((j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1))) ok = false;
+            if (ok && j > 0 && !mbar_wait_warp(pv_full + ((j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1))) ok = false;
             if (ok) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(PA_THREADS, 1) prompt_attention_kernel(const _
             alpha_prev = alpha;
             vfac_prev = __uint_as_float((uint32_t)(114 + ie) << 23);
         }
-        if (ok && !mbar_wait_parked(pv_full + ((tiles - 1) & 1), (uint32_t)(((tiles - 1) >> 1) & 1))) ok = false;
+        if (ok && !mbar_wait_warp(pv_full + ((tiles - 1) & 1), (uint32_t)(((tiles - 1) >> 1) & 1))) ok = false;
         if (ok) {
             tc_fence_after();
             add_output();

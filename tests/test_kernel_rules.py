@@ -100,3 +100,24 @@ def test_no_warp_leaves_a_loop_with_a_barrier(name):
             if BARRIER.search(loop):
                 for cond, then in conditions(loop):
                     assert not ("mbar_wait" in cond and re.search(r"\b(break|return)\b", then)), f"{name}: {kernel}: {cond}"
+
+
+def headers(text, at):
+    """What stands in front of every brace that is open at `at`."""
+    out, depth = [], 0
+    for i in range(at - 1, -1, -1):
+        depth += (text[i] == "}") - (text[i] == "{")
+        if depth < 0:
+            depth = 0
+            out.append(text[max(text.rfind(c, 0, i) for c in ";{}") + 1:i])
+    return out
+
+
+@pytest.mark.parametrize("name", [f for f in FILES if "tmem_ld" in source(f) and f != "tcgen05.cuh"])
+def test_a_warp_decides_together_whether_a_wait_ran_out(name):
+    """Loads and stores of tensor memory, votes and shuffles need all threads of a warp.  So where a whole warp waits, its threads agree on the verdict; alone
+    wait only threads that work alone."""
+    for kernel, _, body in kernels(source(name)):
+        for m in re.finditer(r"\bmbar_wait_(?:bounded|parked)\(", body):
+            together = re.search(r"__all_sync\(0xffffffffu,\s*$", body[:m.start()])
+            assert together or any("lane == 0" in h for h in headers(body, m.start())), f"{name}: {kernel}: {body[m.start():m.start() + 60]}"
