@@ -94,3 +94,33 @@ def test_prompt_passes_take_the_room_there_is(pkg, synth):
     assert np.abs(tight.logits - roomy.logits).max() < 2e-5 * float(roomy.logits.max() - roomy.logits.min())
     for m in models:
         m.close()
+
+
+@pytest.mark.parametrize("n_in,ncols", [(14336, 148), (14336, 149), (28672, 74), (28672, 75)])
+def test_columns_of_long_rows(pkg, orc, synth, n_in, ncols):
+    """Where a column's blocks are so few that a warp has more than two super-blocks of it (the second of each pair), its values are read a second time.
+    Bound as above."""
+    A = synth.matrix(12, n_in, 64, seed=n_in)
+    X = synth.normal_f32(ncols * n_in, ncols, 1.0).reshape(ncols, n_in)
+    Y = np.full((ncols, 64), np.nan, np.float32)
+    pkg.matmul_(Y, A, X)
+    for c in range(ncols):
+        want = orc.matmul_f64(A, X[c])
+        assert np.abs(Y[c] - want).max() <= 4e-6 * np.abs(want).max(), c
+
+
+@pytest.mark.parametrize("dim,hidden,heads,kv", [(256, 14336, 4, 2), (8448, 256, 66, 2)])
+def test_prompt_of_long_rows(pkg, orc, synth, dim, hidden, heads, kv):
+    """The same behind the feed-forward's activation and behind the residual update and the norm.  Bound as above."""
+    cfg = pkg.ModelConfig(dim, hidden, 1, heads, kv, 512, 160, 10000.0, False)
+    w = synth.model_weights(cfg, dict(synth.ALL(12), output=14), seed=hidden)
+    w.layers[0].rms_att_weight, w.layers[0].rms_ffn_weight = (1 + synth.normal_f32(dim, i, 0.2) for i in (1, 2))
+    ids = synth.tokens(150, 23, 3, cfg.vocab_size)
+    tokens, want = orc.OracleModel(cfg, w).sample_greedy(ids, 151, want_logits=True)
+    model = pkg.LanguageModel(cfg, None, w)
+    st = pkg.RunState(model)
+    assert pkg.prefill(st, ids, 0) == int(tokens[149])
+    assert np.abs(st.logits - want[149]).max() / float(want[149].max() - want[149].min()) < 5e-5
+    pkg.transformer_(int(tokens[149]), 150, cfg, st)
+    assert np.abs(st.logits - want[150]).max() / float(want[150].max() - want[150].min()) < 5e-5
+    model.close()

@@ -91,6 +91,24 @@ def test_shapes_against_oracle(pkg, orc, synth, case):
     model.close()
 
 
+@pytest.mark.parametrize("dim,hidden,heads,kv,neox", [(512, 768, 8, 4, False), (768, 1528, 12, 12, True), (1024, 1536, 16, 2, False), (1536, 1544, 12, 12, False), (392, 776, 7, 7, False)])
+def test_f32_models_of_other_widths(pkg, orc, synth, dim, hidden, heads, kv, neox):
+    """f32 models whose rows take each of the widths that a warp keeps in registers (up to 384, 768, 1536 values), and longer ones, with every prologue and
+    epilogue.  A product's error is at most (4 * 12 + 5) * 2^-24 = 3.2e-6 of the sum of its terms' magnitudes; six of them in a row per layer."""
+    cfg = pkg.ModelConfig(dim, hidden, 2, heads, kv, 600, 40, 10000.0, neox)
+    w = synth.model_weights(cfg, dict(synth.ALL(0), output=0), seed=dim)
+    for i, layer in enumerate(w.layers):
+        layer.rms_att_weight, layer.rms_ffn_weight = (1 + synth.normal_f32(dim, 10 * i + j, 0.2) for j in (1, 2))
+    prompt = synth.tokens(4, 5, 3, cfg.vocab_size)
+    want_tokens, want = orc.OracleModel(cfg, w).sample_greedy(prompt, 40, want_logits=True)
+    model = pkg.LanguageModel(cfg, None, w)
+    got, _ = pkg.generate(model, prompt, 40)
+    assert np.array_equal(got, want_tokens)
+    logits = teacher_forced(pkg, model, np.concatenate([prompt[:1], want_tokens]), 40)
+    assert max(logit_err(logits[p], want[p]) for p in range(40)) < 2e-5
+    model.close()
+
+
 def test_decode_next_session_semantics(pkg, synth):
     """One-step calls, reset, determinism, argument checks."""
     import ctypes as C

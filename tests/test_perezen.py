@@ -130,6 +130,19 @@ def test_prompt_decode_and_portions(pkg, case, compute):
     model.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("compute", COMPUTE)
+@pytest.mark.parametrize("width, ff, vocab", [(248, 257, 90), (264, 256, 700), (2048, 4104, 130), (2056, 330, 130), (4096, 264, 2500), (4104, 4096, 130)])
+def test_decode_products_by_row_length(pkg, width, ff, vocab, compute):
+    """Decode products whose rows a warp keeps in registers (up to 256, 2048 and 4096 values; pairs of them up to 256 and 2048) and longer ones, with fewer
+    results than blocks, one per block, fewer and more per block than warps."""
+    cfg = pc.config([(pc.attention(heads=2, kv_heads=1), ff), (pc.mlstm(heads=2), None)], width=width, vocab=vocab, positions=6)
+    w, t = pc.weights(cfg, 51), pc.tokens(cfg, 6, 52)
+    model = build(pkg, cfg, w, 6, compute)
+    check(feed(pkg, pkg.RunState(model), t, [1]), expected(cfg, w, t), compute)
+    model.close()
+
+
 def only(cfg, w, keep):
     """Weights whose other mechanisms are silent: what is not named in `keep` adds zero to the residual stream."""
     w = {k: v.copy() for k, v in w.items()}

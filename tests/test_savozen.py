@@ -139,6 +139,19 @@ def test_products_at_tile_edges(pkg, width, ff, n):
     model.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("compute", COMPUTE)
+@pytest.mark.parametrize("width, ff, vocab", [(248, 257, 90), (264, 256, 700), (2048, 4104, 130), (2056, 330, 130), (4096, 264, 2500), (4104, 4096, 130)])
+def test_decode_products_by_row_length(pkg, width, ff, vocab, compute):
+    """Decode products whose rows a warp keeps in registers (up to 256, 2048 and 4096 values; pairs of them up to 256 and 2048) and longer ones, with fewer
+    results than blocks, one per block, fewer and more per block than warps."""
+    cfg = sc.config([(sc.mixer(heads=2), ff)], width=width, vocab=vocab, side=40)
+    w, t = sc.weights(cfg, 51), sc.tokens(cfg, 6, 52)
+    model = build(pkg, cfg, w, 6, compute)
+    check(feed(pkg, pkg.RunState(model), t, [1]), expected(cfg, w, t), compute)
+    model.close()
+
+
 def only(cfg, w, keep):
     """Weights whose other mechanisms are silent: residual contributions not named in `keep` are zero."""
     w = {k: v.copy() for k, v in w.items()}
