@@ -453,8 +453,8 @@ static int gemm_max_parts(const GemmSplit& s) { return s.U % s.nb == 0 ? 1 : s.n
 static int gemm_row_tiles(const DevMatrix& w) { return (int)((w.out + GM_ROWS - 1) / GM_ROWS); }
 
 template <int MODE>
-static int32_t launch_split_rows(const SplitRowsParams& q, cudaStream_t st, bool pdl = true) {
-    const SplitRowsShape sh = split_rows_shape(q.n, q.n_tok);
+static int32_t launch_split_rows(const SplitRowsParams& q, int sms, cudaStream_t st, bool pdl = true) {
+    const SplitRowsShape sh = split_rows_shape(q.n, q.n_tok, sms);
     CU(launch_kernel(split_rows_kernel<MODE>, dim3(sh.cluster, q.n_tok), dim3(sh.warps * 32), (size_t)(q.n / QK_K) * 4, st, pdl, q, sh.cluster));
     return L2B_OK;
 }
@@ -534,7 +534,7 @@ static int32_t launch_columns(const DevMatrix& w, const float* x, int ncols, flo
     for (int c = 0; c < ncols; c += PRODUCT_SLAB) {
         const int n = std::min(ncols - c, PRODUCT_SLAB);
         const GemmInput in = gemm_input(workspace, w.in, n);
-        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(const_cast<float*>(x) + (size_t)c * w.in, nullptr, (int)w.in, n, in), st, false));
+        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(const_cast<float*>(x) + (size_t)c * w.in, nullptr, (int)w.in, n, in), sms, st, false));
         L2B_TRY(launch_product(w, in, n, y + (size_t)c * w.out, (float*)(workspace + product_operand_bytes(w, n)), sms, status, st));
     }
     return L2B_OK;
@@ -1962,7 +1962,7 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
     GemmSplit sp;
     size_t stride = 0;
     int ldy = 0;
-    L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.x, m->layers[0].rms_att, c.dim, n, in_dim), st, false));
+    L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.x, m->layers[0].rms_att, c.dim, n, in_dim), B.sms, st, false));
     for (int l = 0; l < c.n_layers; ++l) {
         const LayerW& w = m->layers[l];
         float* kcl = kc + (size_t)l * layer_stride;
@@ -1996,14 +1996,14 @@ static int32_t enqueue_layers_gemm(const l2b_model* m, const GemmBufs& B, int n,
             if (n < 2) return fail(L2B_ERR_BAD_ARG, "a many-token pass needs at least two tokens");
             CU(launch_attention(a, gq, st, true));
         }
-        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.att, nullptr, c.dim, n, in_dim), st));
+        L2B_TRY(launch_split_rows<SR_PLAIN>(split_rows_params(B.att, nullptr, c.dim, n, in_dim), B.sms, st));
         L2B_TRY(product({&w.wo}, in_dim, sp, stride, ldy));
-        L2B_TRY(launch_split_rows<SR_RESIDUAL>(behind(split_rows_params(B.x, w.rms_ffn, c.dim, n, in_dim), sp, stride, ldy, 0), st));
+        L2B_TRY(launch_split_rows<SR_RESIDUAL>(behind(split_rows_params(B.x, w.rms_ffn, c.dim, n, in_dim), sp, stride, ldy, 0), B.sms, st));
         L2B_TRY(product({&w.w1, &w.w3}, in_dim, sp, stride, ldy));
-        L2B_TRY(launch_split_rows<SR_SWIGLU>(behind(split_rows_params(B.h, nullptr, c.hidden_dim, n, in_hid), sp, stride, ldy, gemm_row_tiles(w.w1) * GM_ROWS), st));
+        L2B_TRY(launch_split_rows<SR_SWIGLU>(behind(split_rows_params(B.h, nullptr, c.hidden_dim, n, in_hid), sp, stride, ldy, gemm_row_tiles(w.w1) * GM_ROWS), B.sms, st));
         L2B_TRY(product({&w.w2}, in_hid, sp, stride, ldy));
         const float* gain = l + 1 < c.n_layers ? m->layers[l + 1].rms_att : final_gain;
-        L2B_TRY(launch_split_rows<SR_RESIDUAL>(behind(split_rows_params(B.x, gain, c.dim, n, gain ? in_dim : GemmInput()), sp, stride, ldy, 0), st));
+        L2B_TRY(launch_split_rows<SR_RESIDUAL>(behind(split_rows_params(B.x, gain, c.dim, n, gain ? in_dim : GemmInput()), sp, stride, ldy, 0), B.sms, st));
     }
     return L2B_OK;
 }

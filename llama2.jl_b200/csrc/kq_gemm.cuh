@@ -161,16 +161,16 @@ struct SplitRowsParams {
     uint8_t *act, *xs;   // null: only the values are wanted (x; not with SR_SWIGLU)
     float* scale;
 };
-constexpr int SR_MAX_CLUSTER = 8, SR_MAX_WARPS = 16, SR_KEEP = 2, SR_MAX_BLOCKS = 2 * 148;  // SR_KEEP: super-blocks that a warp keeps in registers
+constexpr int SR_MAX_CLUSTER = 8, SR_MAX_WARPS = 16, SR_KEEP = 2;  // SR_KEEP: super-blocks that a warp keeps in registers
 // Blocks per token (a cluster) and warps per block.  The sum of squares is added up super-block by super-block, whatever the shape is.  As many
 // blocks as give every SM two: beyond that clusters cost more than they bring (512 tokens of 8192 values, SwiGLU: 45 us with eight blocks each, 21 with one).
 struct SplitRowsShape {
     int cluster, warps;
 };
-inline SplitRowsShape split_rows_shape(int n, int n_tok) {
+inline SplitRowsShape split_rows_shape(int n, int n_tok, int sms) {
     const int nb = n / QK_K;
     int cl = SR_MAX_CLUSTER;
-    while (cl > 1 && (cl * n_tok > SR_MAX_BLOCKS || nb < 2 * cl)) cl /= 2;
+    while (cl > 1 && (cl * n_tok > 2 * sms || nb < 2 * cl)) cl /= 2;
     const int per = (nb + cl - 1) / cl;
     return {cl, per < SR_MAX_WARPS ? per : SR_MAX_WARPS};
 }
