@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(MP_THREADS, 1) mlstm_state_kernel(const __grid
             const bf16* src = p.v + (size_t)(c * MP_L + tok) * S.heads * p.vp + (size_t)h * p.vp + cc;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                v[i] = c < p.nchunk && c * MP_L + tok < p.n && cc + 8 * i < p.vp ? __ldcg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
+                v[i] = c < p.nchunk && c * MP_L + tok < p.n && cc + 8 * i < p.vp ? reinterpret_cast<const uint4*>(src)[i] : make_uint4(0u, 0u, 0u, 0u);
             u = c < p.nchunk ? __ldcg(p.u + ((size_t)h * p.nchunk + c) * MP_L + tok) : 0.f;
         };
         auto weigh = [&](int c) {  // u V of chunk c in two terms; rows are tokens

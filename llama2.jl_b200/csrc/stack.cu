@@ -1005,7 +1005,7 @@ static int32_t enqueue_latent_rows(StackSession* s, int run, int n, int pos0, co
     const bf16* cache = static_cast<const bf16*>(a.c.cache);
     L2B_TRY(launch_gemm(s, w.uk, cache, sh.row, npos, dense_epilogue_of(DE_STORE_ACT, nullptr, s->pk, sh.heads * sh.dp), status, st));
     L2B_TRY(launch_gemm(s, w.uv, cache, sh.row, npos, dense_epilogue_of(DE_STORE_T, nullptr, s->pv, s->pv_ld), status, st));
-    CU(launch_kernel_args(latent_queries_kernel, dim3(n, sh.heads), dim3(128), 0, st, true, 1, (const float*)s->in, a.ld, a.rope, pos0, sh, dq, s->pq));
+    CU(launch_kernel_args(latent_queries_kernel, dim3(n, std::max(1, std::min(sh.heads, 32 * s->di.sms / n))), dim3(128), 0, st, true, 1, (const float*)s->in, a.ld, a.rope, pos0, sh, dq, s->pq));
     LatentPrefillParams f;
     memset(&f, 0, sizeof(f));
     f.n = n; f.pos0 = pos0; f.dim = sh.dim; f.rot = sh.rot; f.vdim = sh.vdim; f.dp = sh.dp; f.dq = dq; f.vp = sh.vp; f.kstages = kstages;

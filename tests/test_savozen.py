@@ -152,6 +152,17 @@ def test_decode_products_by_row_length(pkg, width, ff, vocab, compute):
     model.close()
 
 
+@pytest.mark.gpu
+def test_queries_of_long_portions(pkg):
+    """Portions so long that a block of the kernel that makes the query operands takes several heads (more than 32 blocks per SM otherwise): 7 heads in 3 parts,
+    and in 4 behind them."""
+    cfg = sc.config([(sc.mixer(heads=7), None)], width=72, vocab=130)
+    w, t = sc.weights(cfg, 61), sc.tokens(cfg, 2500, 62)
+    model = build(pkg, cfg, w, 2500, "bfloat16")
+    check(feed(pkg, pkg.RunState(model), t, [1400, 1100]), expected(cfg, w, t), "bfloat16")
+    model.close()
+
+
 def only(cfg, w, keep):
     """Weights whose other mechanisms are silent: residual contributions not named in `keep` are zero."""
     w = {k: v.copy() for k, v in w.items()}
