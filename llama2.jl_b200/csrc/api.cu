@@ -1898,8 +1898,9 @@ constexpr int PF_MAX_TOK = 512;
 // Shortest run of forced positions (their last one is followed by a prompt token) that takes a pass: where l2b_generate stops inside the prompt, and in
 // front of the last position of a prompt of several passes.  From the integer form of the product; not measured anew.
 constexpr int PF_MIN_TOK = 12;
-// Shortest prompt whose last position goes through the pass too, so that the matrices are read once for all of it.  At the 8B shape a pass of a
-// few tokens takes 6.4 ms and the decode kernels 1.6 ms per position or pair of forced positions: even at about eight.
+// Shortest prompt whose last position goes through the pass too, so that the matrices are read once for all of it.  Where the line lies dates from passes of
+// 6.4 ms (8B shape, few tokens), which were even with the decode kernels at about eight positions.  A pass of 10 takes 3.8 ms now (Phi-3 shape 2.7), while the
+// decode kernels take 3.1 ms for 2 positions, 5.0 for 4, 8.8 for 9 (2.4, 3.7, 6.8): the line would lie at three or four.
 constexpr int PF_MIN_ALL = 10;
 constexpr int BATCH_MAX_SEQ = 240;
 constexpr int STACK_MIN_ROWS = 2;  // layer-stack models
@@ -1918,7 +1919,7 @@ static bool prompt_attention_better(int n, int pos0, int n_heads, int gq, int hs
     return tiled < split;
 }
 // Parts that a query's positions are in, for the split kernel: so many that few queries still make about four blocks per SM (29 queries behind 211, 32
-// heads on 8: 25 us with one part each, 14 us with eight).
+// heads on 8: 25 us with one part each, 14 us with eight).  SPLIT_BLOCKS: four for each of a B200's 148 SMs; buffers are sized by it.
 constexpr int SPLIT_BLOCKS = 600, SPLIT_MOST = 8;
 static int prompt_splits(int n, int groups, const GemmBufs& B) { return std::max(B.nsplit, std::min(SPLIT_MOST, SPLIT_BLOCKS / std::max(1, n * groups))); }
 static int32_t launch_prompt_attention(const PromptAttnParams& a, int gq, cudaStream_t st) {
@@ -2116,8 +2117,8 @@ static int32_t enqueue_forced_positions(l2b_session* s, int from, int to, const 
 // All positions [from, end) of a prompt in one many-token pass, the last one included: its logits and the choice of the token behind it as the
 // one-position graph leaves them (and its row in the buffers that l2b_session_read shows).  False: not taken, nothing enqueued.
 static int32_t enqueue_whole_prompt(l2b_session* s, int from, int end, int32_t last_token, bool& taken) {
-    // Prompts of one pass: there one more reading of the matrices would weigh (1.3 of 8 ms at 128 positions of the 8B shape).  Behind longer ones it
-    // is 2 % (1.3 of 61 ms, Phi-3 shape, 2048 positions), and the row takes the decode kernels as in every other model.
+    // Prompts of one pass: there one more reading of the matrices would weigh (1.5 of 7 ms at 128 positions of the 8B shape).  Behind longer ones it
+    // is 2 - 3 % (1.6 of 64 ms, Phi-3 shape, 2048 positions), and the row takes the decode kernels as in every other model.
     taken = !s->stack && end - from >= PF_MIN_ALL && prefill_gemm_eligible(s) && end - from <= s->pf.tokens;
     if (!taken) return L2B_OK;
     const l2b_model* m = s->model;

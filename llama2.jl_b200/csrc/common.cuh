@@ -149,7 +149,8 @@ __device__ __forceinline__ void bulk_g2s_plain(void* dst_smem, const void* src_g
 
 // Programmatic dependent launch: let the next kernel in the stream start its prologue,
 // and wait until the previous kernel's memory is visible.  What earlier kernels of a chain wrote is read after the wait with __ldcg or plain
-// loads; __ldg and const __restrict__ are for what nobody writes while the kernel runs (weights, gains, tables).
+// loads; __ldg and const __restrict__ are for what nobody writes while the kernel runs (weights, gains, tables).  A block has let the next kernel go
+// when the first of its threads says so; a warp with nothing more to do says so long before the block's end.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) bf16_gemm_kernel(const __grid_c
     }
     // every path ends here, in both blocks: no products, arrivals or copies of the other one are under way when this one leaves
     __syncwarp();
-    pdl_launch_dependents();
+    pdl_launch_dependents();  // (a block's first warp here releases the next kernel: the second block's warp 1 at once, the first one's producer behind its last copy)
     tc_fence_before();
     cluster_sync_all();
     if (warp == 1) tmem_dealloc_pair(tmem, 512);

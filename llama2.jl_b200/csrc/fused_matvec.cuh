@@ -1224,12 +1224,12 @@ __global__ void __launch_bounds__((MV_MAX_CONSUMERS + 2) * 32, 1) fused_matvec_k
 
 // ---- f32 matrices of short rows -----------------------------------------------------------------
 // The launches of a small f32 model (llama2.c checkpoints, whose weights stay in L2) last as long as their chain of dependent latencies:
-// previous kernel done -> vector read -> norm -> products -> result.  So a warp works alone, with no barrier and no shared memory: it
-// fetches its first row pair and the gains before the wait on the previous kernel, keeps its part of the vector (4 NV values per lane) in
-// registers, adds up the squares beside the products and applies 1/rms to the results (W (c z) = c (W z)); the next pair's rows are
-// under way while this one's sums go round the lanes.  Rows of up to 128 * NV values; longer ones take fused_matvec_kernel<false>, which
-// keeps the vector in shared memory.  A launch of the 288-wide model (6 layers) takes 2.3 us in the chain, 4.7 us there (79 positions: 12.3
-// and 6.0 ms).
+// previous kernel done -> vector read -> norm -> products -> result.  So a warp works alone, with no barrier and no shared memory (but for the
+// classifier, whose warps bring their maxima together at the end): it fetches its first row pair and the gains before the wait on the previous
+// kernel, keeps its part of the vector (4 NV values per lane) in registers, adds up the squares beside the products and applies 1/rms to the
+// results (W (c z) = c (W z)); the next pair's rows are under way while this one's sums go round the lanes.  Rows of up to 128 * NV values;
+// longer ones take fused_matvec_kernel<false>, which keeps the vector in shared memory.  A launch of the 288-wide model (6 layers) takes 2.3 us
+// in the chain, 4.7 us there (79 positions: 12.3 and 6.0 ms).
 constexpr int f32_max_warps(int nv) { return nv <= 6 ? MV_MAX_CONSUMERS : MV_MAX_CONSUMERS / 2; }  // so that 20 NV values find their registers
 template <int NV>
 __global__ void __launch_bounds__(f32_max_warps(NV) * 32, 1) f32_matvec_kernel(const __grid_constant__ MvParams p) {

@@ -96,11 +96,12 @@ struct GemmMaps {
 // of one super-block made the kernel issue-bound.)
 // AT: with 128 tokens the products read 64 KB of shared memory per 64 values when the weights come from there too (each of the two terms
 // reads them again), as much as an SM delivers while they run, and copies and unpacking want another 57 KB.  From tensor memory the weights cost
-// nothing of it, and there is room for four slots of activations: 1240 -> 930 cycles per 64 values (q4_K 28672 x 4096 times 128).  That leaves two
+// nothing of it, and there is room for four slots of activations: 1240 -> 930 cycles per step (q4_K 28672 x 4096 times 128).  That leaves two
 // sets of accumulators instead of three.  (Blocks in pairs that share the activations, cta_group::2: 1270 - 1350 cycles; 16 epilogue warps: no
 // faster.)  With 32 tokens an MMA takes 46 cycles instead of 16 for the weights' sake, and the unpack warps, whose instructions bound the kernel
 // there, wait behind it: 24 sequences of the 8B shape 10.6 -> 10.1 ms, 29 tokens 2.46 -> 2.31 ms.  With 64 there is no room beside two slots of
-// accumulators; a chunk per step, which leaves some, costs more in hand-overs (56 against 53 us, q5_K 14336 x 4096 times 37).
+// accumulators; a chunk per step, which leaves some, costs more in hand-overs (56 against 53 us, q5_K 14336 x 4096 times 37, weights not in L2).
+// The same matrix by columns, launches back to back / with L2 flushed before: 16: 33 / 49 us, 30: 35 / 46, 37: 41 / 53, 64: 42 / 55, 65: 46 / 58, 128: 50 / 63.
 // Whatever the tile holds, a column's sums are the same ones in the same order: low terms, then high terms of 64 values in one accumulator,
 // added to the f32 sum chunk by chunk, the shared part behind them.  So a column's result does not hang on how many columns came with it.
 template <int NT>
@@ -882,7 +883,9 @@ __global__ void __launch_bounds__(GmCfg<NT>::THREADS, 1) kq_gemm_kernel(const __
         if (!ok && lane == 0) atomicExch(p.status, DEV_ERR_TMA_TIMEOUT);
     }
     // every path ends here; the tensor memory is freed by the warp that allocated it
-    pdl_launch_dependents();  // (here: blocks of the next kernel that start earlier would all share the few SMs this grid leaves free)
+    // A block has released the next kernel when its first warp comes here: the one of the packed copies, with the last of them under way.  (At the start it
+    // would let the next kernel's blocks crowd onto the few SMs that this grid leaves free.)
+    pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
     if (warp == 9) tmem_dealloc(tmem_base, 512);

@@ -1,6 +1,7 @@
 // Small kernels behind the isolated-operator entry points and the upload path.  Dequantisation, the activation
 // prologue (export_activation_kernel) and the epilogues (epilogue_probe_kernel: RoPE, SwiGLU) call the very device
-// functions the fused decode kernels call, so a parity test of those entry points tests the token path's arithmetic.
+// functions the fused decode kernels call, so a parity test of those entry points tests the token path's arithmetic.  (The rms norm of f32 rows of
+// up to 1536 values apart: f32_matvec_kernel applies 1/rms to the results, and tests of whole f32 models cover it.)
 #pragma once
 #include "fused_matvec.cuh"
 

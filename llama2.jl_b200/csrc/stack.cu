@@ -415,7 +415,7 @@ static size_t act_bytes(const StackModel* m) { return m->f32 ? 4 : 2; }
 
 constexpr int ABSORB_ROWS = 64;  // rows per pass of the absorbed form of the attention (bounds its scratch)
 // The tiled forms of the attention (latent_prefill.cuh, head_prefill.cuh) and the chunked form of the recurrence (mlstm_prefill.cuh)
-// are for portions of at least this many rows.
+// are for portions of at least this many rows.  (Chosen before the products and the launches between them got faster; not measured anew.)
 constexpr int EXPAND_MIN_ROWS = 48, MLSTM_MIN_ROWS = 32;
 
 // Blocks of query vectors and ranges of positions of the scan kernel: about one block per SM in a decode step, two for several rows.
